@@ -27,6 +27,7 @@ int set_error(int code, const char* fmt, ...) {
 }
 
 static std::atomic<long long> g_gates{0}, g_passes{0}, g_param_bytes{0};
+static std::atomic<int> g_live_states[64];  // per device
 static std::atomic<int> g_tile_hint{0};
 int current_tile_hint() { return g_tile_hint.load(); }
 static std::atomic<int> g_k1_rbits{4};
@@ -241,6 +242,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
     delete st;
     return rc;
   }
+  if (cudaGetDevice(&st->dev) == cudaSuccess) ++g_live_states[st->dev & 63];
   *out = st;
   return HS_OK;
 }
@@ -249,6 +251,7 @@ int hs_state_destroy(hs_state* st) {
   if (!st) return HS_OK;
   if (st->amp) cudaFree(st->amp);
   st->amp = nullptr;
+  if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev);
   delete st;
   return HS_OK;
 }
@@ -691,36 +694,23 @@ int hs_measure(hs_state* st, const int32_t* qubits, int num_qubits, uint32_t num
   const int cb = std::min(st->n, 16);
   std::vector<double> chunk(size_t(1) << (st->n - cb));
   HS_TRY(reduce_chunks(st->amp, st->dtype, st->n, cb, chunk.data(), nullptr));
-  const size_t b = amp_bytes(st->dtype);
-  std::vector<char> host((size_t(1) << cb) * b);
+  // the chunk of every sample, from the chunks' masses; the device finds the
+  // amplitude within it
+  std::vector<MeasureChunk> touched;
   uint32_t k = 0;
   double cum = 0;
-  auto emit = [&](uint64_t pos) {
-    for (int j = 0; j < num_qubits; ++j) out[size_t(k) * num_qubits + j] = int32_t((pos >> slots[j]) & 1);
-    ++k;
-  };
   for (size_t c = 0; c < chunk.size() && k < num_samples; ++c) {
-    if (u[k] >= cum + chunk[c]) {
-      cum += chunk[c];
-      continue;
-    }
-    const uint64_t first = uint64_t(c) << cb;
-    HS_CUDA(cudaMemcpy(host.data(), static_cast<char*>(st->amp) + first * b, host.size(),
-                       cudaMemcpyDeviceToHost));
-    for (uint64_t i = 0; i < (1ull << cb) && k < num_samples; ++i) {
-      double re, im;
-      if (st->dtype == HS_DTYPE_C128) {
-        re = reinterpret_cast<double*>(host.data())[2 * i];
-        im = reinterpret_cast<double*>(host.data())[2 * i + 1];
-      } else {
-        re = reinterpret_cast<float*>(host.data())[2 * i];
-        im = reinterpret_cast<float*>(host.data())[2 * i + 1];
-      }
-      const double p = re * re + im * im;
-      while (k < num_samples && u[k] < cum + p) emit(first + i);
-      cum += p;
-    }
+    const uint32_t s0 = k;
+    while (k < num_samples && u[k] < cum + chunk[c]) ++k;
+    if (k > s0) touched.push_back({uint64_t(c) << cb, cum, s0, k - s0});
+    cum += chunk[c];
   }
+  const uint32_t placed = k;
+  std::vector<uint64_t> pos(num_samples);
+  HS_TRY(sample_chunks(st->amp, st->dtype, cb, touched, u, pos.data(), nullptr));
+  for (k = 0; k < placed; ++k)
+    for (int j = 0; j < num_qubits; ++j)
+      out[size_t(k) * num_qubits + j] = int32_t((pos[k] >> slots[j]) & 1);
   // samples beyond the accumulated mass read as all ones (state_vector.hpp:969-978)
   for (; k < num_samples; ++k)
     for (int j = 0; j < num_qubits; ++j) out[size_t(k) * num_qubits + j] = 1;

@@ -349,6 +349,20 @@ int reduce_zz(const void* amp, int dtype, int n, const int32_t* slot_pairs, int 
               double* out, cudaStream_t s);
 int reduce_chunks(const void* amp, int dtype, int n, int chunk_bits, double* host_out,
                   cudaStream_t s);
+// frees the reductions' kept scratch blocks of device `dev` (its last state is gone)
+void scratch_release(int dev);
+// a chunk of amplitudes with samples: its first amplitude, the mass before it,
+// its samples [s0, s0 + ns) of the sorted sample points
+struct MeasureChunk {
+  uint64_t first;
+  double base;
+  uint32_t s0, ns;
+};
+// pos[k] = amplitude where the cumulative distribution passes u[k], for the
+// samples of the listed chunks (u and pos hold every sample)
+int sample_chunks(const void* amp, int dtype, int chunk_bits,
+                  const std::vector<MeasureChunk>& chunks, const std::vector<double>& u,
+                  uint64_t* pos, cudaStream_t s);
 int set_basis_kernel(void* amp, int dtype, int n, uint64_t index, cudaStream_t s);
 // out[j] = in[offset | deposit(j, old_slots)] for j < 2^out_bits
 int project_kernel(const void* in, void* out, int dtype, int out_bits, const int* old_slots,
@@ -411,5 +425,6 @@ struct hs_state {
   int n = 0;
   int dtype = HS_DTYPE_C128;
   void* amp = nullptr;  // device, slot-ordered
+  int dev = 0;          // the device it was created on
   std::vector<int> q2s, s2q;
 };

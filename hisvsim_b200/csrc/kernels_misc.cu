@@ -1,6 +1,7 @@
 // K2 (in-place bit-swap permutation), K3 (FP64 reductions) and small
 // elementwise kernels (basis-state set, dtype conversion).
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "bounds.cuh"
@@ -10,6 +11,62 @@ namespace hisv {
 namespace {
 
 int num_sms() { return device_sms(); }
+
+// Scratch of one reduction call.  Blocks of kScratchBlock bytes are kept per
+// device (at most kScratchKept) and handed to one call at a time; a call gives
+// its block back after it has synchronised its stream, so a block is idle
+// whenever it changes hands, whatever the threads and streams.  Allocating from
+// a stream-ordered pool instead costs 0.45 ms per call that synchronises,
+// whatever the size of the state.  The blocks are freed with the device's last
+// state (scratch_release); larger requests are allocated for the call.
+constexpr size_t kScratchBlock = 1ull << 20;
+constexpr size_t kScratchKept = 4;
+
+std::mutex g_scratch_mu;
+std::vector<void*> g_scratch[64];
+
+class Scratch {
+ public:
+  ~Scratch() {
+    if (!p_) return;
+    if (idle_ && block_) {
+      std::lock_guard<std::mutex> lk(g_scratch_mu);
+      if (g_scratch[dev_].size() < kScratchKept) {
+        g_scratch[dev_].push_back(p_);
+        return;
+      }
+    }
+    cudaFree(p_);
+  }
+  int get(size_t bytes) {
+    HS_CUDA(cudaGetDevice(&dev_));
+    block_ = bytes <= kScratchBlock && dev_ >= 0 && dev_ < 64;
+    if (block_) {
+      std::lock_guard<std::mutex> lk(g_scratch_mu);
+      g_scratch[dev_].reserve(kScratchKept);
+      if (!g_scratch[dev_].empty()) {
+        p_ = g_scratch[dev_].back();
+        g_scratch[dev_].pop_back();
+        return HS_OK;
+      }
+    }
+    HS_CUDA(cudaMalloc(&p_, block_ ? kScratchBlock : bytes));
+    return HS_OK;
+  }
+  // waits for the call's work; what is left behind may then be handed on
+  cudaError_t finish(cudaStream_t s) {
+    const cudaError_t e = cudaStreamSynchronize(s);
+    idle_ = e == cudaSuccess;
+    return e;
+  }
+  double* doubles() const { return static_cast<double*>(p_); }
+  char* bytes() const { return static_cast<char*>(p_); }
+
+ private:
+  void* p_ = nullptr;
+  int dev_ = 0;
+  bool block_ = false, idle_ = false;
+};
 
 // ---- K2 -------------------------------------------------------------------
 // Replaces the MPI redistribution (gather_slots, mpi_redistributer.hpp:265-344)
@@ -81,13 +138,13 @@ __device__ __forceinline__ double block_max(double x, double* sh) {
   return r;
 }
 
-enum RedKind { RED_NORM = 0, RED_PROB0 = 1, RED_ZZ = 2, RED_INNER = 3, RED_MAXDIFF = 4 };
+enum RedKind { RED_NORM = 0, RED_INNER = 3, RED_MAXDIFF = 4 };
 
 // partial[k * gridDim.x + blockIdx.x] for k < nout
 template <typename V>
 __global__ void __launch_bounds__(kRedThreads) k3_reduce(const V* __restrict__ a,
                                                          const V* __restrict__ b, uint64_t size,
-                                                         int kind, uint64_t m1, uint64_t m2,
+                                                         int kind,
                                                          double* __restrict__ partial) {
   __shared__ double sh[kRedThreads / 32];
   double s0 = 0, s1 = 0;
@@ -96,12 +153,6 @@ __global__ void __launch_bounds__(kRedThreads) k3_reduce(const V* __restrict__ a
     const double2 u = ld2(a, i);
     if (kind == RED_NORM) {
       s0 += u.x * u.x + u.y * u.y;
-    } else if (kind == RED_PROB0) {
-      if (!(i & m1)) s0 += u.x * u.x + u.y * u.y;
-    } else if (kind == RED_ZZ) {
-      const double p = u.x * u.x + u.y * u.y;
-      const bool odd = (__popcll(i & m1) + __popcll(i & m2)) & 1;
-      s0 += odd ? -p : p;
     } else if (kind == RED_INNER) {
       const double2 w = ld2(b, i);  // conj(u) * w
       s0 += u.x * w.x + u.y * w.y;
@@ -125,6 +176,23 @@ __global__ void __launch_bounds__(kRedThreads) k3_reduce(const V* __restrict__ a
   }
 }
 
+// mass of the amplitudes with bit `slot` clear: only those are read (half of
+// the state where the slot is above the 128-byte line)
+template <typename V>
+__global__ void __launch_bounds__(kRedThreads) k3_prob0(const V* __restrict__ a, uint64_t half,
+                                                        int slot, double* __restrict__ partial) {
+  __shared__ double sh[kRedThreads / 32];
+  double s = 0;
+  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x, low = (1ull << slot) - 1;
+#pragma unroll 4
+  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < half; j += stride) {
+    const double2 u = ld2(a, ((j & ~low) << 1) | (j & low));
+    s += u.x * u.x + u.y * u.y;
+  }
+  const double r = block_sum(s, sh);
+  if (threadIdx.x == 0) partial[blockIdx.x] = r;
+}
+
 __global__ void k3_finish(const double* __restrict__ partial, int nblocks, int kind,
                           double* __restrict__ out) {
   __shared__ double sh[kRedThreads / 32];
@@ -141,23 +209,21 @@ __global__ void k3_finish(const double* __restrict__ partial, int nblocks, int k
 }
 
 template <typename V>
-int run_reduce(const void* a, const void* b, int n, int kind, uint64_t m1, uint64_t m2,
-               double out[2], cudaStream_t s) {
+int run_reduce(const void* a, const void* b, int n, int kind, double out[2], cudaStream_t s) {
   const uint64_t size = 1ull << n;
   const int blocks = int(std::min<uint64_t>(kRedBlocks, (size + kRedThreads - 1) / kRedThreads));
-  double* scratch = nullptr;  // [2*blocks partials | 2 results]
-  HS_CUDA(cudaMallocAsync(&scratch, sizeof(double) * (2 * blocks + 2), s));
+  Scratch sc;  // [2*blocks partials | 2 results]
+  HS_TRY(sc.get(sizeof(double) * (2 * blocks + 2)));
+  double* scratch = sc.doubles();
   k3_reduce<V><<<blocks, kRedThreads, 0, s>>>(static_cast<const V*>(a),
-                                               static_cast<const V*>(b), size, kind, m1, m2,
-                                               scratch);
+                                               static_cast<const V*>(b), size, kind, scratch);
   k3_finish<<<1, kRedThreads, 0, s>>>(scratch, blocks, kind, scratch + 2 * blocks);
   cudaError_t e1 = cudaGetLastError();
   double host[2] = {0, 0};
   cudaError_t e2 = cudaMemcpyAsync(host, scratch + 2 * blocks, sizeof(host),
                                    cudaMemcpyDeviceToHost, s);
-  cudaError_t e3 = cudaFreeAsync(scratch, s);
-  cudaError_t e4 = cudaStreamSynchronize(s);
-  for (cudaError_t e : {e1, e2, e3, e4})
+  cudaError_t e3 = sc.finish(s);
+  for (cudaError_t e : {e1, e2, e3})
     if (e != cudaSuccess)
       return set_error(HS_E_CUDA, "reduction: %s", cudaGetErrorString(e));
   out[0] = host[0];
@@ -165,10 +231,172 @@ int run_reduce(const void* a, const void* b, int n, int kind, uint64_t m1, uint6
   return HS_OK;
 }
 
-int reduce_any(const void* a, const void* b, int dtype, int n, int kind, uint64_t m1,
-               uint64_t m2, double out[2], cudaStream_t s) {
-  if (dtype == HS_DTYPE_C128) return run_reduce<double2>(a, b, n, kind, m1, m2, out, s);
-  return run_reduce<float2>(a, b, n, kind, m1, m2, out, s);
+int reduce_any(const void* a, const void* b, int dtype, int n, int kind, double out[2],
+               cudaStream_t s) {
+  if (dtype == HS_DTYPE_C128) return run_reduce<double2>(a, b, n, kind, out, s);
+  return run_reduce<float2>(a, b, n, kind, out, s);
+}
+
+// <Z_i Z_j> of up to kZzPairs pairs in one pass over the state.  The sign of
+// amplitude x for pair q is bit q of a word that is linear over GF(2) in x
+// (bit b of x adds word[b]).  A thread takes 16 amplitudes per chunk of 2^12
+// (x = chunk, 4 bits, 8 thread bits), turns their probabilities into the 11
+// signed sums over at most two of the 4 bits, and adds to pair q's accumulator
+// the sum of the bits that the pair has among the 4, with the sign the other
+// bits give: 1/16 of an addition per amplitude and pair instead of one, which
+// keeps the pass bound by HBM.  28 pairs at 2^28 complex128 amplitudes: one
+// read of the state instead of 28.
+constexpr int kZzPairs = 32;
+constexpr int kZzRegBits = 4;
+
+struct ZzParams {
+  uint32_t word[64];         // pairs that contain slot b
+  uint8_t sum[kZzPairs];     // row of the pair's sum in shared memory
+  int32_t npairs;
+};
+
+// row of the sum over mask (a subset of the 4 register bits of at most two)
+__host__ __device__ constexpr int zz_row(int mask) {
+  constexpr int row[16] = {0, 1, 2, 5, 3, 6, 7, 0, 4, 8, 9, 0, 10, 0, 0, 0};
+  return row[mask];
+}
+constexpr int kZzRows = 11;
+
+template <typename V>
+__global__ void __launch_bounds__(kRedThreads, 2)
+    k3_zz(const V* __restrict__ a, uint64_t size, const __grid_constant__ ZzParams P,
+          double* __restrict__ partial) {
+  __shared__ double sums[kZzRows][kRedThreads];
+  __shared__ double sh[kRedThreads / 32];
+  constexpr int K = 1 << kZzRegBits;
+  const int t = threadIdx.x;
+  uint32_t wt = 0;  // sign word of the thread bits
+  for (int b = 0; b < 8; ++b)
+    if ((t >> b) & 1) wt ^= P.word[b];
+  double acc[kZzPairs];
+#pragma unroll
+  for (int q = 0; q < kZzPairs; ++q) acc[q] = 0;
+  const uint64_t nchunks = (size + K * kRedThreads - 1) / (K * kRedThreads);
+  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+    double p[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint64_t i = c * (K * kRedThreads) + uint64_t(k) * kRedThreads + t;
+      p[k] = 0;
+      if (i < size) {
+        const double2 u = ld2(a, i);
+        p[k] = u.x * u.x + u.y * u.y;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < K; ++m) {  // sums over the signs of the bits in m
+      if (m != 0 && zz_row(m) == 0) continue;
+      double s = 0;
+#pragma unroll
+      for (int k = 0; k < K; ++k) s += (__popc(k & m) & 1) ? -p[k] : p[k];
+      sums[zz_row(m)][t] = s;  // read by this thread alone
+    }
+    uint32_t w = wt;
+    for (int b = 12; (c >> (b - 12)) != 0; ++b)
+      if ((c >> (b - 12)) & 1ull) w ^= P.word[b];
+#pragma unroll
+    for (int q = 0; q < kZzPairs; ++q) {
+      const double s = sums[P.sum[q]][t];
+      acc[q] += __hiloint2double(__double2hiint(s) ^ int((w << (31 - q)) & 0x80000000u),
+                                 __double2loint(s));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kZzPairs; ++q) {
+    const double r = block_sum(acc[q], sh);
+    if (t == 0) partial[size_t(q) * gridDim.x + blockIdx.x] = r;
+  }
+}
+
+// block q adds row q of the partials in a fixed order
+__global__ void __launch_bounds__(kRedThreads)
+    k3_rows(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
+  __shared__ double sh[kRedThreads / 32];
+  double s = 0;
+  for (int i = threadIdx.x; i < nblocks; i += kRedThreads)
+    s += partial[size_t(blockIdx.x) * nblocks + i];
+  const double r = block_sum(s, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = r;
+}
+
+// Samples: the amplitude at which the cumulative distribution, starting from
+// `base` at the first amplitude of the sample's chunk, passes u.
+struct SampleChunk {
+  uint64_t first;      // first amplitude of the chunk
+  double base;         // mass before it
+  uint32_t s0, ns;     // its samples in u / pos
+};
+
+// One block per chunk with samples.  The chunk (2^chunk_bits amplitudes) is cut
+// into up to 256 runs; the warps sum the runs, one warp scans the run sums, and
+// each sample's warp then walks its run in steps of 32 amplitudes.  A sample
+// that the rounding of the sums leaves beyond the chunk takes the chunk's last
+// amplitude of non-zero probability.
+template <typename V>
+__global__ void __launch_bounds__(kRedThreads)
+    k3_sample(const V* __restrict__ a, int chunk_bits, const SampleChunk* __restrict__ chunks,
+              const double* __restrict__ u, uint64_t* __restrict__ pos) {
+  __shared__ double run[kRedThreads];  // sums, then the mass up to and including each run
+  const SampleChunk C = chunks[blockIdx.x];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kRedThreads / 32;
+  const int run_bits = chunk_bits > 8 ? chunk_bits - 8 : 0;
+  const int nruns = 1 << (chunk_bits - run_bits), len = 1 << run_bits;
+  const V* base = a + C.first;
+  auto prob = [&](int i) {
+    const double2 v = ld2(base, uint64_t(i));
+    return v.x * v.x + v.y * v.y;
+  };
+  for (int r = warp; r < nruns; r += nw) {
+    double s = 0;
+    for (int i = lane; i < len; i += 32) s += prob(r * len + i);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) run[r] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double cum = C.base;
+    for (int r = 0; r < nruns; ++r) {
+      cum += run[r];
+      run[r] = cum;
+    }
+  }
+  __syncthreads();
+  for (uint32_t k = warp; k < C.ns; k += nw) {
+    const double x = u[C.s0 + k];
+    int lo = 0, hi = nruns - 1;  // first run whose end passes x
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (x < run[mid]) hi = mid; else lo = mid + 1;
+    }
+    double cum = lo ? run[lo - 1] : C.base;
+    int found = -1, last = -1;
+    for (int i0 = lo * len; i0 < nruns * len && found < 0; i0 += 32) {
+      const int i = i0 + lane;
+      const double p = i < nruns * len ? prob(i) : 0.0;
+      double s = p;  // inclusive scan over the warp
+      for (int o = 1; o < 32; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += v;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, p > 0.0 && x < cum + s);
+      const uint32_t some = __ballot_sync(0xffffffffu, p > 0.0);
+      if (hit) found = i0 + __ffs(int(hit)) - 1;
+      if (some) last = i0 + 31 - __clz(int(some));
+      cum += __shfl_sync(0xffffffffu, s, 31);
+    }
+    // beyond the chunk's mass: its last amplitude of non-zero probability
+    for (int i1 = lo * len; found < 0 && last < 0 && i1 > 0; i1 -= 32) {
+      const int i = i1 - 32 + lane;
+      const uint32_t some = __ballot_sync(0xffffffffu, i >= 0 && prob(i < 0 ? 0 : i) > 0.0);
+      if (some) last = i1 - 1 - __clz(int(some));
+    }
+    if (lane == 0) pos[C.s0 + k] = C.first + uint64_t(found >= 0 ? found : last >= 0 ? last : 0);
+  }
 }
 
 // per-chunk probability mass: block b sums |a_i|^2 over chunk b (fixed order)
@@ -259,22 +487,29 @@ __global__ void k3_compare_finish(const double* __restrict__ partial, int nblock
 template <typename VA, typename VB>
 int run_compare(const void* a, const void* b, uint64_t size, double out[4], cudaStream_t s) {
   const int blocks = int(std::min<uint64_t>(kRedBlocks, (size + kRedThreads - 1) / kRedThreads));
-  double* scratch = nullptr;
-  HS_CUDA(cudaMallocAsync(&scratch, sizeof(double) * (4 * blocks + 4), s));
+  Scratch sc;
+  HS_TRY(sc.get(sizeof(double) * (4 * blocks + 4)));
+  double* scratch = sc.doubles();
   k3_compare<VA, VB><<<blocks, kRedThreads, 0, s>>>(static_cast<const VA*>(a),
                                                     static_cast<const VB*>(b), size, scratch);
   k3_compare_finish<<<1, kRedThreads, 0, s>>>(scratch, blocks, scratch + 4 * blocks);
   cudaError_t e1 = cudaGetLastError();
   cudaError_t e2 = cudaMemcpyAsync(out, scratch + 4 * blocks, 4 * sizeof(double),
                                    cudaMemcpyDeviceToHost, s);
-  cudaError_t e3 = cudaFreeAsync(scratch, s);
-  cudaError_t e4 = cudaStreamSynchronize(s);
-  for (cudaError_t e : {e1, e2, e3, e4})
+  cudaError_t e3 = sc.finish(s);
+  for (cudaError_t e : {e1, e2, e3})
     if (e != cudaSuccess) return set_error(HS_E_CUDA, "compare: %s", cudaGetErrorString(e));
   return HS_OK;
 }
 
 }  // namespace
+
+void scratch_release(int dev) {
+  if (dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  for (void* p : g_scratch[dev]) cudaFree(p);
+  g_scratch[dev].clear();
+}
 
 int reduce_compare(const void* a, int adtype, const void* b, int bdtype, int n, double out[4],
                    cudaStream_t s) {
@@ -295,8 +530,9 @@ int reduce_compare_count(const void* a, int adtype, const void* b, int bdtype, u
 int reduce_chunks(const void* amp, int dtype, int n, int chunk_bits, double* host_out,
                   cudaStream_t s) {
   const uint64_t nchunks = 1ull << (n - chunk_bits);
-  double* scratch = nullptr;
-  HS_CUDA(cudaMallocAsync(&scratch, sizeof(double) * nchunks, s));
+  Scratch sc;
+  HS_TRY(sc.get(sizeof(double) * nchunks));
+  double* scratch = sc.doubles();
   if (dtype == HS_DTYPE_C128)
     k3_chunks<double2><<<unsigned(nchunks), kRedThreads, 0, s>>>(
         static_cast<const double2*>(amp), chunk_bits, scratch);
@@ -306,9 +542,8 @@ int reduce_chunks(const void* amp, int dtype, int n, int chunk_bits, double* hos
   cudaError_t e1 = cudaGetLastError();
   cudaError_t e2 = cudaMemcpyAsync(host_out, scratch, sizeof(double) * nchunks,
                                    cudaMemcpyDeviceToHost, s);
-  cudaError_t e3 = cudaFreeAsync(scratch, s);
-  cudaError_t e4 = cudaStreamSynchronize(s);
-  for (cudaError_t e : {e1, e2, e3, e4})
+  cudaError_t e3 = sc.finish(s);
+  for (cudaError_t e : {e1, e2, e3})
     if (e != cudaSuccess) return set_error(HS_E_CUDA, "chunk sums: %s", cudaGetErrorString(e));
   return HS_OK;
 }
@@ -471,39 +706,114 @@ int launch_permute(void* amp, int dtype, int n, const int32_t* pairs, int npairs
 
 int reduce_norm2(const void* amp, int dtype, int n, double* out, cudaStream_t s) {
   double r[2];
-  HS_TRY(reduce_any(amp, amp, dtype, n, RED_NORM, 0, 0, r, s));
+  HS_TRY(reduce_any(amp, amp, dtype, n, RED_NORM, r, s));
   *out = r[0];
   return HS_OK;
 }
 
 int reduce_inner(const void* a, const void* b, int dtype, int n, double out[2],
                  cudaStream_t s) {
-  return reduce_any(a, b, dtype, n, RED_INNER, 0, 0, out, s);
+  return reduce_any(a, b, dtype, n, RED_INNER, out, s);
 }
 
 int reduce_maxdiff(const void* a, const void* b, int dtype, int n, double* out,
                    cudaStream_t s) {
   double r[2];
-  HS_TRY(reduce_any(a, b, dtype, n, RED_MAXDIFF, 0, 0, r, s));
+  HS_TRY(reduce_any(a, b, dtype, n, RED_MAXDIFF, r, s));
   *out = r[0];
   return HS_OK;
 }
 
 int reduce_prob0(const void* amp, int dtype, int n, int slot, double* out, cudaStream_t s) {
-  double r[2];
-  HS_TRY(reduce_any(amp, amp, dtype, n, RED_PROB0, 1ull << slot, 0, r, s));
-  *out = r[0];
+  const uint64_t half = 1ull << (n - 1);
+  const int blocks = int(std::min<uint64_t>(kRedBlocks, (half + kRedThreads - 1) / kRedThreads));
+  Scratch sc;  // [partials | result]
+  HS_TRY(sc.get(sizeof(double) * (blocks + 1)));
+  double* scratch = sc.doubles();
+  if (dtype == HS_DTYPE_C128)
+    k3_prob0<double2><<<blocks, kRedThreads, 0, s>>>(static_cast<const double2*>(amp), half, slot,
+                                                     scratch);
+  else
+    k3_prob0<float2><<<blocks, kRedThreads, 0, s>>>(static_cast<const float2*>(amp), half, slot,
+                                                    scratch);
+  k3_rows<<<1, kRedThreads, 0, s>>>(scratch, blocks, scratch + blocks);
+  const cudaError_t e1 = cudaGetLastError();
+  const cudaError_t e2 =
+      cudaMemcpyAsync(out, scratch + blocks, sizeof(double), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e3 = sc.finish(s);
+  for (cudaError_t e : {e1, e2, e3})
+    if (e != cudaSuccess) return set_error(HS_E_CUDA, "reduction: %s", cudaGetErrorString(e));
   return HS_OK;
 }
 
+namespace {
+template <typename V>
+int run_zz(const void* amp, int n, const int32_t* pairs, int np, double* out, cudaStream_t s) {
+  const uint64_t size = 1ull << n;
+  const uint64_t nchunks = (size + 16 * kRedThreads - 1) / (16 * kRedThreads);
+  const int blocks = int(std::min<uint64_t>(2 * uint64_t(num_sms()), nchunks));
+  Scratch sc;  // [pair][block] partials, then the results
+  HS_TRY(sc.get(sizeof(double) * size_t(kZzPairs) * (blocks + 1)));
+  double* scratch = sc.doubles();
+  double* res = scratch + size_t(kZzPairs) * blocks;
+  cudaError_t e = cudaSuccess;
+  for (int first = 0; first < np && e == cudaSuccess; first += kZzPairs) {
+    ZzParams P{};
+    P.npairs = std::min(kZzPairs, np - first);
+    for (int q = 0; q < P.npairs; ++q) {
+      uint64_t m = 0;  // a pair of one slot twice is the identity
+      for (int k = 0; k < 2; ++k) m ^= 1ull << pairs[2 * (first + q) + k];
+      for (int b = 0; b < 64; ++b)
+        if ((m >> b) & 1ull) P.word[b] |= 1u << q;
+      P.sum[q] = uint8_t(zz_row(int(m >> 8) & 15));
+    }
+    for (int b = 8; b < 12; ++b) P.word[b] = 0;  // signs inside the sums
+    k3_zz<V><<<blocks, kRedThreads, 0, s>>>(static_cast<const V*>(amp), size, P, scratch);
+    k3_rows<<<P.npairs, kRedThreads, 0, s>>>(scratch, blocks, res);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out + first, res, sizeof(double) * P.npairs, cudaMemcpyDeviceToHost, s);
+  }
+  const cudaError_t e2 = sc.finish(s);
+  for (cudaError_t x : {e, e2})
+    if (x != cudaSuccess) return set_error(HS_E_CUDA, "reduction: %s", cudaGetErrorString(x));
+  return HS_OK;
+}
+}  // namespace
+
 int reduce_zz(const void* amp, int dtype, int n, const int32_t* slot_pairs, int npairs,
               double* out, cudaStream_t s) {
-  for (int i = 0; i < npairs; ++i) {
-    double r[2];
-    HS_TRY(reduce_any(amp, amp, dtype, n, RED_ZZ, 1ull << slot_pairs[2 * i],
-                      1ull << slot_pairs[2 * i + 1], r, s));
-    out[i] = r[0];
-  }
+  if (npairs <= 0) return HS_OK;
+  if (dtype == HS_DTYPE_C128) return run_zz<double2>(amp, n, slot_pairs, npairs, out, s);
+  return run_zz<float2>(amp, n, slot_pairs, npairs, out, s);
+}
+
+int sample_chunks(const void* amp, int dtype, int chunk_bits,
+                  const std::vector<MeasureChunk>& chunks, const std::vector<double>& u,
+                  uint64_t* pos, cudaStream_t s) {
+  static_assert(sizeof(SampleChunk) == sizeof(MeasureChunk), "chunk layout");
+  if (chunks.empty()) return HS_OK;
+  const size_t cb = sizeof(SampleChunk) * chunks.size(), ub = sizeof(double) * u.size();
+  Scratch sc;  // [chunks | u | positions]
+  HS_TRY(sc.get(cb + 2 * ub));
+  char* scratch = sc.bytes();
+  auto* dc = reinterpret_cast<SampleChunk*>(scratch);
+  auto* du = reinterpret_cast<double*>(scratch + cb);
+  auto* dp = reinterpret_cast<uint64_t*>(scratch + cb + ub);
+  cudaError_t e[5];
+  e[0] = cudaMemcpyAsync(dc, chunks.data(), cb, cudaMemcpyHostToDevice, s);
+  e[1] = cudaMemcpyAsync(du, u.data(), ub, cudaMemcpyHostToDevice, s);
+  if (dtype == HS_DTYPE_C128)
+    k3_sample<double2><<<unsigned(chunks.size()), kRedThreads, 0, s>>>(
+        static_cast<const double2*>(amp), chunk_bits, dc, du, dp);
+  else
+    k3_sample<float2><<<unsigned(chunks.size()), kRedThreads, 0, s>>>(
+        static_cast<const float2*>(amp), chunk_bits, dc, du, dp);
+  e[2] = cudaGetLastError();
+  e[3] = cudaMemcpyAsync(pos, dp, ub, cudaMemcpyDeviceToHost, s);
+  e[4] = sc.finish(s);
+  for (cudaError_t x : e)
+    if (x != cudaSuccess) return set_error(HS_E_CUDA, "samples: %s", cudaGetErrorString(x));
   return HS_OK;
 }
 
