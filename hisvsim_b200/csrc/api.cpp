@@ -134,18 +134,31 @@ int permute_positions(hs_state* st, const std::vector<int>& pi, cudaStream_t s) 
   return HS_OK;
 }
 
-int run_lowered(hs_state* st, const std::vector<LoweredGate>& lg, long long ngates,
-                cudaStream_t s) {
-  std::vector<PartProgram> progs;
-  HS_TRY(plan_part(st->n, st->q2s, lg, g_tile_hint.load(), st->dtype, &progs));
-  TimedRegion tr(s);
-  for (const auto& p : progs) {
-    HS_TRY(launch_part(st->amp, st->dtype, p, s));
-    count_pass(p.nops);
-    g_param_bytes += (long long)sizeof(PartProgram);
+int launch_passes(hs_state* st, const std::vector<PlannedPass>& passes, cudaStream_t s) {
+  for (const auto& p : passes) {
+    HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, s)
+                  : launch_part(st->amp, st->dtype, *p.part, s));
+    count_pass(p.nops());
+    g_param_bytes += (long long)p.bytes();
   }
-  (void)ngates;
   return HS_OK;
+}
+
+// plan a gate sequence (frames in and out, applied by the last pass with
+// `flush`) and launch its passes
+int run_lowered(hs_state* st, const std::vector<LoweredGate>& lg, Frames* fr, bool flush,
+                cudaStream_t s) {
+  std::vector<PlannedPass> passes;
+  HS_TRY(plan_passes(st->n, st->q2s, lg, fr, flush, g_tile_hint.load(), st->dtype, &passes));
+  TimedRegion tr(s);
+  return launch_passes(st, passes, s);
+}
+
+// one self-contained part: fresh frames, flushed at the end
+int run_part(hs_state* st, const std::vector<LoweredGate>& lg, cudaStream_t s) {
+  Frames fr;
+  fr.reset(st->n);
+  return run_lowered(st, lg, &fr, true, s);
 }
 
 int lower_all(const hs_state* st, const hs_gate* gates, int num, std::vector<LoweredGate>* out) {
@@ -337,7 +350,7 @@ int hs_gate_apply(hs_state* st, const hs_gate* gate, void* stream) {
   if (!gate) return set_error(HS_E_INVALID, "null gate");
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gate, 1, &lg));
-  return run_lowered(st, lg, 1, S(stream));
+  return run_part(st, lg, S(stream));
 }
 
 int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream) {
@@ -346,7 +359,7 @@ int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream)
   if (num_gates == 0) return HS_OK;
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gates, num_gates, &lg));
-  return run_lowered(st, lg, num_gates, S(stream));
+  return run_part(st, lg, S(stream));
 }
 
 int hs_frames_create(int num_qubits, hs_frames** out) {
@@ -379,30 +392,14 @@ int hs_part_run_carry(hs_state* st, hs_frames* fr, const hs_gate* gates, int num
   if (num_gates == 0) return HS_OK;
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gates, num_gates, &lg));
-  std::vector<PartProgram> progs;
-  HS_TRY(plan_gates(st->n, st->q2s, lg, &fr->fr, false, g_tile_hint.load(), st->dtype, &progs));
-  TimedRegion tr(S(stream));
-  for (const auto& pr : progs) {
-    HS_TRY(launch_part(st->amp, st->dtype, pr, S(stream)));
-    count_pass(pr.nops);
-    g_param_bytes += (long long)sizeof(PartProgram);
-  }
-  return HS_OK;
+  return run_lowered(st, lg, &fr->fr, false, S(stream));
 }
 
 int hs_frames_flush(hs_state* st, hs_frames* fr, void* stream) {
   HS_TRY(check_state(st));
   if (!fr || fr->n != st->n) return set_error(HS_E_INVALID, "frames missing or of another size");
   if (fr->fr.identity()) return HS_OK;
-  std::vector<PartProgram> progs;
-  HS_TRY(plan_gates(st->n, st->q2s, {}, &fr->fr, true, g_tile_hint.load(), st->dtype, &progs));
-  TimedRegion tr(S(stream));
-  for (const auto& pr : progs) {
-    HS_TRY(launch_part(st->amp, st->dtype, pr, S(stream)));
-    count_pass(pr.nops);
-    g_param_bytes += (long long)sizeof(PartProgram);
-  }
-  return HS_OK;
+  return run_lowered(st, {}, &fr->fr, true, S(stream));
 }
 
 int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,
@@ -423,17 +420,8 @@ int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets
   // rotations is carried from part to part and applied by the last one
   Frames fr;
   fr.reset(st->n);
-  std::vector<PartProgram> progs;
-  for (int p = 0; p < num_parts; ++p) {
-    HS_TRY(plan_gates(st->n, st->q2s, all[p], &fr, p == num_parts - 1, g_tile_hint.load(),
-                      st->dtype, &progs));
-    TimedRegion tr(S(stream));
-    for (const auto& pr : progs) {
-      HS_TRY(launch_part(st->amp, st->dtype, pr, S(stream)));
-      count_pass(pr.nops);
-      g_param_bytes += (long long)sizeof(PartProgram);
-    }
-  }
+  for (int p = 0; p < num_parts; ++p)
+    HS_TRY(run_lowered(st, all[p], &fr, p == num_parts - 1, S(stream)));
   return HS_OK;
 }
 
@@ -447,14 +435,14 @@ int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_o
       return set_error(HS_E_INVALID, "part offsets must be non-decreasing");
   // plan every part before the first launch, so that the device never waits
   // for the host between two parts and each event pair brackets one part only
-  std::vector<std::vector<PartProgram>> progs(num_parts);
+  std::vector<std::vector<PlannedPass>> progs(num_parts);
   Frames fr;
   fr.reset(st->n);
   for (int p = 0; p < num_parts; ++p) {
     std::vector<LoweredGate> lg;
     HS_TRY(lower_all(st, gates + part_offsets[p], part_offsets[p + 1] - part_offsets[p], &lg));
-    HS_TRY(plan_gates(st->n, st->q2s, lg, &fr, p == num_parts - 1, g_tile_hint.load(),
-                      st->dtype, &progs[p]));
+    HS_TRY(plan_passes(st->n, st->q2s, lg, &fr, p == num_parts - 1, g_tile_hint.load(),
+                       st->dtype, &progs[p]));
   }
   std::vector<cudaEvent_t> ev(num_parts + 1, nullptr);
   int rc = HS_OK;
@@ -464,10 +452,7 @@ int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_o
   if (rc == HS_OK && cudaEventRecord(ev[0], s) != cudaSuccess)
     rc = set_error(HS_E_CUDA, "event record");
   for (int p = 0; p < num_parts && rc == HS_OK; ++p) {
-    for (const auto& pr : progs[p]) {
-      if ((rc = launch_part(st->amp, st->dtype, pr, s)) != HS_OK) break;
-      count_pass(pr.nops);
-    }
+    rc = launch_passes(st, progs[p], s);
     if (rc == HS_OK && cudaEventRecord(ev[p + 1], s) != cudaSuccess)
       rc = set_error(HS_E_CUDA, "event record");
   }
@@ -611,7 +596,7 @@ int hs_bounds_status(uint32_t* flags, int reset) {
   *flags = 0;
 #ifdef HS_BOUNDS
   HS_CUDA(cudaDeviceSynchronize());
-  *flags = bounds_take_part(reset) | bounds_take_misc(reset) | bounds_take_fused(reset) |
+  *flags = bounds_take_part(reset) | bounds_take_wide(reset) | bounds_take_misc(reset) | bounds_take_fused(reset) |
            bounds_take_batch(reset);
   return HS_OK;
 #else

@@ -33,8 +33,9 @@ __device__ unsigned int g_bounds_flag;  // one per translation unit
 #define HS_IN_BOUNDS(cond, bit) true
 #endif
 
-// the flags of the four kernel files (bounds-checked build only)
+// the flags of the kernel files (bounds-checked build only)
 unsigned bounds_take_part(int reset);
+unsigned bounds_take_wide(int reset);
 unsigned bounds_take_misc(int reset);
 unsigned bounds_take_fused(int reset);
 unsigned bounds_take_batch(int reset);

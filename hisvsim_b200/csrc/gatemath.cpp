@@ -25,24 +25,33 @@ void set2(cplx* m, cplx a, cplx b, cplx c, cplx d) {
   m[3] = d;
 }
 
+// cos, sin and exp(i a) of an angle that is real in all but custom uses: the
+// real functions give the complex ones' values there at a fraction of the cost
+bool is_real(cplx a) { return a.imag() == 0.0; }
+cplx ccos(cplx a) { return is_real(a) ? cplx(std::cos(a.real())) : std::cos(a); }
+cplx csin(cplx a) { return is_real(a) ? cplx(std::sin(a.real())) : std::sin(a); }
+cplx expi(cplx a) {
+  return is_real(a) ? cplx(std::cos(a.real()), std::sin(a.real())) : std::exp(kI * a);
+}
+
 // RX(theta): cos(theta/2), i sin(theta/2) -> [[c, -is], [-is, c]] (basic_gates.hpp:343-363)
 void rx(cplx th, cplx* m) {
-  cplx c = std::cos(th / cplx(2)), is = kI * std::sin(th / cplx(2));
+  const cplx h = th / 2.0, c = ccos(h), is = kI * csin(h);
   set2(m, c, -is, -is, c);
 }
 // RY(theta) -> [[c, -s], [s, c]] (basic_gates.hpp:401-422)
 void ry(cplx th, cplx* m) {
-  cplx c = std::cos(th / cplx(2)), s = std::sin(th / cplx(2));
+  const cplx h = th / 2.0, c = ccos(h), s = csin(h);
   set2(m, c, -s, s, c);
 }
 // RI(theta) -> exp(-i theta/2) * I (basic_gates.hpp:460-478)
 void ri(cplx th, cplx* m) {
-  cplx e = std::exp(-kI * th / cplx(2));
+  const cplx e = expi(-th / 2.0);
   set2(m, e, 0.0, 0.0, e);
 }
 // RZ(theta) == U1 -> diag(exp(-i theta/2), exp(i theta/2)) (basic_gates.hpp:515-535,571)
 void rz(cplx th, cplx* m) {
-  set2(m, std::exp(-kI * th / cplx(2)), 0.0, 0.0, std::exp(kI * th / cplx(2)));
+  set2(m, expi(-th / 2.0), 0.0, 0.0, expi(th / 2.0));
 }
 // *Frac(numerator, power): -pi * numerator / 2^(power-1) with unsigned
 // arithmetic (basic_gates.hpp:732-733; power-1 wraps for power == 0).
@@ -153,7 +162,12 @@ int lower_gate(const hs_gate& g, int num_qubits, LoweredGate* out) {
     }
     case HS_GATE_U3: {  // basic_gates.hpp:1044-1052
       cplx t = param(g, 0), p = param(g, 1), l = param(g, 2);
-      cplx c = std::cos(t / 2.0), s = std::sin(t / 2.0);
+      const cplx c = ccos(t / 2.0), s = csin(t / 2.0);
+      if (is_real(t) && is_real(p) && is_real(l)) {
+        const cplx a = expi((p + l) / 2.0), d = expi((p - l) / 2.0);
+        set2(m, c.real() * std::conj(a), -s.real() * std::conj(d), s.real() * d, c.real() * a);
+        break;
+      }
       set2(m, c * std::cos((-p - l) / 2.0) + kI * c * std::sin((-p - l) / 2.0),
            -s * std::cos((-p + l) / 2.0) + kI * -s * std::sin((-p + l) / 2.0),
            s * std::cos((p - l) / 2.0) + kI * s * std::sin((p - l) / 2.0),

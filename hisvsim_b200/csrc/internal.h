@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <complex>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -178,6 +179,120 @@ struct PartProgram {
 static_assert(sizeof(PartProgram) <= 32000, "kernel parameter space");
 static_assert(kMaxOps <= 256 && kMaxCoef <= 1024, "round packing: 8-bit op indices, 9-bit coefficient pairs");
 
+// ---- wide K1 program (kernels_wide.cu) -----------------------------------------
+// The same pass with 32 amplitudes per thread, for chunks whose gates are
+// rotations, diagonal gates, controlled X and swaps.  A register group is a
+// list of steps; a step holds at most one rotation per register bit and, before
+// its rotations, the diagonal work of the step:
+//   * signs: a pending Z on a register bit under thread / outer conditions (a
+//     CZ across that border) is one bit of a per-thread word z.  A rotation
+//     on the bit commutes with it by negating its shear coefficients
+//     (Z M Z), so the elements are touched once, at the end of the group (or
+//     before a controlled X or swap of the bit: `apply`);
+//   * the phase parts of the rotations and every factor of modulus 1 that
+//     depends on register bits alone (CZ between register bits among them), as
+//     one complex factor per element (a table of 32) instead of one per gate;
+//     (only where that is cheaper: single phase parts stay with their
+//     rotation, single CZ negate their eight elements);
+//   * phase runs: factors with thread / outer conditions that share a register
+//     mask are multiplied up per thread and applied once.
+constexpr int kWideBits = 5;  // register bits: 2^5 amplitudes per thread
+constexpr int kWideMaxTileBits = 12;
+constexpr int kWideMinTileBits = 10;  // CTAs of at least one full warp
+// thread bits: seven, and one to keep WideGroup at 64 bytes with its tables
+// on 16-byte boundaries (uniform vector loads; with 60 bytes a pass takes 2%
+// (rotations) to 13% (complex64, phase runs) longer)
+constexpr int kWideMaxThrBits = 8;
+constexpr int kWideMaxGroups = 32;
+constexpr int kWideMaxSteps = 176;
+constexpr int kWideMaxSigns = 136;
+constexpr int kWideMaxConds = 200;
+constexpr int kWideMaxOps = 200;
+constexpr int kWideMaxCoef = 800;
+constexpr int kWideMaxChunks = 32;  // 16-byte chunks a thread copies per tile
+
+// a step, read as three 64-bit words
+struct alignas(8) WideStep {
+  uint16_t rot[kWideBits];  // register bit j: first coefficient of its rotation, 0 = none
+  uint16_t table;           // first coefficient of the factor table, 0 = none
+  uint16_t first_sign, first_op;
+  uint16_t forms;           // bits 2j, 2j+1: shear form of bit j's rotation (RoundDesc)
+  uint8_t zmask;            // bit j: its phase part follows its coefficient
+  uint8_t apply;            // apply the pending signs before the rotations
+  uint8_t nsigns;
+  uint8_t nruns;            // ops [first_op, +nruns): phase runs and negations, before the rotations
+  uint8_t nperms;           // the next nperms ops: controlled X and swaps, after them
+  uint8_t pad;
+};
+static_assert(sizeof(WideStep) == 24, "WideStep layout");
+
+// z ^= bits where the thread / outer bits cover the masks: bit j a Z on register
+// bit j, bit 5 a sign of the whole thread
+struct WideSign {
+  uint32_t bits, cthr;
+  uint64_t couter;
+};
+struct WideCond {  // factor coef[coef] where the thread / outer bits cover the masks
+  uint32_t cthr, coef;
+  uint64_t couter;
+};
+enum WideCode : uint8_t { wk_run = 0, wk_neg = 1, wk_cx = 2, wk_swap = 3 };
+// index of the register bits a < b among the ten pairs
+constexpr int wide_pair(int a, int b) { return b - 1 + a * (7 - a) / 2; }
+struct WideOp {
+  uint8_t code;
+  uint8_t reg;        // run: register mask; cx: target bit; neg, swap: pair of bits (wide_pair)
+  uint16_t first, n;  // run: its conditions
+  uint16_t coef;      // run: constant factor, 0 = none
+  uint32_t elems;     // cx: elements (target bit 0) whose register controls hold
+  uint32_t cthr;      // cx: thread / outer controls
+  uint64_t couter;
+};
+static_assert(sizeof(WideOp) == 24, "WideOp layout");
+
+struct alignas(16) WideGroup {
+  uint32_t dx[kWideBits];       // shared-memory byte offset of register bit j
+  uint32_t tw[kWideMaxThrBits]; // thread bit b: its tile bit (low half), byte offset (high half)
+  uint16_t first_step, num_steps;
+  uint8_t reg_tbit[kWideBits];
+  uint8_t pad[3];
+};
+static_assert(sizeof(WideGroup) == 64, "WideGroup layout");
+
+struct WideProgram {
+  int32_t n, m;
+  int32_t ngroups, nops, ncoef;
+  int32_t nsteps, nsigns, nconds, nwops;
+  int32_t per_thr;          // chunks a thread copies
+  uint64_t ntiles;
+  Runs tile, outer;
+  uint8_t tile_slot[16];
+  uint8_t fold[16];         // shared-memory layout, as in PartProgram
+  // the tile copy: thread t's chunk k goes from global gthr(t) + gchunk[k] to
+  // shared slot cthr(t) ^ cslot[k] (bytes); both are sums over the thread's bits
+  uint64_t gthr[kWideMaxThrBits], gchunk[kWideMaxChunks];
+  uint32_t cthr[kWideMaxThrBits], cslot[kWideMaxChunks];
+  // the last group's direct store: global offset of thread and register bits
+  uint64_t sthr[kWideMaxThrBits], sreg[kWideBits];
+  WideGroup groups[kWideMaxGroups];
+  WideStep steps[kWideMaxSteps];
+  WideSign signs[kWideMaxSigns];
+  WideCond conds[kWideMaxConds];
+  WideOp ops[kWideMaxOps];
+  // coef[0] is unused (index 0 means none); for complex64 the rotations' and
+  // tables' entries hold two floats, the runs' two doubles
+  double2 coef[kWideMaxCoef];
+};
+static_assert(sizeof(WideProgram) <= 32700, "kernel parameter space");
+
+// One state pass as planned: a PartProgram or a WideProgram.
+struct PlannedPass {
+  std::unique_ptr<PartProgram> part;
+  std::unique_ptr<WideProgram> wide;
+  int nops() const { return wide ? wide->nops : part->nops; }
+  size_t bytes() const { return wide ? sizeof(WideProgram) : sizeof(PartProgram); }
+};
+
 // Pending diagonal of a state under planning: the true state is
 // G * (prod_q diag(1, r[q]) on qubit q) * (the stored amplitudes).  Uncontrolled
 // one-qubit gates are applied as rotations in factored form, and the phases
@@ -202,6 +317,11 @@ struct Frames {
 int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
                Frames* fr, bool flush, int tile_bits_hint, int dtype,
                std::vector<PartProgram>* programs);
+// The same for the device: chunks that qualify become wide programs (use_wide),
+// the others the programs of plan_gates.  Passes without any op are left out.
+int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
+                Frames* fr, bool flush, int tile_bits_hint, int dtype,
+                std::vector<PlannedPass>* passes);
 // one self-contained part: fresh frames, flushed at the end
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
               int tile_bits_hint, int dtype, std::vector<PartProgram>* programs);
@@ -337,6 +457,7 @@ int launch_batch_expect(const BatchInstance* d_inst, int ninst, int max_n, doubl
 
 // ---- launchers (kernels_*.cu) ----------------------------------------------
 int launch_part(void* amp, int dtype, const PartProgram& prog, cudaStream_t s);
+int launch_wide(void* amp, int dtype, const WideProgram& prog, cudaStream_t s);
 int launch_permute(void* amp, int dtype, int n, const int32_t* pairs, int npairs,
                    cudaStream_t s);
 int reduce_norm2(const void* amp, int dtype, int n, double* out, cudaStream_t s);

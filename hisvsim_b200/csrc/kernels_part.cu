@@ -606,7 +606,9 @@ int launch_shape(V* a, const PartProgram& P, cudaStream_t s) {
       case 1: return launch_k1<1, false, true, WIDE>(a, P, s);
       case 2: return launch_k1<2, false, true, WIDE>(a, P, s);
       case 3: return launch_k1<3, false, true, WIDE>(a, P, s);
-      default: return launch_k1<4, false, true, WIDE>(a, P, s);
+      default:
+        // 2^12 tiles of such programs are planned as wide programs
+        if constexpr (!WIDE) return launch_k1<4, false, true, WIDE>(a, P, s);
     }
   }
   if (full) {

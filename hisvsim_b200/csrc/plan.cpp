@@ -8,6 +8,10 @@
 // is the same gather, widened by the three lowest slots so that every global
 // access moves whole 128-byte lines of complex128 (the GPU form of opt_slots,
 // execute.hpp:184-199).
+// Chunks of rotations, diagonal gates, controlled X and swaps become wide
+// programs (32 amplitudes per thread, kernels_wide.cu; plan_wide_chunk below);
+// the rest of this comment is about the others, and about the rewriting that
+// both share.
 // Each tile is held by one CTA: 2^R amplitudes per thread in registers, where
 // R tile bits are "register bits".  A non-diagonal gate's targets must be
 // register bits; consecutive gates whose targets fit in R bits form a group,
@@ -41,8 +45,8 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstddef>
 #include <cstring>
-#include <functional>
 
 #include "internal.h"
 
@@ -95,6 +99,7 @@ bool is_diagonal(const LoweredGate& g) {
 struct Rot {
   bool has_z;        // phase part present (beta != 0)
   double tz, sz;     // shears of the phase: tan(beta/2), sin(beta)
+  cplx b1;           // e^{i beta}
   int form;
   double t, s;
   cplx g0, g1;       // left diagonal
@@ -127,16 +132,16 @@ bool factor_rotation(const cplx* W, bool scaled, Rot* R) {
   const double tol = 1e-12;
   if (!(rho > 0.0) || !std::isfinite(rho)) return false;
   const cplx w1 = W[1] / rho, w3 = W[3] / rho;
-  const double c1 = std::abs(w3), s1 = std::abs(w1);
-  if (std::fabs(c * c + s * s - 1.0) > tol || std::fabs(c1 * c1 + s1 * s1 - 1.0) > tol ||
-      std::abs(std::conj(W[0]) * w1 + std::conj(W[2]) * w3) > tol)
+  if (!(std::fabs(c * c + s * s - 1.0) <= tol) ||
+      !(std::norm(std::conj(W[0]) * w1 + std::conj(W[2]) * w3) <= tol * tol))
     return false;
   cplx a0, a1, b1;
   double cc = c, ss = s;
   if (c > 0.0 && s > 0.0) {
     a0 = W[0] / c;
     a1 = W[2] / s;
-    b1 = c >= s ? w3 / (a1 * c) : -w1 / (a0 * s);
+    // (a0, a1 are of modulus 1: dividing by them is multiplying by the conjugate)
+    b1 = c >= s ? w3 * std::conj(a1) : -w1 * std::conj(a0);
     b1 /= std::abs(b1);
   } else if (c == 0.0) {  // anti-diagonal
     a0 = -w1;
@@ -147,7 +152,9 @@ bool factor_rotation(const cplx* W, bool scaled, Rot* R) {
   } else {
     return false;  // diagonal: handled by the caller
   }
-  // the norms of the rows are 1 to 1e-12; keep the phases unit-modulus
+  // the norms of the rows are 1 to 1e-12; keep the phases unit-modulus (by the
+  // exact modulus: the square root of a norm this close to 1 rounds to 1 and
+  // doubles the state's error)
   a0 /= std::abs(a0);
   a1 /= std::abs(a1);
   const double nrm = std::hypot(cc, ss);
@@ -188,6 +195,7 @@ bool factor_rotation(const cplx* W, bool scaled, Rot* R) {
   // tan(beta/2) = sin(beta) / (1 + cos(beta)), cos(beta) >= 0
   R->tz = R->has_z ? b1.imag() / (1.0 + b1.real()) : 0.0;
   R->sz = R->has_z ? b1.imag() : 0.0;
+  R->b1 = b1;
   return true;
 }
 
@@ -225,6 +233,52 @@ RGate phase_gate(int q, cplx r) {
   return x;
 }
 
+bool is_x(const cplx* m) {
+  return exact(m[0], 0) && exact(m[1], 1) && exact(m[2], 1) && exact(m[3], 0);
+}
+
+// A controlled or two-qubit diagonal gate of unit factors as phases on sets of
+// qubits (one-qubit phases and the global one join the pending diagonal, the
+// others become phase gates): diag(d0, d1) on t under the controls C is d0 on C
+// times d1 / d0 on C and t; a two-target diag takes the four sets of its
+// targets.  False when some factor is not of unit modulus (custom C1, C2).
+bool split_diagonal(const LoweredGate& g, Frames* F, std::vector<RGate>* out) {
+  const int d = g.nt == 1 ? 2 : 4;
+  cplx f[4];
+  for (int i = 0; i < d; ++i) {
+    f[i] = g.m[d * i + i];
+    if (std::fabs(std::norm(f[i]) - 1.0) > 2e-12) return false;
+  }
+  const cplx one(1.0, 0.0);
+  auto over = [&](cplx a, cplx b) { return b == one ? a : a / b; };
+  // factor c on the controls and `nt` of the targets
+  auto put = [&](int nt, int ta, int tb, cplx c) {
+    if (c == one) return;
+    if (g.nc + nt == 0) {
+      F->G *= c;
+    } else if (g.nc + nt == 1) {
+      F->r[nt ? ta : g.controls[0]] *= c;
+    } else {
+      out->push_back(phase_gate(nt ? ta : g.controls[g.nc - 1], c));
+      LoweredGate& x = out->back().g;
+      x.nc = nt ? g.nc : g.nc - 1;
+      for (int i = 0; i < x.nc; ++i) x.controls[i] = g.controls[i];
+      if (nt > 1) x.controls[x.nc++] = tb;
+    }
+  };
+  const int t0 = g.targets[0], t1 = g.targets[1];
+  if (g.nt == 2 && g.nc == HS_MAX_CONTROLS) return false;  // no room for the second target
+  put(0, 0, 0, f[0]);
+  if (g.nt == 1) {
+    put(1, t0, 0, over(f[1], f[0]));
+  } else {  // reference index i = 2*b(t0) + b(t1)
+    put(1, t0, 0, over(f[2], f[0]));
+    put(1, t1, 0, over(f[1], f[0]));
+    put(2, t0, t1, over(f[3] * f[0], f[1] * f[2]));
+  }
+  return true;
+}
+
 RGate flush_gate(Frames* F) {
   RGate x;
   x.kind = RK_FLUSH;
@@ -241,9 +295,16 @@ RGate flush_gate(Frames* F) {
   return x;
 }
 
+// |G| outside 2^+-lim
+bool out_of_range(cplx G, double lim) {
+  const double top = std::ldexp(1.0, int(2 * lim)), g = std::norm(G);
+  return !(g <= top && g * top >= 1.0);
+}
+
 // `scaled`: rotations may leave real scales in the frames (complex128);
-// `lim`: the global factor's scale is flushed once it leaves 2^+-lim.
-void rewrite(const std::vector<LoweredGate>& in, Frames* F, bool scaled, double lim,
+// `lim`: the global factor's scale is flushed once it leaves 2^+-lim; `split`:
+// diagonal gates become phases (split_diagonal), for wide programs.
+void rewrite(const std::vector<LoweredGate>& in, Frames* F, bool scaled, double lim, bool split,
              std::vector<RGate>* out) {
   for (const auto& g : in) {
     if (g.nt == 0) continue;
@@ -276,7 +337,7 @@ void rewrite(const std::vector<LoweredGate>& in, Frames* F, bool scaled, double 
         F->r[q] = 1.0;
       }
       out->push_back(x);
-      if (std::fabs(std::log2(std::abs(F->G))) > lim) {
+      if (out_of_range(F->G, lim)) {
         // bring the stored amplitudes' scale back (one multiply of the state)
         Frames sc;
         sc.G = std::abs(F->G);
@@ -286,6 +347,7 @@ void rewrite(const std::vector<LoweredGate>& in, Frames* F, bool scaled, double 
       continue;
     }
     if (diag) {  // controlled or two-qubit diagonal: commutes with the pending diagonal
+      if (split && split_diagonal(g, F, out)) continue;
       RGate x;
       x.g = g;
       out->push_back(x);
@@ -330,7 +392,8 @@ struct SlotGate {
   bool diag;
   int nt;
   int ts[2];                 // non-diagonal target slots
-  std::vector<int> slots;    // every slot the gate touches (dependencies)
+  uint64_t tmask;            // the same as a mask
+  uint64_t dmask;            // slots it acts on diagonally: controls, diagonal targets
 };
 
 int coef_count(const SlotGate& sg) {
@@ -626,19 +689,18 @@ void build_rounds(PartProgram* P, GroupDesc* gd) {
 // ---- shared-memory layout ----------------------------------------------------
 // Slot s of the tile (16 bytes) sits at s ^ fold(s), fold(s) = XOR over the
 // set bits k of s of fold[k] (3 bits: a move within the 128-byte row).
-uint32_t fold_of(const PartProgram& P, uint32_t s) {
+uint32_t fold_of(const uint8_t* fold, uint32_t s) {
   uint32_t r = 0;
-  for (int k = 0; k < 16; ++k)
-    if ((s >> k) & 1u) r ^= P.fold[k];
+  for (; s; s &= s - 1) r ^= fold[__builtin_ctz(s)];
   return r;
 }
 
 // Byte offset change of setting tile bit tbit (the map is linear over GF(2)).
-uint32_t smem_dx(const PartProgram& P, int tbit, int dtype) {
+uint32_t smem_dx(const uint8_t* fold, int tbit, int dtype) {
   const int sh = dtype == HS_DTYPE_C64 ? 1 : 0;
   const uint32_t b = 1u << tbit;
   const uint32_t slot = b >> sh;
-  return ((slot ^ fold_of(P, slot)) << 4) ^ ((b & ((1u << sh) - 1u)) * uint32_t(amp_bytes(dtype)));
+  return ((slot ^ fold_of(fold, slot)) << 4) ^ ((b & ((1u << sh) - 1u)) * uint32_t(amp_bytes(dtype)));
 }
 
 // Pick fold so that, in every register group, the lanes of one access phase
@@ -649,22 +711,20 @@ uint32_t smem_dx(const PartProgram& P, int tbit, int dtype) {
 // the chunked tile copy (lanes over consecutive slots) is conflict-free too.
 // Small backtracking search, the fixed fold of the earlier layout (bit k >= 3
 // onto bit k mod 3) first; kept when no assignment is found.
-void choose_fold(PartProgram* P, int dtype) {
+// `regs`: bit mask of the register tile bits of each group; fold: 16 entries.
+void choose_fold(uint8_t* fold, int m, int rbits, const std::vector<uint32_t>& regs, int dtype) {
   const int sh = dtype == HS_DTYPE_C64 ? 1 : 0;
-  const int nslot = P->m - sh;
-  const int lane_bits = std::min(dtype == HS_DTYPE_C64 ? 4 : 3, P->m - P->rbits);
-  std::memset(P->fold, 0, sizeof(P->fold));
-  for (int k = 3; k < nslot; ++k) P->fold[k] = uint8_t(1u << (k % 3));
+  const int nslot = m - sh;
+  const int lane_bits = std::min(dtype == HS_DTYPE_C64 ? 4 : 3, m - rbits);
+  std::memset(fold, 0, 16);
+  for (int k = 3; k < nslot; ++k) fold[k] = uint8_t(1u << (k % 3));
   if (lane_bits < 1 || nslot <= 3) return;
   // constraints: the lane tile bits of each group
   std::vector<std::vector<int>> cons;
-  for (int g = 0; g < P->ngroups; ++g) {
+  for (uint32_t reg : regs) {
     std::vector<int> lb;
-    for (int b = 0; b < P->m && int(lb.size()) < lane_bits; ++b) {
-      bool reg = false;
-      for (int j = 0; j < P->rbits; ++j) reg |= P->groups[g].reg_tbit[j] == b;
-      if (!reg) lb.push_back(b);
-    }
+    for (int b = 0; b < m && int(lb.size()) < lane_bits; ++b)
+      if (!((reg >> b) & 1u)) lb.push_back(b);
     cons.push_back(lb);
   }
   auto vec = [&](const uint8_t* F, int tbit) -> uint32_t {
@@ -696,13 +756,13 @@ void choose_fold(PartProgram* P, int dtype) {
     return t;
   };
   uint8_t F[16];
-  std::memcpy(F, P->fold, sizeof(F));
+  std::memcpy(F, fold, sizeof(F));
   bool ok = true;
   for (const auto& c : cons)
     if (!independent(F, c)) ok = false;
   if (ok) return;
   int budget = 20000;
-  std::function<bool(int)> dfs = [&](int k) -> bool {
+  auto dfs = [&](auto& self, int k) -> bool {
     if (--budget < 0) return false;
     if (k >= nslot) return true;
     const uint8_t first = uint8_t(1u << (k % 3));
@@ -715,27 +775,547 @@ void choose_fold(PartProgram* P, int dtype) {
           good = false;
           break;
         }
-      if (good && dfs(k + 1)) return true;
+      if (good && self(self, k + 1)) return true;
     }
     F[k] = first;
     return false;
   };
   // constraints that involve only slot bits 0..2 do not depend on fold
-  if (dfs(3)) std::memcpy(P->fold, F, sizeof(F));
+  if (dfs(dfs, 3)) std::memcpy(fold, F, sizeof(F));
 }
 
 void finish_layout(PartProgram* P, int dtype) {
-  choose_fold(P, dtype);
+  std::vector<uint32_t> regs(P->ngroups, 0);
   for (int g = 0; g < P->ngroups; ++g)
-    for (int j = 0; j < P->rbits; ++j) P->groups[g].dx[j] = smem_dx(*P, P->groups[g].reg_tbit[j], dtype);
+    for (int j = 0; j < P->rbits; ++j) regs[g] |= 1u << P->groups[g].reg_tbit[j];
+  choose_fold(P->fold, P->m, P->rbits, regs, dtype);
+  for (int g = 0; g < P->ngroups; ++g)
+    for (int j = 0; j < P->rbits; ++j)
+      P->groups[g].dx[j] = smem_dx(P->fold, P->groups[g].reg_tbit[j], dtype);
 }
 
-}  // namespace
+// ---- register groups -----------------------------------------------------------
+// A second-level acyclic partition of a chunk: a group takes, in circuit order,
+// every remaining gate whose non-diagonal targets fit the R register bits and
+// that does not have to follow a gate left for a later group.
+void take_group(const std::vector<SlotGate>& sgs, const std::vector<int>& remaining,
+                const std::vector<int>& tbit_of_slot, int R, uint32_t* regs,
+                std::vector<int>* members, std::vector<int>* rest) {
+  uint64_t blocked = 0;  // slots held back by a deferred gate
+  for (int x : remaining) {
+    const SlotGate& g = sgs[x];
+    uint32_t r2 = *regs;
+    for (int i = 0; i < g.nt; ++i) r2 |= 1u << tbit_of_slot[g.ts[i]];
+    if (((g.tmask | g.dmask) & blocked) || __builtin_popcount(r2) > R) {
+      blocked |= g.tmask | g.dmask;
+      rest->push_back(x);
+      continue;
+    }
+    *regs = r2;
+    members->push_back(x);
+  }
+}
 
-int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
-               Frames* fr, bool flush, int tile_bits_hint, int dtype,
-               std::vector<PartProgram>* programs) {
-  programs->clear();
+// The same with the slots' roles told apart (wide programs): a gate acts
+// diagonally on its controls and on every slot of a diagonal gate, and two
+// gates that meet on such slots only commute.  Fewer groups than take_group,
+// whose grouping the cost model's features are counted with.
+void take_group_roles(const std::vector<SlotGate>& sgs, const std::vector<int>& remaining,
+                      const std::vector<int>& tbit_of_slot, int R, uint32_t* regs,
+                      std::vector<int>* members, std::vector<int>* rest) {
+  uint64_t held_t = 0, held_d = 0;  // slots of deferred gates: targets, diagonal roles
+  for (int x : remaining) {
+    const SlotGate& g = sgs[x];
+    uint32_t r2 = *regs;
+    for (int i = 0; i < g.nt; ++i) r2 |= 1u << tbit_of_slot[g.ts[i]];
+    if ((g.tmask & (held_t | held_d)) || (g.dmask & held_t) || __builtin_popcount(r2) > R) {
+      held_t |= g.tmask;
+      held_d |= g.dmask;
+      rest->push_back(x);
+      continue;
+    }
+    *regs = r2;
+    members->push_back(x);
+  }
+}
+
+// ---- wide programs (WideProgram, internal.h) --------------------------------------
+// Whether a state of n qubits runs wide programs where its chunks qualify.
+bool use_wide(int n, int dtype) {
+  return k1_reg_bits(dtype) == kRegBits && n >= kWideMinTileBits;
+}
+
+// Gates a wide program can hold: rotations, flushes, phases, X under any
+// controls, and the plain swap.
+bool wide_gate(const SlotGate& s) {
+  const RGate& r = *s.rg;
+  if (r.kind != RK_MATRIX) return true;
+  if (s.diag) return r.g.nt == 1 && exact(r.g.m[0], 1);
+  if (r.g.nt == 1) return r.g.nc > 0 && is_x(r.g.m);
+  return r.g.nc == 0 && is_swap4(r.g.m);
+}
+
+// A set of a group's ops.
+constexpr int kRecWords = 3;
+struct RecSet {
+  uint64_t w[kRecWords] = {};
+  void add(int i) { w[i >> 6] |= 1ull << (i & 63); }
+  RecSet& operator|=(const RecSet& o) {
+    for (int k = 0; k < kRecWords; ++k) w[k] |= o.w[k];
+    return *this;
+  }
+  RecSet operator|(const RecSet& o) const {
+    RecSet r = *this;
+    return r |= o;
+  }
+  bool within(const RecSet& o) const {
+    for (int k = 0; k < kRecWords; ++k)
+      if (w[k] & ~o.w[k]) return false;
+    return true;
+  }
+};
+
+// An op of a group before it is scheduled.
+struct WideRec {
+  enum Kind { kRot, kNeg, kPhase, kCx, kSwap } kind;
+  uint32_t mask = 0;     // register bits it acts on (a cx's controls included)
+  uint32_t target = 0;   // of these, the ones it acts on non-diagonally
+  int j = 0, jb = 0;
+  uint32_t cthr = 0;     // thread / outer condition
+  uint64_t couter = 0;
+  cplx c{1.0, 0.0};      // kPhase
+  const Rot* rot = nullptr;
+  bool z = false;        // kRot: its phase part is still to be applied
+  bool done = false;
+  bool diag() const { return kind == kNeg || kind == kPhase; }
+  bool uniform() const { return cthr == 0 && couter == 0; }
+};
+
+uint32_t elements_of(uint32_t mask) {  // elements whose register bits cover mask
+  uint32_t w = 0;
+  for (uint32_t e = 0; e < 32; ++e)
+    if ((e & mask) == mask) w |= 1u << e;
+  return w;
+}
+
+void wide_records(const SlotGate& sg, const Layout& L, const std::vector<int>& q2s,
+                  std::vector<WideRec>* out) {
+  const RGate& r = *sg.rg;
+  auto bit = [&](int q, WideRec* w) {  // adds qubit q to the masks
+    uint8_t where, pos;
+    locate(L, q2s[q], &where, &pos);
+    if (where == TW_OUT)
+      w->couter |= 1ull << pos;
+    else if (where == TW_REG)
+      w->mask |= 1u << pos;
+    else
+      w->cthr |= 1u << pos;
+  };
+  auto regpos = [&](int slot) { return L.regpos_of_tbit[(*L.tbit_of_slot)[slot]]; };
+  WideRec w;
+  if (r.kind == RK_FLUSH) {
+    w.kind = WideRec::kPhase;
+    for (size_t i = 0; i < r.flq.size(); ++i) {
+      WideRec x = w;
+      bit(r.flq[i], &x);
+      x.c = r.flr[i];
+      out->push_back(x);
+    }
+    w.c = r.flG;
+    if (w.c != cplx(1.0, 0.0)) out->push_back(w);
+    return;
+  }
+  const LoweredGate& g = r.g;
+  if (r.kind == RK_ROT) {
+    w.kind = WideRec::kRot;
+    w.j = regpos(sg.ts[0]);
+    w.mask = w.target = 1u << w.j;
+    w.rot = &r.rot;
+    w.z = r.rot.has_z;
+  } else if (sg.diag) {
+    for (int i = 0; i < g.nc; ++i) bit(g.controls[i], &w);
+    bit(g.targets[0], &w);
+    w.kind = exact(g.m[3], -1) ? WideRec::kNeg : WideRec::kPhase;
+    w.c = g.m[3];
+  } else if (g.nt == 1) {
+    w.kind = WideRec::kCx;
+    for (int i = 0; i < g.nc; ++i) bit(g.controls[i], &w);
+    w.j = regpos(sg.ts[0]);
+    w.target = 1u << w.j;
+    w.mask |= w.target;
+  } else {
+    w.kind = WideRec::kSwap;
+    const int a = regpos(sg.ts[0]), b = regpos(sg.ts[1]);
+    w.j = std::min(a, b);
+    w.jb = std::max(a, b);
+    w.mask = w.target = 1u << a | 1u << b;
+  }
+  out->push_back(w);
+}
+
+// Schedules a group's ops into steps.  Op b has to follow an earlier op a when
+// they share a register bit on which one of them is not diagonal.  A step runs
+// its diagonal ops (signs, factor table, phase runs), then its rotations, then
+// its controlled X and swaps.  Conditional signs join the thread's sign word as
+// soon as they may; other diagonal ops wait until a step acts on their bits, so
+// that runs with one register mask are shared; the phase parts of every
+// rotation that is next on its bit and the register-only factors of modulus 1
+// join the table of the first step that needs one.  `reserve`: coefficients to
+// be left for the program's later groups.
+int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* G, int reserve) {
+  const int n = int(rec.size()), size = 1 << kWideBits;
+  G->first_step = uint16_t(P->nsteps);
+  // dependencies as bit sets over the ops: the last non-diagonal op on a bit,
+  // and for a non-diagonal op the diagonal ones since (what came before those
+  // follows from them)
+  if (n > kRecWords * 64) return set_error(HS_E_UNSUPPORTED, "%d ops in a group", n);
+  RecSet preds[kRecWords * 64], done{}, diag{};
+  {
+    int last[kWideBits];
+    RecSet since[kWideBits] = {};
+    for (int j = 0; j < kWideBits; ++j) last[j] = -1;
+    for (int b = 0; b < n; ++b) {
+      RecSet p{};
+      for (int j = 0; j < kWideBits; ++j) {
+        if (!((rec[b].mask >> j) & 1u)) continue;
+        if (last[j] >= 0) p.add(last[j]);
+        if ((rec[b].target >> j) & 1u) {
+          p |= since[j];
+          last[j] = b;
+          since[j] = RecSet{};
+        } else {
+          since[j].add(b);
+        }
+      }
+      preds[b] = p;
+      if (rec[b].diag()) diag.add(b);
+    }
+  }
+  int left = n;
+  bool pend_any = false;      // signs wait in the word
+  uint32_t pend = 0;          // register bits they act on
+  auto push_coef = [&](cplx c) {
+    P->coef[P->ncoef].x = c.real();
+    P->coef[P->ncoef].y = c.imag();
+    return P->ncoef++;
+  };
+  auto push_amp_coef = [&](cplx c) {  // in the amplitudes' precision
+    if (dtype == HS_DTYPE_C128) return push_coef(c);
+    const float f[2] = {float(c.real()), float(c.imag())};
+    std::memcpy(&P->coef[P->ncoef], f, sizeof(f));
+    return P->ncoef++;
+  };
+  // a diagonal op may run at the start of this step: everything it follows is done
+  auto available = [&](int i) { return preds[i].within(done); };
+  // a non-diagonal op may run in this step: what it follows is done, or is a
+  // diagonal op that may run at the start of the step (`open`)
+  RecSet open;
+  auto ready = [&](int i) { return preds[i].within(done | open); };
+  // a conditional sign of the thread or of one register bit
+  auto is_sign = [&](int i) {
+    return rec[i].kind == WideRec::kNeg && (rec[i].mask & (rec[i].mask - 1)) == 0 &&
+           !(rec[i].uniform() && rec[i].mask != 0);
+  };
+  // a factor of modulus 1 on register bits alone
+  auto unit = [&](int i) {
+    return rec[i].uniform() && rec[i].mask != 0 && std::fabs(std::norm(rec[i].c) - 1.0) < 1e-12;
+  };
+  auto finish = [&](int i) {
+    rec[i].done = true;
+    done.add(i);
+    --left;
+  };
+  while (left > 0 || pend_any) {
+    if (P->nsteps >= kWideMaxSteps) return set_error(HS_E_UNSUPPORTED, "too many steps in a pass");
+    WideStep& S = P->steps[P->nsteps++];
+    std::memset(&S, 0, sizeof(S));
+    S.first_sign = uint16_t(P->nsigns);
+    S.first_op = uint16_t(P->nwops);
+    open = RecSet{};
+    for (int i = 0; i < n; ++i)
+      if (rec[i].diag() && !rec[i].done && available(i)) open.add(i);
+    // ---- the step's non-diagonal ops
+    int rot[kWideBits];
+    uint32_t touched = 0, moved = 0;  // register bits acted on; by controlled X and swaps
+    std::vector<int> perms;
+    for (int j = 0; j < kWideBits; ++j) {
+      rot[j] = -1;
+      for (int i = 0; i < n; ++i)
+        if (!rec[i].done && rec[i].kind == WideRec::kRot && rec[i].j == j) {
+          if (ready(i)) rot[j] = i;
+          break;
+        }
+      if (rot[j] >= 0) touched |= 1u << j;
+    }
+    for (int i = 0; i < n; ++i) {
+      if (rec[i].done || (rec[i].kind != WideRec::kCx && rec[i].kind != WideRec::kSwap)) continue;
+      RecSet here = done | open;  // the step's rotations and earlier perms run first
+      for (int j = 0; j < kWideBits; ++j)
+        if (rot[j] >= 0) here.add(rot[j]);
+      for (int a : perms) here.add(a);
+      const bool ok = preds[i].within(here);
+      if (ok) {
+        perms.push_back(i);
+        moved |= rec[i].target;
+      }
+    }
+    touched |= moved;
+    const bool last = touched == 0;  // diagonal ops alone are left
+    // ---- diagonal ops
+    std::vector<int> run;
+    for (int i = 0; i < n; ++i) {
+      if (rec[i].done || !rec[i].diag() || !available(i)) continue;
+      if (is_sign(i)) {
+        WideSign& q = P->signs[P->nsigns++];
+        q.bits = rec[i].mask ? rec[i].mask : 32u;
+        q.cthr = rec[i].cthr;
+        q.couter = rec[i].couter;
+        ++S.nsigns;
+        pend_any = true;
+        pend |= rec[i].mask;
+      } else if (last || (rec[i].mask & touched)) {
+        run.push_back(i);
+      }
+    }
+    for (int i = 0; i < n; ++i)  // (after the scan: available() looks at done)
+      if (!rec[i].done && rec[i].diag() && is_sign(i) && available(i)) finish(i);
+    // phase parts: of the rotations next on their bits
+    int zs[kWideBits], nz = 0;
+    bool need = false;
+    for (int j = 0; j < kWideBits; ++j)
+      for (int i = 0; i < n; ++i)
+        if (!rec[i].done && ((rec[i].target >> j) & 1u)) {
+          if (rec[i].kind == WideRec::kRot && rec[i].z) {
+            // nothing non-diagonal on the bit is ahead of it
+            if (preds[i].within(done | diag)) {
+              zs[nz++] = i;
+              need |= rot[j] == i;
+            }
+          }
+          break;
+        }
+    // multiply-adds per amplitude of a table (2^R - 1 complex factors) and of
+    // the same work op by op; a negation counts its integer operations
+    double single = 1.5 * nz;
+    bool any = need;
+    for (int i : run)
+      if (unit(i)) {
+        any = true;
+        const int bits = __builtin_popcount(rec[i].mask);
+        single += rec[i].kind == WideRec::kNeg && bits == 2 ? 0.5 : 4.0 / (1 << bits);
+      }
+    if (any && single > 4.0 * (size - 1) / size &&
+        P->ncoef + size + reserve + 2 * n <= kWideMaxCoef) {
+      cplx f[1 << kWideBits], by_bit[kWideBits];
+      for (auto& x : by_bit) x = 1.0;
+      for (int k = 0; k < nz; ++k) {
+        by_bit[rec[zs[k]].j] = rec[zs[k]].rot->b1;
+        rec[zs[k]].z = false;
+      }
+      f[0] = 1.0;
+      for (int e = 1; e < size; ++e)  // the lowest set bit's factor times the others'
+        f[e] = f[e & (e - 1)] * by_bit[__builtin_ctz(unsigned(e))];
+      for (int i = 0; i < n; ++i) {  // every such factor that may run now
+        if (rec[i].done || !rec[i].diag() || !unit(i) || !available(i)) continue;
+        for (uint32_t e = rec[i].mask; e < uint32_t(size); e = (e + 1) | rec[i].mask)
+          f[e] *= rec[i].c;
+        run.erase(std::remove(run.begin(), run.end(), i), run.end());
+        finish(i);
+      }
+      S.table = uint16_t(P->ncoef);
+      for (int e = 0; e < size; ++e) push_amp_coef(f[e]);
+    }
+    S.apply = pend_any && ((pend & moved) || (last && left == int(run.size())));
+    if (S.apply) {
+      pend_any = false;
+      pend = 0;
+    }
+    // negations of register pairs, then runs, one per register mask
+    for (size_t k = 0; k < run.size();) {
+      const WideRec& x = rec[run[k]];
+      if (x.kind != WideRec::kNeg || !x.uniform() || __builtin_popcount(x.mask) != 2) {
+        ++k;
+        continue;
+      }
+      WideOp& op = P->ops[P->nwops++];
+      std::memset(&op, 0, sizeof(op));
+      op.code = wk_neg;
+      op.reg = uint8_t(wide_pair(__builtin_ctz(x.mask), 31 - __builtin_clz(x.mask)));
+      ++S.nruns;
+      finish(run[k]);
+      run.erase(run.begin() + k);
+    }
+    while (!run.empty()) {
+      WideOp& op = P->ops[P->nwops++];
+      std::memset(&op, 0, sizeof(op));
+      op.code = wk_run;
+      op.reg = uint8_t(rec[run[0]].mask);
+      op.first = uint16_t(P->nconds);
+      cplx c = 1.0;
+      std::vector<int> rest;
+      for (int i : run) {
+        if (rec[i].mask != op.reg) {
+          rest.push_back(i);
+          continue;
+        }
+        if (rec[i].uniform()) {
+          c *= rec[i].c;
+        } else {
+          WideCond& q = P->conds[P->nconds++];
+          q.cthr = rec[i].cthr;
+          q.couter = rec[i].couter;
+          q.coef = uint32_t(push_coef(rec[i].c));
+          ++op.n;
+        }
+        finish(i);
+      }
+      if (c != cplx(1.0, 0.0)) op.coef = uint16_t(push_coef(c));
+      ++S.nruns;
+      run = rest;
+    }
+    for (int j = 0; j < kWideBits; ++j) {
+      if (rot[j] < 0) continue;
+      const Rot& r = *rec[rot[j]].rot;
+      S.forms |= uint16_t(r.form << (2 * j));
+      S.rot[j] = uint16_t(push_amp_coef(cplx(r.t, r.s)));
+      if (rec[rot[j]].z) {
+        S.zmask |= uint8_t(1u << j);
+        push_amp_coef(cplx(r.tz, r.sz));
+      }
+      finish(rot[j]);
+    }
+    for (int i : perms) {
+      WideOp& op = P->ops[P->nwops++];
+      std::memset(&op, 0, sizeof(op));
+      if (rec[i].kind == WideRec::kCx) {
+        op.code = wk_cx;
+        op.reg = uint8_t(rec[i].j);
+        op.elems = elements_of(rec[i].mask & ~rec[i].target);
+      } else {
+        op.code = wk_swap;
+        op.reg = uint8_t(wide_pair(rec[i].j, rec[i].jb));
+      }
+      op.cthr = rec[i].cthr;
+      op.couter = rec[i].couter;
+      ++S.nperms;
+      finish(i);
+    }
+  }
+  G->num_steps = uint16_t(P->nsteps - G->first_step);
+  return HS_OK;
+}
+
+// the shared-memory layout and the copy / store tables
+void finish_wide(WideProgram* P, const std::vector<uint32_t>& regs, int dtype) {
+  const int sh = dtype == HS_DTYPE_C64 ? 1 : 0;
+  const int thr_bits = P->m - kWideBits;
+  choose_fold(P->fold, P->m, kWideBits, regs, dtype);
+  uint64_t slot[kWideMaxTileBits];  // global and shared offset of each tile bit
+  uint32_t off[kWideMaxTileBits];
+  for (int b = 0; b < P->m; ++b) {
+    slot[b] = uint64_t(1) << P->tile_slot[b];
+    off[b] = smem_dx(P->fold, b, dtype);
+  }
+  for (int g = 0; g < P->ngroups; ++g) {
+    WideGroup& G = P->groups[g];
+    for (int j = 0; j < kWideBits; ++j) G.dx[j] = off[G.reg_tbit[j]];
+    int b = 0;
+    for (int tb = 0; tb < P->m; ++tb) {
+      if ((regs[g] >> tb) & 1u) continue;
+      G.tw[b] = 1u << tb | off[tb] << 16;
+      if (g == P->ngroups - 1) P->sthr[b] = slot[tb];
+      ++b;
+    }
+  }
+  const WideGroup& last = P->groups[P->ngroups - 1];
+  for (int j = 0; j < kWideBits; ++j) P->sreg[j] = slot[last.reg_tbit[j]];
+  // chunk c = t + k * threads holds tile indices [c << sh, (c + 1) << sh)
+  P->per_thr = ((1 << P->m) >> sh) >> thr_bits;
+  for (int b = 0; b < thr_bits; ++b) {
+    P->gthr[b] = slot[b + sh];
+    P->cthr[b] = off[b + sh];
+  }
+  P->gchunk[0] = 0;
+  P->cslot[0] = 0;
+  for (int k = 1; k < P->per_thr; ++k) {
+    const int b = __builtin_ctz(unsigned(k)) + sh + thr_bits, rest = k & (k - 1);
+    P->gchunk[k] = P->gchunk[rest] | slot[b];
+    P->cslot[k] = P->cslot[rest] ^ off[b];
+  }
+}
+
+// A chunk (gates [first, last) of sgs, every one a wide_gate) as wide programs:
+// one, or more where its groups outgrow a program.
+int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
+                    const std::vector<SlotGate>& sgs, size_t first, size_t last,
+                    const std::vector<int>& tile, const std::vector<int>& tbit_of_slot,
+                    std::vector<PlannedPass>* passes) {
+  const int m = int(tile.size());
+  WideProgram* P = nullptr;
+  std::vector<uint32_t> regs_of;
+  auto new_program = [&]() {
+    if (P) finish_wide(P, regs_of, dtype);
+    regs_of.clear();
+    passes->emplace_back();
+    passes->back().wide.reset(new WideProgram);
+    P = passes->back().wide.get();
+    // the lists are written entry by entry; only what is read is initialised
+    std::memset(P, 0, offsetof(WideProgram, groups));
+    P->n = n;
+    P->m = m;
+    P->ntiles = 1ull << (n - m);
+    P->ncoef = 1;
+    build_runs(tile, &P->tile);
+    for (int b = 0; b < m; ++b) P->tile_slot[b] = uint8_t(tile[b]);
+    std::vector<int> outer;
+    for (int s = 0; s < n; ++s)
+      if (tbit_of_slot[s] < 0) outer.push_back(s);
+    build_runs(outer, &P->outer);
+  };
+  new_program();
+  std::vector<int> remaining, members, rest;
+  std::vector<WideRec> rec;
+  for (size_t x = first; x < last; ++x) remaining.push_back(int(x));
+  while (!remaining.empty()) {
+    uint32_t rmask = 0;
+    members.clear();
+    rest.clear();
+    rec.clear();
+    take_group_roles(sgs, remaining, tbit_of_slot, kWideBits, &rmask, &members, &rest);
+    if (P->ngroups == kWideMaxGroups) new_program();
+    WideGroup& G = P->groups[P->ngroups++];
+    std::memset(&G, 0, sizeof(G));
+    // free register bits take the highest tile bits, so that the lanes stay on
+    // the low, contiguous slots
+    for (int b = m - 1; b >= 0 && __builtin_popcount(rmask) < kWideBits; --b) rmask |= 1u << b;
+    regs_of.push_back(rmask);
+    Layout L;
+    L.tbit_of_slot = &tbit_of_slot;
+    for (int b = 0, j = 0; b < kMaxTileBits; ++b) {
+      L.regpos_of_tbit[b] = -1;
+      if ((rmask >> b) & 1u) {
+        G.reg_tbit[j] = uint8_t(b);
+        L.regpos_of_tbit[b] = j++;
+      }
+    }
+    for (int x : members) wide_records(sgs[x], L, q2s, &rec);
+    P->nops += int(rec.size());
+    // every later op needs at most two coefficients
+    int reserve = 2;
+    for (int x : rest)
+      reserve += sgs[x].rg->kind == RK_FLUSH ? 2 + 2 * int(sgs[x].rg->flq.size()) : 2;
+    HS_TRY(wide_steps(rec, dtype, P, &G, reserve));
+    remaining.swap(rest);
+  }
+  finish_wide(P, regs_of, dtype);
+  return HS_OK;
+}
+
+// The planner of both program kinds: into `programs` (PartPrograms only) or,
+// with `passes`, as PartPrograms and WidePrograms.
+int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
+                Frames* fr, bool flush, int tile_bits_hint, int dtype,
+                std::vector<PartProgram>* programs, std::vector<PlannedPass>* passes) {
   if (n < 1 || n > 63) return set_error(HS_E_INVALID, "bad qubit count %d", n);
   if (int(fr->r.size()) != n) fr->reset(n);
   std::vector<RGate> rg;
@@ -743,10 +1323,11 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
   // keep the carried scale within a few dozen binary orders (it moves with
   // the scaled rotation forms and non-unitary diagonal gates)
   const double lim = dtype == HS_DTYPE_C64 ? 24.0 : 48.0;
-  rewrite(gates, fr, dtype == HS_DTYPE_C128, lim, &rg);
+  const bool wide = passes && use_wide(n, dtype);
+  rewrite(gates, fr, dtype == HS_DTYPE_C128, lim, wide, &rg);
   if (flush) {
     if (!fr->identity()) rg.push_back(flush_gate(fr));
-  } else if (std::fabs(std::log2(std::abs(fr->G))) > lim) {
+  } else if (out_of_range(fr->G, lim)) {
     Frames scale;
     scale.G = std::abs(fr->G);
     rg.push_back(flush_gate(&scale));
@@ -771,24 +1352,27 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
     SlotGate s;
     s.rg = &r;
     s.nt = 0;
+    s.tmask = s.dmask = 0;
     if (r.kind == RK_FLUSH) {
       s.diag = true;
-      for (int q : r.flq) s.slots.push_back(q2s[q]);
+      for (int q : r.flq) s.dmask |= 1ull << q2s[q];
     } else {
       s.diag = r.kind == RK_MATRIX && is_diagonal(r.g);
       for (int i = 0; i < r.g.nt; ++i) {
-        s.slots.push_back(q2s[r.g.targets[i]]);
-        if (!s.diag) s.ts[s.nt++] = q2s[r.g.targets[i]];
+        const int t = q2s[r.g.targets[i]];
+        if (s.diag) {
+          s.dmask |= 1ull << t;
+        } else {
+          s.tmask |= 1ull << t;
+          s.ts[s.nt++] = t;
+        }
       }
-      for (int i = 0; i < r.g.nc; ++i) s.slots.push_back(q2s[r.g.controls[i]]);
+      for (int i = 0; i < r.g.nc; ++i) s.dmask |= 1ull << q2s[r.g.controls[i]];
     }
-    sgs.push_back(std::move(s));
+    sgs.push_back(s);
   }
-  auto low_union_size = [&](const std::vector<int>& t, int lows) {
-    int extra = 0;
-    for (int s = 0; s < lows; ++s)
-      if (std::find(t.begin(), t.end(), s) == t.end()) ++extra;
-    return int(t.size()) + extra;
+  auto low_union_size = [&](uint64_t t, int lows) {
+    return __builtin_popcountll(t | ((1ull << lows) - 1ull));
   };
   // a chunk only needs the low slots the 16-byte chunk copy requires (slot 0
   // for complex64); where the targets leave room the tile takes all three:
@@ -797,14 +1381,11 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
   size_t gi = 0;
   while (gi < sgs.size()) {
     // ---- chunk: gates whose non-diagonal target slots (+ low slots) fit one tile
-    std::vector<int> tset;
+    uint64_t tset = 0;
     size_t gend = gi;
     int ops = 0, coefs = 0, fls = 0;
     while (gend < sgs.size()) {
-      std::vector<int> t2 = tset;
-      for (int i = 0; i < sgs[gend].nt; ++i)
-        if (std::find(t2.begin(), t2.end(), sgs[gend].ts[i]) == t2.end())
-          t2.push_back(sgs[gend].ts[i]);
+      const uint64_t t2 = tset | sgs[gend].tmask;
       const int cc = coef_count(sgs[gend]);
       const int nops_g = sgs[gend].rg->kind == RK_FLUSH ? 1 + int(sgs[gend].rg->flq.size()) : 1;
       const int nfl_g = sgs[gend].rg->kind == RK_FLUSH ? int(sgs[gend].rg->flq.size()) : 0;
@@ -818,25 +1399,46 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
       ++gend;
     }
     if (gend == gi) return set_error(HS_E_INVALID, "gate does not fit a tile");
+    const bool wide_chunk =
+        wide && std::all_of(sgs.begin() + gi, sgs.begin() + gend, wide_gate);
+    // wide chunks with controlled X or swaps on states beyond the L2 take the
+    // largest tile (CTAs of four warps): 7.35 against 7.97 ms for 8 random
+    // layers of 26 qubits; in the L2, and without them, 2^10 is the faster
+    const bool big = wide_chunk && tile_bits_hint <= 0 && (amp_bytes(dtype) << n) > (128ull << 20) &&
+                     std::any_of(sgs.begin() + gi, sgs.begin() + gend, [](const SlotGate& s) {
+                       return s.rg->kind == RK_MATRIX && !s.diag;
+                     });
     // ---- tile: non-diagonal target slots + lowest slots up to the target size
-    std::vector<int> tile = tset;
-    const int m = std::min(max_tile, std::max(m_target, low_union_size(tset, low_min)));
-    for (int s = 0; s < n && int(tile.size()) < m; ++s)
-      if (std::find(tile.begin(), tile.end(), s) == tile.end()) tile.push_back(s);
-    std::sort(tile.begin(), tile.end());
+    const int m = std::min(max_tile, std::max(big ? kWideMaxTileBits : m_target,
+                                              low_union_size(tset, low_min)));
+    for (int s = 0; s < n && __builtin_popcountll(tset) < m; ++s) tset |= 1ull << s;
+    std::vector<int> tile;
+    for (int s = 0; s < n; ++s)
+      if ((tset >> s) & 1ull) tile.push_back(s);
     const int R = std::min(rbits, m);
     std::vector<int> tbit_of_slot(n, -1);
     for (int i = 0; i < m; ++i) tbit_of_slot[tile[i]] = i;
+    if (wide_chunk && m >= kWideMinTileBits) {
+      HS_TRY(plan_wide_chunk(n, dtype, q2s, sgs, gi, gend, tile, tbit_of_slot, passes));
+      gi = gend;
+      continue;
+    }
     PartProgram* P = nullptr;
     auto new_program = [&]() {
-      programs->emplace_back();
-      P = &programs->back();
+      if (passes) {
+        passes->emplace_back();
+        passes->back().part.reset(new PartProgram);
+        P = passes->back().part.get();
+      } else {
+        programs->emplace_back();
+        P = &programs->back();
+      }
       std::memset(P, 0, sizeof(*P));
       P->n = n;
       P->m = m;
       P->ntiles = 1ull << (n - m);
       P->rbits = R;
-      build_runs(tile, &P->tile);
+        build_runs(tile, &P->tile);
       for (int b = 0; b < m; ++b) P->tile_slot[b] = uint8_t(tile[b]);
       std::vector<int> outer;
       for (int s = 0; s < n; ++s)
@@ -844,54 +1446,21 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
       build_runs(outer, &P->outer);
     };
     new_program();
-    // ---- groups: a second-level acyclic partition of the chunk.  Each group
-    // takes, in circuit order, every remaining gate whose non-diagonal targets
-    // fit the R register bits and none of whose qubits is held by a gate left
-    // for a later group (so every gate still follows all gates it depends on).
-    std::vector<size_t> remaining;
-    for (size_t x = gi; x < gend; ++x) remaining.push_back(x);
+    // ---- groups
+    std::vector<int> remaining;
+    for (size_t x = gi; x < gend; ++x) remaining.push_back(int(x));
     while (!remaining.empty()) {
-      std::vector<int> regs;
-      std::vector<size_t> members, rest;
-      std::vector<int> blocked;  // slots held back by a deferred gate
-      auto touches = [&](const SlotGate& g) {
-        for (int s : g.slots)
-          if (std::find(blocked.begin(), blocked.end(), s) != blocked.end()) return true;
-        return false;
-      };
-      auto block = [&](const SlotGate& g) {
-        for (int s : g.slots) blocked.push_back(s);
-      };
-      for (size_t x : remaining) {
-        const SlotGate& g = sgs[x];
-        if (touches(g)) {
-          block(g);
-          rest.push_back(x);
-          continue;
-        }
-        if (!g.diag) {
-          std::vector<int> r2 = regs;
-          for (int i = 0; i < g.nt; ++i) {
-            const int tb = tbit_of_slot[g.ts[i]];
-            if (std::find(r2.begin(), r2.end(), tb) == r2.end()) r2.push_back(tb);
-          }
-          if (int(r2.size()) > R) {
-            block(g);
-            rest.push_back(x);
-            continue;
-          }
-          regs = r2;
-        }
-        members.push_back(x);
-      }
+      uint32_t rmask = 0;
+      std::vector<int> regs, members, rest;
+      take_group(sgs, remaining, tbit_of_slot, R, &rmask, &members, &rest);
       if (P->ngroups == kMaxGroups) new_program();  // a new pass (rare)
       GroupDesc& gd = P->groups[P->ngroups++];
       std::memset(&gd, 0, sizeof(gd));
       // fill the register set with the highest unused tile bits so that the
       // thread (lane) bits stay on the low, contiguous slots
-      for (int b = m - 1; b >= 0 && int(regs.size()) < R; --b)
-        if (std::find(regs.begin(), regs.end(), b) == regs.end()) regs.push_back(b);
-      std::sort(regs.begin(), regs.end());
+      for (int b = m - 1; b >= 0 && __builtin_popcount(rmask) < R; --b) rmask |= 1u << b;
+      for (int b = 0; b < m; ++b)
+        if ((rmask >> b) & 1u) regs.push_back(b);
       for (int j = 0; j < R; ++j) gd.reg_tbit[j] = uint8_t(regs[j]);
       std::vector<int> thr;
       for (int b = 0; b < m; ++b)
@@ -903,7 +1472,7 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
       for (int j = 0; j < R; ++j) L.regpos_of_tbit[regs[j]] = j;
       gd.first_op = uint16_t(P->nops);
       Emitter E{P, &q2s};
-      for (size_t x : members) {
+      for (int x : members) {
         const SlotGate& sg = sgs[x];
         if (sg.rg->kind == RK_ROT)
           emit_rot(sg, L, E);
@@ -918,8 +1487,33 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
     }
     gi = gend;
   }
-  for (auto& P : *programs) finish_layout(&P, dtype);
+  if (!passes) {
+    for (auto& P : *programs) finish_layout(&P, dtype);
+    return HS_OK;
+  }
+  for (auto& p : *passes)
+    if (p.part) finish_layout(p.part.get(), dtype);
+  // a pass without ops has nothing to do
+  passes->erase(std::remove_if(passes->begin(), passes->end(),
+                               [](const PlannedPass& p) { return p.nops() < 1; }),
+                passes->end());
   return HS_OK;
+}
+
+}  // namespace
+
+int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
+               Frames* fr, bool flush, int tile_bits_hint, int dtype,
+               std::vector<PartProgram>* programs) {
+  programs->clear();
+  return plan_chunks(n, q2s, gates, fr, flush, tile_bits_hint, dtype, programs, nullptr);
+}
+
+int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
+                Frames* fr, bool flush, int tile_bits_hint, int dtype,
+                std::vector<PlannedPass>* passes) {
+  passes->clear();
+  return plan_chunks(n, q2s, gates, fr, flush, tile_bits_hint, dtype, nullptr, passes);
 }
 
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,

@@ -1,0 +1,38 @@
+"""The wide part kernel on the GPU against the oracle: every gate kind it holds
+at the smallest state it takes, odd sizes and every tile size, after a slot
+permutation, and with frames carried from call to call; complex128 <= 1e-12,
+complex64 <= 1e-5."""
+import numpy as np
+import pytest
+
+from hisvsim_b200 import abi, circuits, partition
+from hisvsim_b200.gates import part_offsets, to_records
+from test_k1_wide import _mixed
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,tol", [(abi.C128, 1e-12), (abi.C64, 1e-5)])
+@pytest.mark.parametrize("hint", [0, 10, 11, 12])
+@pytest.mark.parametrize("n", [10, 11, 12, 13, 16, 17])
+def test_wide_passes_match_oracle(port, n, hint, dtype, tol):
+    gates = _mixed(n, 3, n) + circuits.random_u3_cz(n, 3, n)
+    want = port.run(n, to_records(gates))
+    parts = partition.partition_frontier(gates, 8, free_diagonal=True)
+    rec, offs = part_offsets(partition.parts_to_gates(gates, parts))
+    rng = np.random.default_rng(n)
+    prev = abi.set_tile_qubits(hint)
+    try:
+        st = abi.State(n, dtype)
+        st.run_parts(rec, offs)
+        assert np.abs(st.amplitudes() - want).max() <= tol
+        st.set_basis(0)
+        fr = abi.Frames(n)
+        for p in range(len(offs) - 1):
+            st.run_part_carry(fr, rec[offs[p]:offs[p + 1]])
+            if p % 3 == 1:  # the factors follow their qubits
+                st.permute_bits([int(v) for v in rng.permutation(n)[:4]])
+        st.flush(fr)
+        assert np.abs(st.amplitudes() - want).max() <= tol
+    finally:
+        abi.set_tile_qubits(prev)

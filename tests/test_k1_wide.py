@@ -1,0 +1,138 @@
+"""Wide K1 programs on the CPU: the library's planner (plan.cpp) compiled with
+the host emulator tests/emu/k1_wide_emu.cpp, which runs the planned programs as
+the kernel does and range-checks every offset.  Compared with the oracle
+(port.c) over every form of chunk that takes the wide path: each gate kind it
+holds with its bits in registers, threads and outer slots, slot orders, both
+data types, tile sizes from 2^10 to 2^12, carried and flushed frames.
+Tolerances: 1e-12 (complex128) as for every plain form, 1e-5 (complex64)."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from hisvsim_b200 import circuits, partition
+from hisvsim_b200.gates import Gate, part_offsets, to_records
+
+CSRC = os.path.join(ROOT, "hisvsim_b200", "csrc")
+SRCS = [os.path.join(ROOT, "tests", "emu", "k1_wide_emu.cpp"), os.path.join(CSRC, "plan.cpp"),
+        os.path.join(CSRC, "gatemath.cpp")]
+
+
+@pytest.fixture(scope="module")
+def emu(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("wide") / "libwideemu.so")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include",
+           "-I" + os.path.join(ROOT, "include"), "-I" + CSRC] + SRCS + ["-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        pytest.fail("emulator build failed:\n" + r.stderr[-3000:])
+    lib = ctypes.CDLL(out)
+    P = ctypes.c_void_p
+    lib.wide_parts_run.argtypes = [ctypes.c_int, ctypes.c_int, P, P, ctypes.c_int, P, ctypes.c_int,
+                                   ctypes.c_int, P, P]
+    lib.wide_last_error.restype = ctypes.c_char_p
+
+    def run(n, parts, dtype=0, hint=0, per_part=False, q2s=None):
+        """Amplitudes in qubit order of the parts run from |0...0>, and the statistics."""
+        rec, offs = part_offsets(parts)
+        q2s = np.arange(n, dtype=np.int32) if q2s is None else np.asarray(q2s, dtype=np.int32)
+        a = np.zeros(1 << n, complex)
+        a[0] = 1
+        st = np.zeros(5, np.int32)
+        rc = lib.wide_parts_run(n, dtype, rec.ctypes.data, offs.ctypes.data, len(offs) - 1,
+                                q2s.ctypes.data, hint, int(per_part), a.ctypes.data, st.ctypes.data)
+        if rc:
+            raise RuntimeError(lib.wide_last_error().decode())
+        x = np.arange(1 << n)
+        slot = sum(((x >> q) & 1) << int(q2s[q]) for q in range(n))
+        return a[slot], dict(zip(["passes", "wide", "groups", "steps", "tables"], st.tolist()))
+    return run
+
+
+def _mixed(n, layers, seed):
+    """Every gate kind of the wide form on random qubits."""
+    rng = np.random.default_rng(seed)
+    u = lambda: float(rng.uniform(0, 2 * np.pi))  # noqa: E731
+    g = []
+    for _ in range(layers):
+        for q in range(n):
+            g.append(Gate("U3", (q,), params=(u(), u(), u())) if rng.integers(2) else Gate("H", (q,)))
+        for _ in range(n):
+            q = [int(v) for v in rng.permutation(n)[:4]]
+            k = int(rng.integers(11))
+            g.append([Gate("X", (q[0],), (q[1],)), Gate("X", (q[0],), (q[1], q[2])),
+                      Gate("Z", (q[0],), (q[1],)), Gate("Z", (q[0],), (q[1], q[2])),
+                      Gate("SWAP", (q[0], q[1])), Gate("RZZ", (q[0], q[1]), params=(u(),)),
+                      Gate("U1", (q[0],), (q[1],), params=(u(),)),
+                      Gate("C1", (q[0],), (q[1], q[2]), params=(1.0, 0.0, 0.0, np.exp(1j * u()))),
+                      Gate("T", (q[0],)), Gate("RZ", (q[0],), params=(u(),)),
+                      Gate("RZZ", (q[0], q[1]), (q[2],), params=(u(),))][k])
+    return g
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("hint", [0, 10, 11, 12])
+@pytest.mark.parametrize("kind,n,k", [("mixed", 10, 10), ("mixed", 13, 8), ("u3cz", 14, 9),
+                                      ("layered", 13, 7), ("qft", 12, 6), ("qft", 13, 10)])
+def test_wide_programs_match_oracle(emu, port, kind, n, k, hint, dtype):
+    gates = {"mixed": lambda: _mixed(n, 4, 7), "u3cz": lambda: circuits.random_u3_cz(n, 8, 3),
+             "layered": lambda: circuits.random_layered(n, 8, 4),
+             "qft": lambda: circuits.qft(n, 2)[0]}[kind]()
+    want = port.run(n, to_records(gates))
+    tol = 1e-5 if dtype else 1e-12
+    for split in (partition.partition_acyclic, partition.partition_dfs):
+        parts = partition.parts_to_gates(gates, split(gates, k))
+        for per_part in (False, True):
+            got, st = emu(n, parts, dtype=dtype, hint=hint, per_part=per_part)
+            assert st["wide"] == st["passes"] > 0
+            assert np.abs(got - want).max() <= tol
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_any_slot_order(emu, port, seed):
+    """The chunk's qubits in shuffled slots (after a redistribution)."""
+    n = 13
+    gates = _mixed(n, 3, 100 + seed)
+    want = port.run(n, to_records(gates))
+    q2s = np.random.default_rng(seed).permutation(n)
+    parts = partition.parts_to_gates(gates, partition.partition_frontier(gates, 8, free_diagonal=True))
+    for dtype, tol in ((0, 1e-12), (1, 1e-5)):
+        got, st = emu(n, parts, dtype=dtype, q2s=q2s)
+        assert st["wide"] == st["passes"]
+        assert np.abs(got - want).max() <= tol
+
+
+def test_program_limits(emu, port):
+    """Parts at the limits of one program: many rotations of one qubit in a row
+    (a step each), more conditional phases and sign flips than a program holds,
+    and a flush with every qubit pending."""
+    rng = np.random.default_rng(3)
+    n = 12
+    u = lambda: tuple(float(v) for v in rng.uniform(0, 2 * np.pi, 3))  # noqa: E731
+    deep = [g for i in range(150) for g in (Gate("U3", (3,), params=u()), Gate("Z", (3,), (i % 3,)))]
+    many = [Gate("U3", (q,), params=u()) for q in range(n)]
+    for i in range(300):
+        a, b = (int(x) for x in rng.choice(n, 2, replace=False))
+        many.append(Gate("U1", (a,), (b,), params=(u()[0],)) if i % 2 else Gate("Z", (a,), (b,)))
+    many += [Gate("U3", (q,), params=u()) for q in range(n)]
+    for gates in (deep, many):
+        want = port.run(n, to_records(gates))
+        for per_part in (False, True):
+            got, st = emu(n, [gates], per_part=per_part)
+            assert st["wide"] == st["passes"] > 0
+            assert np.abs(got - want).max() <= 1e-12
+
+
+def test_other_gates_keep_the_general_form(emu):
+    """Gates outside the wide form (dense controlled, two-qubit dense, custom
+    non-unitary diagonals, controlled swaps) and small states are not taken."""
+    wide = [Gate("H", (q,)) for q in range(11)]
+    for g in (Gate("H", (0,), (1,)), Gate("RXX", (0, 1), params=(0.3,)),
+              Gate("C1", (0,), (1,), params=(0.5, 0.0, 0.0, 1.0)), Gate("SWAP", (0, 1), (2,))):
+        _, st = emu(11, [wide + [g]])
+        assert st["passes"] == 1 and st["wide"] == 0
+    _, st = emu(9, [[Gate("H", (q,)) for q in range(9)]])
+    assert st["passes"] == 1 and st["wide"] == 0
