@@ -134,13 +134,11 @@ int permute_positions(hs_state* st, const std::vector<int>& pi, cudaStream_t s) 
   return HS_OK;
 }
 
-int launch_passes(hs_state* st, const std::vector<PlannedPass>& passes, cudaStream_t s) {
-  for (const auto& p : passes) {
-    HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, s)
-                  : launch_part(st->amp, st->dtype, *p.part, s));
-    count_pass(p.nops());
-    g_param_bytes += (long long)p.bytes();
-  }
+int launch_pass(hs_state* st, const PlannedPass& p, cudaStream_t s) {
+  HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, s)
+                : launch_part(st->amp, st->dtype, *p.part, s));
+  count_pass(p.nops());
+  g_param_bytes += (long long)p.bytes();
   return HS_OK;
 }
 
@@ -151,7 +149,8 @@ int run_lowered(hs_state* st, const std::vector<LoweredGate>& lg, Frames* fr, bo
   std::vector<PlannedPass> passes;
   HS_TRY(plan_passes(st->n, st->q2s, lg, fr, flush, g_tile_hint.load(), st->dtype, &passes));
   TimedRegion tr(s);
-  return launch_passes(st, passes, s);
+  for (const auto& p : passes) HS_TRY(launch_pass(st, p, s));
+  return HS_OK;
 }
 
 // one self-contained part: fresh frames, flushed at the end
@@ -416,13 +415,15 @@ int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets
   for (int p = 0; p < num_parts; ++p)
     HS_TRY(lower_all(st, gates + part_offsets[p], part_offsets[p + 1] - part_offsets[p],
                      &all[p]));
-  // one pass (or more) per part; the pending diagonal of the factored
-  // rotations is carried from part to part and applied by the last one
+  // the pending diagonal of the factored rotations is carried from part to part
+  // and applied by the last pass; each pass is launched as soon as it is planned
   Frames fr;
   fr.reset(st->n);
-  for (int p = 0; p < num_parts; ++p)
-    HS_TRY(run_lowered(st, all[p], &fr, p == num_parts - 1, S(stream)));
-  return HS_OK;
+  return plan_parts(st->n, st->q2s, all, &fr, true, g_tile_hint.load(), st->dtype,
+                    [&](PlannedPass& p) {
+                      TimedRegion tr(S(stream));
+                      return launch_pass(st, p, S(stream));
+                    });
 }
 
 int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,
@@ -452,7 +453,8 @@ int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_o
   if (rc == HS_OK && cudaEventRecord(ev[0], s) != cudaSuccess)
     rc = set_error(HS_E_CUDA, "event record");
   for (int p = 0; p < num_parts && rc == HS_OK; ++p) {
-    rc = launch_passes(st, progs[p], s);
+    for (const auto& ps : progs[p])
+      if ((rc = launch_pass(st, ps, s)) != HS_OK) break;
     if (rc == HS_OK && cudaEventRecord(ev[p + 1], s) != cudaSuccess)
       rc = set_error(HS_E_CUDA, "event record");
   }

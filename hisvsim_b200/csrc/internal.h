@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <complex>
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -322,6 +323,12 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
 int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
                 Frames* fr, bool flush, int tile_bits_hint, int dtype,
                 std::vector<PlannedPass>* passes);
+// The parts of one call, handed to `sink` pass by pass as they are planned (an
+// error it returns ends the planning).  A pass may take gates of later parts.
+using PassSink = std::function<int(PlannedPass&)>;
+int plan_parts(int n, const std::vector<int>& q2s,
+               const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
+               int tile_bits_hint, int dtype, const PassSink& sink);
 // one self-contained part: fresh frames, flushed at the end
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
               int tile_bits_hint, int dtype, std::vector<PartProgram>* programs);

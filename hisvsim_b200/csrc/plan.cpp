@@ -204,6 +204,7 @@ enum RKind { RK_MATRIX = 0, RK_ROT = 1, RK_FLUSH = 2 };
 
 struct RGate {
   RKind kind = RK_MATRIX;
+  int part = 0;               // the part its gate came from
   LoweredGate g;              // targets / controls (and the matrix for RK_MATRIX)
   Rot rot;                    // RK_ROT
   std::vector<int> flq;       // RK_FLUSH: qubits
@@ -304,85 +305,93 @@ bool out_of_range(cplx G, double lim) {
 // `scaled`: rotations may leave real scales in the frames (complex128);
 // `lim`: the global factor's scale is flushed once it leaves 2^+-lim; `split`:
 // diagonal gates become phases (split_diagonal), for wide programs.
-void rewrite(const std::vector<LoweredGate>& in, Frames* F, bool scaled, double lim, bool split,
-             std::vector<RGate>* out) {
-  for (const auto& g : in) {
-    if (g.nt == 0) continue;
-    const bool diag = is_diagonal(g);
-    if (g.nt == 1 && g.nc == 0) {
-      const int q = g.targets[0];
-      const cplx rq = F->r[q];
-      if (diag) {
-        if (g.m[0] != cplx(0.0, 0.0)) {  // joins the pending diagonal
-          F->G *= g.m[0];
-          F->r[q] = g.m[3] * rq / g.m[0];
-        } else {  // degenerate (custom C1): applied with the pending factor
-          RGate x;
-          x.g = g;
-          x.g.m[3] *= rq;
-          F->r[q] = 1.0;
-          out->push_back(x);
-        }
-        continue;
-      }
-      cplx W[4] = {g.m[0], g.m[1] * rq, g.m[2], g.m[3] * rq};
-      RGate x;
-      x.g = g;
-      if (factor_rotation(W, scaled, &x.rot)) {
-        x.kind = RK_ROT;
-        F->G *= x.rot.g0;
-        F->r[q] = x.rot.g1 / x.rot.g0;
-      } else {
-        for (int k = 0; k < 4; ++k) x.g.m[k] = W[k];
+void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double lim, bool split,
+                  std::vector<RGate>* out) {
+  if (g.nt == 0) return;
+  const bool diag = is_diagonal(g);
+  if (g.nt == 1 && g.nc == 0) {
+    const int q = g.targets[0];
+    const cplx rq = F->r[q];
+    if (diag) {
+      if (g.m[0] != cplx(0.0, 0.0)) {  // joins the pending diagonal
+        F->G *= g.m[0];
+        F->r[q] = g.m[3] * rq / g.m[0];
+      } else {  // degenerate (custom C1): applied with the pending factor
+        RGate x;
+        x.g = g;
+        x.g.m[3] *= rq;
         F->r[q] = 1.0;
+        out->push_back(x);
       }
-      out->push_back(x);
-      if (out_of_range(F->G, lim)) {
-        // bring the stored amplitudes' scale back (one multiply of the state)
-        Frames sc;
-        sc.G = std::abs(F->G);
-        out->push_back(flush_gate(&sc));
-        F->G /= std::abs(F->G);
-      }
-      continue;
+      return;
     }
-    if (diag) {  // controlled or two-qubit diagonal: commutes with the pending diagonal
-      if (split && split_diagonal(g, F, out)) continue;
-      RGate x;
-      x.g = g;
-      out->push_back(x);
-      continue;
+    cplx W[4] = {g.m[0], g.m[1] * rq, g.m[2], g.m[3] * rq};
+    RGate x;
+    x.g = g;
+    if (factor_rotation(W, scaled, &x.rot)) {
+      x.kind = RK_ROT;
+      F->G *= x.rot.g0;
+      F->r[q] = x.rot.g1 / x.rot.g0;
+    } else {
+      for (int k = 0; k < 4; ++k) x.g.m[k] = W[k];
+      F->r[q] = 1.0;
     }
-    if (g.nt == 2 && g.nc == 0) {
-      const int t0 = g.targets[0], t1 = g.targets[1];
-      RGate x;
-      x.g = g;
-      if (is_swap4(g.m)) {
-        std::swap(F->r[t0], F->r[t1]);
-      } else {
-        // absorb diag(1, r_t0) (x) diag(1, r_t1); reference index i = 2*b(t0) + b(t1)
-        for (int c = 0; c < 4; ++c) {
-          cplx d = 1.0;
-          if (c & 2) d *= F->r[t0];
-          if (c & 1) d *= F->r[t1];
-          for (int r = 0; r < 4; ++r) x.g.m[4 * r + c] *= d;
-        }
-        F->r[t0] = F->r[t1] = 1.0;
-      }
-      out->push_back(x);
-      continue;
+    out->push_back(x);
+    if (out_of_range(F->G, lim)) {
+      // bring the stored amplitudes' scale back (one multiply of the state)
+      Frames sc;
+      sc.G = std::abs(F->G);
+      out->push_back(flush_gate(&sc));
+      F->G /= std::abs(F->G);
     }
-    // controlled non-diagonal gate: apply the pending factors of its targets first
-    for (int i = 0; i < g.nt; ++i) {
-      const int t = g.targets[i];
-      if (F->r[t] != cplx(1.0, 0.0)) {
-        out->push_back(phase_gate(t, F->r[t]));
-        F->r[t] = 1.0;
-      }
-    }
+    return;
+  }
+  if (diag) {  // controlled or two-qubit diagonal: commutes with the pending diagonal
+    if (split && split_diagonal(g, F, out)) return;
     RGate x;
     x.g = g;
     out->push_back(x);
+    return;
+  }
+  if (g.nt == 2 && g.nc == 0) {
+    const int t0 = g.targets[0], t1 = g.targets[1];
+    RGate x;
+    x.g = g;
+    if (is_swap4(g.m)) {
+      std::swap(F->r[t0], F->r[t1]);
+    } else {
+      // absorb diag(1, r_t0) (x) diag(1, r_t1); reference index i = 2*b(t0) + b(t1)
+      for (int c = 0; c < 4; ++c) {
+        cplx d = 1.0;
+        if (c & 2) d *= F->r[t0];
+        if (c & 1) d *= F->r[t1];
+        for (int r = 0; r < 4; ++r) x.g.m[4 * r + c] *= d;
+      }
+      F->r[t0] = F->r[t1] = 1.0;
+    }
+    out->push_back(x);
+    return;
+  }
+  // controlled non-diagonal gate: apply the pending factors of its targets first
+  for (int i = 0; i < g.nt; ++i) {
+    const int t = g.targets[i];
+    if (F->r[t] != cplx(1.0, 0.0)) {
+      out->push_back(phase_gate(t, F->r[t]));
+      F->r[t] = 1.0;
+    }
+  }
+  RGate x;
+  x.g = g;
+  out->push_back(x);
+}
+
+// every part in turn; the gates keep their part's number
+void rewrite(const std::vector<std::vector<LoweredGate>>& parts, Frames* F, bool scaled, double lim,
+             bool split, std::vector<RGate>* out) {
+  for (size_t p = 0; p < parts.size(); ++p) {
+    const size_t first = out->size();
+    for (const auto& g : parts[p]) rewrite_gate(g, F, scaled, lim, split, out);
+    for (size_t i = first; i < out->size(); ++i) (*out)[i].part = int(p);
   }
 }
 
@@ -868,10 +877,20 @@ struct RecSet {
     RecSet r = *this;
     return r |= o;
   }
+  RecSet minus(const RecSet& o) const {
+    RecSet r;
+    for (int k = 0; k < kRecWords; ++k) r.w[k] = w[k] & ~o.w[k];
+    return r;
+  }
   bool within(const RecSet& o) const {
     for (int k = 0; k < kRecWords; ++k)
       if (w[k] & ~o.w[k]) return false;
     return true;
+  }
+  template <typename F>
+  void each(F&& f) const {  // in order
+    for (int k = 0; k < kRecWords; ++k)
+      for (uint64_t x = w[k]; x; x &= x - 1) f(64 * k + __builtin_ctzll(x));
   }
 };
 
@@ -969,7 +988,9 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
   // and for a non-diagonal op the diagonal ones since (what came before those
   // follows from them)
   if (n > kRecWords * 64) return set_error(HS_E_UNSUPPORTED, "%d ops in a group", n);
-  RecSet preds[kRecWords * 64], done{}, diag{};
+  RecSet preds[kRecWords * 64], done{}, diag{}, perm{};
+  std::vector<int> queue[kWideBits];  // the non-diagonal ops of each bit, in order
+  size_t head[kWideBits] = {};
   {
     int last[kWideBits];
     RecSet since[kWideBits] = {};
@@ -982,6 +1003,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
         if ((rec[b].target >> j) & 1u) {
           p |= since[j];
           last[j] = b;
+          queue[j].push_back(b);
           since[j] = RecSet{};
         } else {
           since[j].add(b);
@@ -989,6 +1011,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
       }
       preds[b] = p;
       if (rec[b].diag()) diag.add(b);
+      if (rec[b].kind == WideRec::kCx || rec[b].kind == WideRec::kSwap) perm.add(b);
     }
   }
   int left = n;
@@ -1032,39 +1055,38 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     S.first_sign = uint16_t(P->nsigns);
     S.first_op = uint16_t(P->nwops);
     open = RecSet{};
-    for (int i = 0; i < n; ++i)
-      if (rec[i].diag() && !rec[i].done && available(i)) open.add(i);
+    diag.minus(done).each([&](int i) {
+      if (available(i)) open.add(i);
+    });
     // ---- the step's non-diagonal ops
     int rot[kWideBits];
     uint32_t touched = 0, moved = 0;  // register bits acted on; by controlled X and swaps
     std::vector<int> perms;
     for (int j = 0; j < kWideBits; ++j) {
       rot[j] = -1;
-      for (int i = 0; i < n; ++i)
-        if (!rec[i].done && rec[i].kind == WideRec::kRot && rec[i].j == j) {
-          if (ready(i)) rot[j] = i;
-          break;
-        }
-      if (rot[j] >= 0) touched |= 1u << j;
+      while (head[j] < queue[j].size() && rec[queue[j][head[j]]].done) ++head[j];
+      if (head[j] == queue[j].size()) continue;
+      const int i = queue[j][head[j]];  // (a later op on the bit has to follow it)
+      if (rec[i].kind == WideRec::kRot && ready(i)) {
+        rot[j] = i;
+        touched |= 1u << j;
+      }
     }
-    for (int i = 0; i < n; ++i) {
-      if (rec[i].done || (rec[i].kind != WideRec::kCx && rec[i].kind != WideRec::kSwap)) continue;
+    perm.minus(done).each([&](int i) {
       RecSet here = done | open;  // the step's rotations and earlier perms run first
       for (int j = 0; j < kWideBits; ++j)
         if (rot[j] >= 0) here.add(rot[j]);
       for (int a : perms) here.add(a);
-      const bool ok = preds[i].within(here);
-      if (ok) {
+      if (preds[i].within(here)) {
         perms.push_back(i);
         moved |= rec[i].target;
       }
-    }
+    });
     touched |= moved;
     const bool last = touched == 0;  // diagonal ops alone are left
     // ---- diagonal ops
     std::vector<int> run;
-    for (int i = 0; i < n; ++i) {
-      if (rec[i].done || !rec[i].diag() || !available(i)) continue;
+    open.each([&](int i) {
       if (is_sign(i)) {
         WideSign& q = P->signs[P->nsigns++];
         q.bits = rec[i].mask ? rec[i].mask : 32u;
@@ -1073,27 +1095,23 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
         ++S.nsigns;
         pend_any = true;
         pend |= rec[i].mask;
+        finish(i);
       } else if (last || (rec[i].mask & touched)) {
         run.push_back(i);
       }
-    }
-    for (int i = 0; i < n; ++i)  // (after the scan: available() looks at done)
-      if (!rec[i].done && rec[i].diag() && is_sign(i) && available(i)) finish(i);
+    });
     // phase parts: of the rotations next on their bits
     int zs[kWideBits], nz = 0;
     bool need = false;
-    for (int j = 0; j < kWideBits; ++j)
-      for (int i = 0; i < n; ++i)
-        if (!rec[i].done && ((rec[i].target >> j) & 1u)) {
-          if (rec[i].kind == WideRec::kRot && rec[i].z) {
-            // nothing non-diagonal on the bit is ahead of it
-            if (preds[i].within(done | diag)) {
-              zs[nz++] = i;
-              need |= rot[j] == i;
-            }
-          }
-          break;
-        }
+    for (int j = 0; j < kWideBits; ++j) {
+      if (head[j] == queue[j].size()) continue;
+      const int i = queue[j][head[j]];
+      // (nothing non-diagonal on the bit is ahead of it)
+      if (rec[i].kind == WideRec::kRot && rec[i].z) {
+        zs[nz++] = i;
+        need |= rot[j] == i;
+      }
+    }
     // multiply-adds per amplitude of a table (2^R - 1 complex factors) and of
     // the same work op by op; a negation counts its integer operations
     double single = 1.5 * nz;
@@ -1115,13 +1133,13 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
       f[0] = 1.0;
       for (int e = 1; e < size; ++e)  // the lowest set bit's factor times the others'
         f[e] = f[e & (e - 1)] * by_bit[__builtin_ctz(unsigned(e))];
-      for (int i = 0; i < n; ++i) {  // every such factor that may run now
-        if (rec[i].done || !rec[i].diag() || !unit(i) || !available(i)) continue;
+      open.minus(done).each([&](int i) {  // every such factor that may run now
+        if (!unit(i)) return;
         for (uint32_t e = rec[i].mask; e < uint32_t(size); e = (e + 1) | rec[i].mask)
           f[e] *= rec[i].c;
         run.erase(std::remove(run.begin(), run.end(), i), run.end());
         finish(i);
-      }
+      });
       S.table = uint16_t(P->ncoef);
       for (int e = 0; e < size; ++e) push_amp_coef(f[e]);
     }
@@ -1244,10 +1262,10 @@ void finish_wide(WideProgram* P, const std::vector<uint32_t>& regs, int dtype) {
   }
 }
 
-// A chunk (gates [first, last) of sgs, every one a wide_gate) as wide programs:
-// one, or more where its groups outgrow a program.
+// A chunk (gates of sgs, every one a wide_gate) as wide programs: one, or more
+// where its groups outgrow a program.
 int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
-                    const std::vector<SlotGate>& sgs, size_t first, size_t last,
+                    const std::vector<SlotGate>& sgs, std::vector<int> remaining,
                     const std::vector<int>& tile, const std::vector<int>& tbit_of_slot,
                     std::vector<PlannedPass>* passes) {
   const int m = int(tile.size());
@@ -1273,9 +1291,8 @@ int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
     build_runs(outer, &P->outer);
   };
   new_program();
-  std::vector<int> remaining, members, rest;
+  std::vector<int> members, rest;
   std::vector<WideRec> rec;
-  for (size_t x = first; x < last; ++x) remaining.push_back(int(x));
   while (!remaining.empty()) {
     uint32_t rmask = 0;
     members.clear();
@@ -1311,22 +1328,49 @@ int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
   return HS_OK;
 }
 
+// What a program has room for, as the chunk grows.
+struct ChunkRoom {
+  int ops = 0, coefs = 0, fls = 0;
+  bool add(const SlotGate& g) {
+    const bool fl = g.rg->kind == RK_FLUSH;
+    const int f = fl ? int(g.rg->flq.size()) : 0, o = fl ? 1 + f : 1, c = coef_count(g);
+    if (ops + o > kMaxOps || coefs + c > kMaxCoef || fls + f > kMaxFlush) return false;
+    ops += o;
+    coefs += c;
+    fls += f;
+    return true;
+  }
+};
+
 // The planner of both program kinds: into `programs` (PartPrograms only) or,
-// with `passes`, as PartPrograms and WidePrograms.
-int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
-                Frames* fr, bool flush, int tile_bits_hint, int dtype,
-                std::vector<PartProgram>* programs, std::vector<PlannedPass>* passes) {
+// with `sink`, as PartPrograms and WidePrograms, handed over pass by pass.
+// A pass takes what fits of the first part left (in order, up to the first gate
+// that does not fit).  Given a sink, a pass of wide gates also takes, where that
+// saves passes, every gate of the parts after it that fits the tile and has to
+// follow no gate left behind: a part bounded by the qubits its gates touch
+// leaves room in the tile, which holds targets alone, and parts so used up cost
+// no pass of their own (27 qubits, parts of 9 touched qubits: 9 passes instead
+// of 13; 20 random layers of 20 qubits in parts of 10: 9 instead of 26).
+int plan_chunks(int n, const std::vector<int>& q2s,
+                const std::vector<std::vector<LoweredGate>>& gates, Frames* fr, bool flush,
+                int tile_bits_hint, int dtype, std::vector<PartProgram>* programs,
+                const PassSink* sink) {
   if (n < 1 || n > 63) return set_error(HS_E_INVALID, "bad qubit count %d", n);
   if (int(fr->r.size()) != n) fr->reset(n);
   std::vector<RGate> rg;
-  rg.reserve(gates.size() + 2);
+  size_t count = 2;
+  for (const auto& g : gates) count += g.size();
+  rg.reserve(count);
   // keep the carried scale within a few dozen binary orders (it moves with
   // the scaled rotation forms and non-unitary diagonal gates)
   const double lim = dtype == HS_DTYPE_C64 ? 24.0 : 48.0;
-  const bool wide = passes && use_wide(n, dtype);
+  const bool wide = sink && use_wide(n, dtype);
   rewrite(gates, fr, dtype == HS_DTYPE_C128, lim, wide, &rg);
   if (flush) {
-    if (!fr->identity()) rg.push_back(flush_gate(fr));
+    if (!fr->identity()) {
+      rg.push_back(flush_gate(fr));
+      rg.back().part = int(gates.size()) - 1;
+    }
   } else if (out_of_range(fr->G, lim)) {
     Frames scale;
     scale.G = std::abs(fr->G);
@@ -1378,35 +1422,74 @@ int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
   // for complex64); where the targets leave room the tile takes all three:
   // shorter runs cost less than another pass
   const int low_need = std::min(n, dtype == HS_DTYPE_C64 ? 1 : 0);
-  size_t gi = 0;
-  while (gi < sgs.size()) {
-    // ---- chunk: gates whose non-diagonal target slots (+ low slots) fit one tile
+  // ---- chunks: gates whose non-diagonal target slots (+ low slots) fit one tile
+  struct Chunk {
+    std::vector<int> gates;
     uint64_t tset = 0;
-    size_t gend = gi;
-    int ops = 0, coefs = 0, fls = 0;
-    while (gend < sgs.size()) {
-      const uint64_t t2 = tset | sgs[gend].tmask;
-      const int cc = coef_count(sgs[gend]);
-      const int nops_g = sgs[gend].rg->kind == RK_FLUSH ? 1 + int(sgs[gend].rg->flq.size()) : 1;
-      const int nfl_g = sgs[gend].rg->kind == RK_FLUSH ? int(sgs[gend].rg->flq.size()) : 0;
-      if (low_union_size(t2, low_need) > max_tile || ops + nops_g > kMaxOps || coefs + cc > kMaxCoef ||
-          fls + nfl_g > kMaxFlush)
-        break;
-      tset = t2;
-      ops += nops_g;
-      coefs += cc;
-      fls += nfl_g;
-      ++gend;
+    bool wide = false;
+  };
+  auto cut = [&](bool merge, std::vector<Chunk>* out) -> bool {
+    std::vector<int> left, rest;
+    for (size_t x = 0; x < sgs.size(); ++x) left.push_back(int(x));
+    while (!left.empty()) {
+      out->emplace_back();
+      Chunk& c = out->back();
+      ChunkRoom room;
+      const int part = sgs[left[0]].rg->part;
+      c.wide = wide;
+      size_t i = 0;
+      for (; i < left.size(); ++i) {
+        const SlotGate& g = sgs[left[i]];
+        if (g.rg->part != part || low_union_size(c.tset | g.tmask, low_need) > max_tile ||
+            !room.add(g))
+          break;
+        c.tset |= g.tmask;
+        c.gates.push_back(left[i]);
+        c.wide = c.wide && wide_gate(g);
+      }
+      if (c.gates.empty()) return false;
+      rest.clear();
+      if (merge && c.wide && low_union_size(c.tset, low_min) <= max_tile) {
+        uint64_t held_t = 0, held_d = 0;  // slots of gates left behind, as in take_group_roles
+        const uint64_t every = (1ull << n) - 1ull;
+        for (; i < left.size() && held_t != every; ++i) {
+          const SlotGate& g = sgs[left[i]];
+          if ((g.tmask & (held_t | held_d)) || (g.dmask & held_t) || !wide_gate(g) ||
+              low_union_size(c.tset | g.tmask, low_min) > max_tile || !room.add(g)) {
+            held_t |= g.tmask;
+            held_d |= g.dmask;
+            rest.push_back(left[i]);
+            continue;
+          }
+          c.tset |= g.tmask;
+          c.gates.push_back(left[i]);
+        }
+      }
+      rest.insert(rest.end(), left.begin() + i, left.end());
+      left.swap(rest);
     }
-    if (gend == gi) return set_error(HS_E_INVALID, "gate does not fit a tile");
-    const bool wide_chunk =
-        wide && std::all_of(sgs.begin() + gi, sgs.begin() + gend, wide_gate);
+    return true;
+  };
+  std::vector<Chunk> chunks, merged;
+  if (!cut(false, &chunks)) return set_error(HS_E_INVALID, "gate does not fit a tile");
+  // moving gates between passes pays where it saves passes: as many passes with
+  // other gates in them only change places of work and widen tiles.  Complex64
+  // calls keep a pass per part: hs_parts_run_timed, which times the parts one by
+  // one, gives the same bits there.
+  if (wide && dtype == HS_DTYPE_C128 && gates.size() > 1 && cut(true, &merged) &&
+      merged.size() < chunks.size())
+    chunks.swap(merged);
+  std::vector<PlannedPass> passes;
+  for (const Chunk& c : chunks) {
+    const std::vector<int>& chunk = c.gates;
+    const bool wide_chunk = c.wide;
+    uint64_t tset = c.tset;
     // wide chunks with controlled X or swaps on states beyond the L2 take the
     // largest tile (CTAs of four warps): 7.35 against 7.97 ms for 8 random
     // layers of 26 qubits; in the L2, and without them, 2^10 is the faster
     const bool big = wide_chunk && tile_bits_hint <= 0 && (amp_bytes(dtype) << n) > (128ull << 20) &&
-                     std::any_of(sgs.begin() + gi, sgs.begin() + gend, [](const SlotGate& s) {
-                       return s.rg->kind == RK_MATRIX && !s.diag;
+                     std::any_of(chunk.begin(), chunk.end(), [&](int x) {
+                       return sgs[x].rg->kind == RK_MATRIX && !sgs[x].diag;
                      });
     // ---- tile: non-diagonal target slots + lowest slots up to the target size
     const int m = std::min(max_tile, std::max(big ? kWideMaxTileBits : m_target,
@@ -1418,17 +1501,25 @@ int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
     const int R = std::min(rbits, m);
     std::vector<int> tbit_of_slot(n, -1);
     for (int i = 0; i < m; ++i) tbit_of_slot[tile[i]] = i;
+    passes.clear();
+    auto hand_over = [&]() -> int {
+      for (auto& p : passes) {
+        if (p.part) finish_layout(p.part.get(), dtype);
+        if (p.nops() > 0) HS_TRY((*sink)(p));  // (a pass without ops has nothing to do)
+      }
+      return HS_OK;
+    };
     if (wide_chunk && m >= kWideMinTileBits) {
-      HS_TRY(plan_wide_chunk(n, dtype, q2s, sgs, gi, gend, tile, tbit_of_slot, passes));
-      gi = gend;
+      HS_TRY(plan_wide_chunk(n, dtype, q2s, sgs, chunk, tile, tbit_of_slot, &passes));
+      HS_TRY(hand_over());
       continue;
     }
     PartProgram* P = nullptr;
     auto new_program = [&]() {
-      if (passes) {
-        passes->emplace_back();
-        passes->back().part.reset(new PartProgram);
-        P = passes->back().part.get();
+      if (sink) {
+        passes.emplace_back();
+        passes.back().part.reset(new PartProgram);
+        P = passes.back().part.get();
       } else {
         programs->emplace_back();
         P = &programs->back();
@@ -1438,7 +1529,7 @@ int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
       P->m = m;
       P->ntiles = 1ull << (n - m);
       P->rbits = R;
-        build_runs(tile, &P->tile);
+      build_runs(tile, &P->tile);
       for (int b = 0; b < m; ++b) P->tile_slot[b] = uint8_t(tile[b]);
       std::vector<int> outer;
       for (int s = 0; s < n; ++s)
@@ -1447,12 +1538,11 @@ int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
     };
     new_program();
     // ---- groups
-    std::vector<int> remaining;
-    for (size_t x = gi; x < gend; ++x) remaining.push_back(int(x));
+    std::vector<int> remaining = chunk;
     while (!remaining.empty()) {
       uint32_t rmask = 0;
-      std::vector<int> regs, members, rest;
-      take_group(sgs, remaining, tbit_of_slot, R, &rmask, &members, &rest);
+      std::vector<int> regs, members, later;
+      take_group(sgs, remaining, tbit_of_slot, R, &rmask, &members, &later);
       if (P->ngroups == kMaxGroups) new_program();  // a new pass (rare)
       GroupDesc& gd = P->groups[P->ngroups++];
       std::memset(&gd, 0, sizeof(gd));
@@ -1483,20 +1573,12 @@ int plan_chunks(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
       }
       gd.num_ops = uint16_t(P->nops - gd.first_op);
       build_rounds(P, &gd);
-      remaining = rest;
+      remaining = later;
     }
-    gi = gend;
+    if (sink) HS_TRY(hand_over());
   }
-  if (!passes) {
+  if (!sink)
     for (auto& P : *programs) finish_layout(&P, dtype);
-    return HS_OK;
-  }
-  for (auto& p : *passes)
-    if (p.part) finish_layout(p.part.get(), dtype);
-  // a pass without ops has nothing to do
-  passes->erase(std::remove_if(passes->begin(), passes->end(),
-                               [](const PlannedPass& p) { return p.nops() < 1; }),
-                passes->end());
   return HS_OK;
 }
 
@@ -1506,14 +1588,24 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
                Frames* fr, bool flush, int tile_bits_hint, int dtype,
                std::vector<PartProgram>* programs) {
   programs->clear();
-  return plan_chunks(n, q2s, gates, fr, flush, tile_bits_hint, dtype, programs, nullptr);
+  return plan_chunks(n, q2s, {gates}, fr, flush, tile_bits_hint, dtype, programs, nullptr);
+}
+
+int plan_parts(int n, const std::vector<int>& q2s,
+               const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
+               int tile_bits_hint, int dtype, const PassSink& sink) {
+  return plan_chunks(n, q2s, parts, fr, flush, tile_bits_hint, dtype, nullptr, &sink);
 }
 
 int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
                 Frames* fr, bool flush, int tile_bits_hint, int dtype,
                 std::vector<PlannedPass>* passes) {
   passes->clear();
-  return plan_chunks(n, q2s, gates, fr, flush, tile_bits_hint, dtype, nullptr, passes);
+  const PassSink sink = [&](PlannedPass& p) {
+    passes->push_back(std::move(p));
+    return HS_OK;
+  };
+  return plan_chunks(n, q2s, {gates}, fr, flush, tile_bits_hint, dtype, nullptr, &sink);
 }
 
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,

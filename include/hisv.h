@@ -165,10 +165,11 @@ int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream)
 /* Several parts back to back (the loop of execute_qasm_parts,
  * qasm_assembler_standalone.py:1784-2018); part i is
  * gates[part_offsets[i] .. part_offsets[i+1]).  One or more K1 passes per
- * part; the phases that the factored one-qubit rotations leave pending are
- * carried from part to part and applied by the last pass, so the state after
- * the call is the reference's (to rounding) while the states between parts
- * are not observable. */
+ * part, or (complex128) fewer passes than parts where gates of later parts fit
+ * into earlier passes; the phases that the factored one-qubit rotations leave
+ * pending are carried from part to part and applied by the last pass, so the
+ * state after the call is the reference's (to rounding) while the states
+ * between parts are not observable. */
 int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,
                  int num_parts, void* stream);
 

@@ -208,12 +208,13 @@ extern "C" {
 
 const char* wide_last_error() { return g_err; }
 
-// Plan parts (frames carried and flushed by the last, or per part) on a state
-// whose qubit q sits in slot q2s[q], run the wide passes on `amps` (slot order,
+// Plan parts (mode 0: one by one, frames carried and flushed by the last; 1:
+// each on its own; 2: as one call, gates moving into earlier parts' passes) on a
+// state whose qubit q sits in slot q2s[q], run the wide passes on `amps` (slot order,
 // 2^n complex128, in/out; complex64 rounds).  stats: {passes, wide passes,
 // groups, steps, tables}.
 int wide_parts_run(int n, int dtype, const hs_gate* gates, const int32_t* offs, int nparts,
-                   const int32_t* q2s_in, int tile_hint, int per_part, double* amps,
+                   const int32_t* q2s_in, int tile_hint, int mode, double* amps,
                    int32_t* stats) {
   const int ab = int(amp_bytes(dtype));
   std::vector<C> sv(size_t(1) << n);
@@ -225,29 +226,41 @@ int wide_parts_run(int n, int dtype, const hs_gate* gates, const int32_t* offs, 
   Frames fr;
   fr.reset(n);
   int32_t st[5] = {0, 0, 0, 0, 0};
+  const PassSink sink = [&](PlannedPass& ps) -> int {
+    ++st[0];
+    if (!ps.wide) return HS_OK;
+    ++st[1];
+    st[2] += ps.wide->ngroups;
+    st[3] += ps.wide->nsteps;
+    for (int s = 0; s < ps.wide->nsteps; ++s) st[4] += ps.wide->steps[s].table != 0;
+    try {
+      Emu{*ps.wide, ab}.run(sv);
+    } catch (const std::exception& e) {
+      std::snprintf(g_err, sizeof(g_err), "%s", e.what());
+      return HS_E_INVALID;
+    }
+    return HS_OK;
+  };
+  std::vector<std::vector<LoweredGate>> parts(nparts);
   for (int p = 0; p < nparts; ++p) {
-    std::vector<LoweredGate> lg(offs[p + 1] - offs[p]);
+    parts[p].resize(offs[p + 1] - offs[p]);
     for (int i = offs[p]; i < offs[p + 1]; ++i) {
-      const int rc = lower_gate(gates[i], n, &lg[i - offs[p]]);
+      const int rc = lower_gate(gates[i], n, &parts[p][i - offs[p]]);
       if (rc != HS_OK) return rc;
     }
-    std::vector<PlannedPass> passes;
-    if (per_part) fr.reset(n);
-    const int rc = plan_passes(n, q2s, lg, &fr, per_part || p == nparts - 1, tile_hint, dtype, &passes);
+  }
+  if (mode == 2) {
+    const int rc = plan_parts(n, q2s, parts, &fr, true, tile_hint, dtype, sink);
     if (rc != HS_OK) return rc;
-    for (const auto& ps : passes) {
-      ++st[0];
-      if (!ps.wide) continue;
-      ++st[1];
-      st[2] += ps.wide->ngroups;
-      st[3] += ps.wide->nsteps;
-      for (int s = 0; s < ps.wide->nsteps; ++s) st[4] += ps.wide->steps[s].table != 0;
-      try {
-        Emu{*ps.wide, ab}.run(sv);
-      } catch (const std::exception& e) {
-        std::snprintf(g_err, sizeof(g_err), "%s", e.what());
-        return HS_E_INVALID;
-      }
+  } else {
+    for (int p = 0; p < nparts; ++p) {
+      std::vector<PlannedPass> passes;
+      if (mode == 1) fr.reset(n);
+      int rc = plan_passes(n, q2s, parts[p], &fr, mode == 1 || p == nparts - 1, tile_hint, dtype,
+                           &passes);
+      for (auto& ps : passes)
+        if (rc == HS_OK) rc = sink(ps);
+      if (rc != HS_OK) return rc;
     }
   }
   for (size_t i = 0; i < sv.size(); ++i) {

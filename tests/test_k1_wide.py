@@ -35,7 +35,7 @@ def emu(tmp_path_factory):
                                    ctypes.c_int, P, P]
     lib.wide_last_error.restype = ctypes.c_char_p
 
-    def run(n, parts, dtype=0, hint=0, per_part=False, q2s=None):
+    def run(n, parts, dtype=0, hint=0, mode=0, q2s=None):
         """Amplitudes in qubit order of the parts run from |0...0>, and the statistics."""
         rec, offs = part_offsets(parts)
         q2s = np.arange(n, dtype=np.int32) if q2s is None else np.asarray(q2s, dtype=np.int32)
@@ -43,7 +43,7 @@ def emu(tmp_path_factory):
         a[0] = 1
         st = np.zeros(5, np.int32)
         rc = lib.wide_parts_run(n, dtype, rec.ctypes.data, offs.ctypes.data, len(offs) - 1,
-                                q2s.ctypes.data, hint, int(per_part), a.ctypes.data, st.ctypes.data)
+                                q2s.ctypes.data, hint, mode, a.ctypes.data, st.ctypes.data)
         if rc:
             raise RuntimeError(lib.wide_last_error().decode())
         x = np.arange(1 << n)
@@ -85,9 +85,11 @@ def test_wide_programs_match_oracle(emu, port, kind, n, k, hint, dtype):
     tol = 1e-5 if dtype else 1e-12
     for split in (partition.partition_acyclic, partition.partition_dfs):
         parts = partition.parts_to_gates(gates, split(gates, k))
-        for per_part in (False, True):
-            got, st = emu(n, parts, dtype=dtype, hint=hint, per_part=per_part)
+        for mode in (0, 1, 2):
+            got, st = emu(n, parts, dtype=dtype, hint=hint, mode=mode)
             assert st["wide"] == st["passes"] > 0
+            # (the flush of the pending factors may take a pass of its own)
+            assert mode != 2 or st["passes"] <= len(parts) + 1
             assert np.abs(got - want).max() <= tol
 
 
@@ -100,9 +102,10 @@ def test_any_slot_order(emu, port, seed):
     q2s = np.random.default_rng(seed).permutation(n)
     parts = partition.parts_to_gates(gates, partition.partition_frontier(gates, 8, free_diagonal=True))
     for dtype, tol in ((0, 1e-12), (1, 1e-5)):
-        got, st = emu(n, parts, dtype=dtype, q2s=q2s)
-        assert st["wide"] == st["passes"]
-        assert np.abs(got - want).max() <= tol
+        for mode in (0, 2):
+            got, st = emu(n, parts, dtype=dtype, mode=mode, q2s=q2s)
+            assert st["wide"] == st["passes"]
+            assert np.abs(got - want).max() <= tol
 
 
 def test_program_limits(emu, port):
@@ -120,10 +123,24 @@ def test_program_limits(emu, port):
     many += [Gate("U3", (q,), params=u()) for q in range(n)]
     for gates in (deep, many):
         want = port.run(n, to_records(gates))
-        for per_part in (False, True):
-            got, st = emu(n, [gates], per_part=per_part)
+        for mode in (0, 1, 2):
+            got, st = emu(n, [gates], mode=mode)
             assert st["wide"] == st["passes"] > 0
             assert np.abs(got - want).max() <= 1e-12
+
+
+def test_passes_take_gates_of_later_parts(emu, port):
+    """Parts bounded by every touched qubit leave room in the tile: one call takes
+    fewer passes than parts, also when the gates in between stay behind."""
+    n = 16
+    for gates in (circuits.random_layered(n, 6, 9), circuits.random_u3_cz(n, 6, 9), _mixed(n, 3, 5)):
+        want = port.run(n, to_records(gates))
+        parts = partition.parts_to_gates(gates, partition.partition_acyclic(gates, 6))
+        got, st = emu(n, parts, mode=2)
+        assert st["passes"] < len(parts)
+        assert np.abs(got - want).max() <= 1e-12
+        # complex64 calls keep a pass per part
+        assert emu(n, parts, dtype=1, mode=2)[1]["passes"] >= len(parts)
 
 
 def test_other_gates_keep_the_general_form(emu):
