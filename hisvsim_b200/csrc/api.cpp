@@ -94,6 +94,63 @@ int check_state(const hs_state* st) {
   return HS_OK;
 }
 
+// Device memory of small states, kept when they are destroyed: mapping and
+// unmapping it costs 0.6 ms (at times several) per state, forty times the
+// planning of a small part, for programs that make a state per circuit.  A
+// block changes hands only when the device has finished everything (the wait
+// that cudaFree implies), whatever streams used it.  At most kKeptBytes per
+// device in blocks of up to kKeptBlock; given back when an allocation fails.
+constexpr size_t kKeptBlock = 16ull << 20, kKeptBytes = 32ull << 20;
+std::mutex g_kept_mu;
+struct KeptBlock {
+  void* p;
+  size_t bytes;
+};
+std::vector<KeptBlock> g_kept[64];
+size_t g_kept_bytes[64];
+
+cudaError_t state_alloc(void** p, size_t bytes) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && bytes <= kKeptBlock) {
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    auto& kept = g_kept[dev];
+    for (size_t i = 0; i < kept.size(); ++i)
+      if (kept[i].bytes == bytes) {
+        *p = kept[i].p;
+        g_kept_bytes[dev] -= bytes;
+        kept.erase(kept.begin() + i);
+        return cudaSuccess;
+      }
+  }
+  const cudaError_t first = cudaMalloc(p, bytes);
+  if (first != cudaErrorMemoryAllocation || dev >= 64) return first;
+  cudaGetLastError();
+  {
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    if (g_kept[dev].empty()) return first;
+    for (const KeptBlock& b : g_kept[dev]) cudaFree(b.p);
+    g_kept[dev].clear();
+    g_kept_bytes[dev] = 0;
+  }
+  return cudaMalloc(p, bytes);
+}
+
+void state_free(void* p, size_t bytes, int dev) {
+  int cur = -1;
+  if (dev >= 0 && dev < 64 && bytes <= kKeptBlock && cudaGetDevice(&cur) == cudaSuccess &&
+      cur == dev && cudaDeviceSynchronize() == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    if (g_kept_bytes[dev] + bytes <= kKeptBytes) {
+      g_kept[dev].push_back({p, bytes});
+      g_kept_bytes[dev] += bytes;
+      return;
+    }
+  }
+  cudaFree(p);
+}
+
 // Apply a permutation of bit positions to the data: the bit at position p
 // moves to position pi[p].  Done as two in-place involution passes of K2:
 // every cycle (c0 -> c1 -> ... ) is the product of two reflections.
@@ -234,7 +291,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
   st->n = num_qubits;
   st->dtype = dtype;
   const size_t bytes = amp_bytes(dtype) << num_qubits;
-  cudaError_t e = cudaMalloc(&st->amp, bytes);
+  cudaError_t e = state_alloc(&st->amp, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     delete st;
@@ -261,7 +318,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
 
 int hs_state_destroy(hs_state* st) {
   if (!st) return HS_OK;
-  if (st->amp) cudaFree(st->amp);
+  if (st->amp) state_free(st->amp, amp_bytes(st->dtype) << st->n, st->dev);
   st->amp = nullptr;
   if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev);
   delete st;

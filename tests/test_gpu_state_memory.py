@@ -1,0 +1,63 @@
+"""Device memory of small states is kept when they are destroyed: a new state
+starts from |0..0> whatever its memory held, work still in flight on another
+stream does not reach it, threads do not share blocks, and what is kept stays
+bounded."""
+import threading
+
+import numpy as np
+import pytest
+
+from hisvsim_b200 import abi, circuits
+from hisvsim_b200.gates import to_records
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,dtype", [(1, abi.C64), (10, abi.C128), (20, abi.C128), (21, abi.C128)])
+def test_new_state_starts_fresh(n, dtype):
+    import torch
+
+    rec = to_records(circuits.random_u3_cz(n, 3, n)) if n > 1 else None
+    side = torch.cuda.Stream()
+    for _ in range(4):
+        st = abi.State(n, dtype)
+        a = st.raw()
+        assert a[0] == 1 and not a[1:].any()
+        if rec is not None:
+            for _ in range(5):  # left in flight on a stream of the caller's
+                st.run_part(rec, stream=side.cuda_stream)
+        st.close()
+
+
+def test_threads_do_not_share_blocks(port):
+    n = 12
+    rec = [to_records(circuits.random_layered(n, 4, s)) for s in range(4)]
+    want = [port.run(n, r) for r in rec]
+    bad = []
+
+    def work(k):
+        abi.set_device(0)
+        for _ in range(20):
+            st = abi.State(n)
+            st.run_part(rec[k])
+            if np.abs(st.amplitudes() - want[k]).max() > 1e-12:
+                bad.append(k)
+            st.close()
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
+
+
+def test_kept_memory_is_bounded():
+    import torch
+
+    torch.cuda.init()
+    abi.State(4).close()
+    before = torch.cuda.mem_get_info()[0]
+    for n in list(range(1, 23)) * 2:
+        states = [abi.State(n) for _ in range(3)]
+        [s.close() for s in states]
+    # 32 MiB of states and the granularity of their mappings
+    assert before - torch.cuda.mem_get_info()[0] <= 96 << 20
