@@ -538,8 +538,12 @@ int launch_mlp_backward(const float* params, int in, const float* x, const float
                         float* loss_partial, int nblk, cudaStream_t s);
 int launch_mlp_reduce(const float* partial, const float* loss_partial, int nblk, int P,
                       float* grad, float* loss, cudaStream_t s);
-int launch_mlp_adam(float* params, const float* grad, float* m, float* v, int P, float lr,
-                    float beta1, float beta2, float eps, int step, cudaStream_t s);
+// Adam step `step` from the partials of a backward pass; *loss = their loss
+int launch_mlp_adam(float* params, const float* partial, const float* loss_partial, int nblk,
+                    float* m, float* v, int P, float lr, float beta1, float beta2, float eps,
+                    int step, float* loss, cudaStream_t s);
+// blocks (partials) of a backward pass over n samples, at most sms
+int mlp_backward_blocks(int n, int sms);
 
 }  // namespace hisv
 

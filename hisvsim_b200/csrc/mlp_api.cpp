@@ -42,10 +42,7 @@ struct DevBuf {  // scratch device buffer freed on scope exit
   }
 };
 
-int blocks_for(const hs_mlp* m, int n) {
-  const int b = (n + kMlpSamples - 1) / kMlpSamples;
-  return b < 1 ? 1 : (b > m->sms ? m->sms : b);
-}
+int blocks_for(const hs_mlp* m, int n) { return mlp_backward_blocks(n, m->sms); }
 
 }  // namespace
 
@@ -179,10 +176,8 @@ int hs_mlp_train(hs_mlp* m, const float* x, const float* y, int n, int epochs, i
       const int nblk = blocks_for(m, nb);
       HS_TRY(launch_mlp_backward(m->d_params, m->in, dx.p, dy.p, didx.p + b0, nb, 2.f / float(nb),
                                  m->d_partial, m->d_lpart, nblk, nullptr));
-      HS_TRY(launch_mlp_reduce(m->d_partial, m->d_lpart, nblk, m->P, m->d_grad, dl.p + st,
-                               nullptr));
-      HS_TRY(launch_mlp_adam(m->d_params, m->d_grad, m->d_m, m->d_v, m->P, lr, 0.9f, 0.999f,
-                             1e-8f, ++m->step, nullptr));
+      HS_TRY(launch_mlp_adam(m->d_params, m->d_partial, m->d_lpart, nblk, m->d_m, m->d_v, m->P, lr,
+                             0.9f, 0.999f, 1e-8f, ++m->step, dl.p + st, nullptr));
     }
     if (epoch_loss) {
       HS_CUDA(cudaMemcpy(losses.data(), dl.p, sizeof(float) * size_t(steps_per_epoch),
