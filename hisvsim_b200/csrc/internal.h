@@ -202,8 +202,10 @@ constexpr int kWideMaxTileBits = 12;
 constexpr int kWideMinTileBits = 10;  // CTAs of at least one full warp
 // thread bits: seven, and one to keep WideGroup at 64 bytes with its tables
 // on 16-byte boundaries (uniform vector loads; with 60 bytes a pass takes 2%
-// (rotations) to 13% (complex64, phase runs) longer)
+// (rotations) to 13% (complex64, phase runs) longer).  No thread has the eighth
+// bit set; its entry of tw holds the offset of the group's flipped bits.
 constexpr int kWideMaxThrBits = 8;
+constexpr int kWideFlipEntry = kWideMaxThrBits - 1;
 constexpr int kWideMaxGroups = 32;
 constexpr int kWideMaxSteps = 176;
 constexpr int kWideMaxSigns = 136;
@@ -256,7 +258,8 @@ struct alignas(16) WideGroup {
   uint32_t tw[kWideMaxThrBits]; // thread bit b: its tile bit (low half), byte offset (high half)
   uint16_t first_step, num_steps;
   uint8_t reg_tbit[kWideBits];
-  uint8_t pad[3];
+  uint8_t flip;    // at its end element e holds register index e ^ flip
+  uint8_t pad[2];
 };
 static_assert(sizeof(WideGroup) == 64, "WideGroup layout");
 
@@ -273,8 +276,11 @@ struct WideProgram {
   // shared slot cthr(t) ^ cslot[k] (bytes); both are sums over the thread's bits
   uint64_t gthr[kWideMaxThrBits], gchunk[kWideMaxChunks];
   uint32_t cthr[kWideMaxThrBits], cslot[kWideMaxChunks];
-  // the last group's direct store: global offset of thread and register bits
-  uint64_t sthr[kWideMaxThrBits], sreg[kWideBits];
+  // the last group's direct store: offsets of thread bits, the step of each
+  // register bit, the offset of element 0
+  uint64_t sthr[kWideMaxThrBits];
+  int64_t sreg[kWideBits];
+  uint64_t sbase;
   WideGroup groups[kWideMaxGroups];
   WideStep steps[kWideMaxSteps];
   WideSign signs[kWideMaxSigns];

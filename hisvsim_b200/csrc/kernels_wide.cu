@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
       if (last) {
         // elements in Gray-code order: each address is the previous one plus
         // or minus one register bit's offset (one live pointer)
-        V* p = sv + gbase;
+        V* p = sv + gbase + P.sbase;
 #pragma unroll
         for (int b = 0; b < kWideMaxThrBits; ++b)
           if ((t >> b) & 1u) p += P.sthr[b];
@@ -395,10 +395,11 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
         }
         cp_async_wait();  // the next tile's copies (the only ones in flight)
       } else {
+        const uint32_t a1 = a0 ^ G.tw[kWideFlipEntry];
 #pragma unroll
         for (int e = 0; e < E; ++e)
-          if (HS_IN_BOUNDS((a0 ^ ux(e)) + sizeof(V) <= tile_bytes, kBoundsK1))
-            *reinterpret_cast<V*>(smem_raw + (a0 ^ ux(e))) = v[e];
+          if (HS_IN_BOUNDS((a1 ^ ux(e)) + sizeof(V) <= tile_bytes, kBoundsK1))
+            *reinterpret_cast<V*>(smem_raw + (a1 ^ ux(e))) = v[e];
       }
       __syncthreads();
     }

@@ -103,12 +103,20 @@ struct Rot {
   int form;
   double t, s;
   cplx g0, g1;       // left diagonal
+  bool flip;         // wide programs: X after the shears (and the left diagonal of X)
+  bool none;         // with flip: no shears at all (an anti-diagonal gate)
 };
 
 // Two-shear forms are used when cos(theta/2) >= kShearPivot: their
 // coefficients stay below ~3 and the pending scale of a qubit within
 // [kShearPivot^2, kShearPivot^-2].
 constexpr double kShearPivot = 0.4;
+// Wide programs write the other rotations as X times one whose cosine is their
+// sine, X being a relabelling of the thread's elements that costs nothing; so
+// every rotation takes two shears.  Complex64 states turn at a larger cosine:
+// a qubit's pending scale then stays within [0.36, 2.8], and the product over
+// 40 qubits, with the global factor's 2^+-24, within the type's exponents.
+constexpr double kFlipPivotC64 = 0.6;
 
 // W = U diag(1, r): U unitary, r the qubit's pending factor, so W's first
 // column is a unit vector and its second |r| = rho times one.  With
@@ -126,7 +134,9 @@ constexpr double kShearPivot = 0.4;
 // the qubit's two values, which complex128 frames carry (`scaled`);
 // complex64 states keep form 0.  False when W is not of the form above to
 // 1e-12 (custom C1 matrices need not be).
-bool factor_rotation(const cplx* W, bool scaled, Rot* R) {
+// `pivot` > 0: cosines below it are turned (Rot::flip).
+bool factor_rotation(const cplx* W, bool scaled, double pivot, Rot* R) {
+  R->flip = R->none = false;
   const double c = std::abs(W[0]), s = std::abs(W[2]);
   const double rho = std::hypot(std::abs(W[1]), std::abs(W[3]));
   const double tol = 1e-12;
@@ -135,6 +145,17 @@ bool factor_rotation(const cplx* W, bool scaled, Rot* R) {
   if (!(std::fabs(c * c + s * s - 1.0) <= tol) ||
       !(std::norm(std::conj(W[0]) * w1 + std::conj(W[2]) * w3) <= tol * tol))
     return false;
+  if (c < pivot) {  // W = X V = X diag(g0, g1) M diag(1, b1) = diag(g1, g0) X M diag(1, b1)
+    if (c == 0.0) {
+      *R = Rot{false, 0.0, 0.0, cplx(1.0), 1, 0.0, 0.0, W[1], W[2], true, true};
+      return true;
+    }
+    const cplx V[4] = {W[2], W[3], W[0], W[1]};
+    if (!factor_rotation(V, scaled, 0.0, R)) return false;
+    std::swap(R->g0, R->g1);
+    R->flip = true;
+    return true;
+  }
   cplx a0, a1, b1;
   double cc = c, ss = s;
   if (c > 0.0 && s > 0.0) {
@@ -305,8 +326,8 @@ bool out_of_range(cplx G, double lim) {
 // `scaled`: rotations may leave real scales in the frames (complex128);
 // `lim`: the global factor's scale is flushed once it leaves 2^+-lim; `split`:
 // diagonal gates become phases (split_diagonal), for wide programs.
-void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double lim, bool split,
-                  std::vector<RGate>* out) {
+void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double pivot, double lim,
+                  bool split, std::vector<RGate>* out) {
   if (g.nt == 0) return;
   const bool diag = is_diagonal(g);
   if (g.nt == 1 && g.nc == 0) {
@@ -328,7 +349,7 @@ void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double lim, bool
     cplx W[4] = {g.m[0], g.m[1] * rq, g.m[2], g.m[3] * rq};
     RGate x;
     x.g = g;
-    if (factor_rotation(W, scaled, &x.rot)) {
+    if (factor_rotation(W, scaled, pivot, &x.rot)) {
       x.kind = RK_ROT;
       F->G *= x.rot.g0;
       F->r[q] = x.rot.g1 / x.rot.g0;
@@ -386,11 +407,11 @@ void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double lim, bool
 }
 
 // every part in turn; the gates keep their part's number
-void rewrite(const std::vector<std::vector<LoweredGate>>& parts, Frames* F, bool scaled, double lim,
-             bool split, std::vector<RGate>* out) {
+void rewrite(const std::vector<std::vector<LoweredGate>>& parts, Frames* F, bool scaled,
+             double pivot, double lim, bool split, std::vector<RGate>* out) {
   for (size_t p = 0; p < parts.size(); ++p) {
     const size_t first = out->size();
-    for (const auto& g : parts[p]) rewrite_gate(g, F, scaled, lim, split, out);
+    for (const auto& g : parts[p]) rewrite_gate(g, F, scaled, pivot, lim, split, out);
     for (size_t i = first; i < out->size(); ++i) (*out)[i].part = int(p);
   }
 }
@@ -894,6 +915,34 @@ struct RecSet {
   }
 };
 
+// Whether every gate of a call ends up in wide programs, which alone hold
+// rotations with a flip: the kinds wide_gate takes, and pending factors (from
+// earlier calls, custom gates among them) that factor_rotation can take in.
+bool all_wide(const std::vector<std::vector<LoweredGate>>& parts, const Frames& F) {
+  for (const cplx& r : F.r)
+    if (!(std::norm(r) > 1e-6 && std::norm(r) < 1e6)) return false;
+  for (const auto& gates : parts)
+    for (const LoweredGate& g : gates) {
+      if (g.nt == 0) continue;
+      if (is_diagonal(g)) {
+        for (int i = 0; i < (g.nt == 1 ? 2 : 4); ++i)
+          if (std::fabs(std::norm(g.m[(g.nt == 1 ? 3 : 5) * i]) - 1.0) > 2e-12) return false;
+        if (g.nt == 2 && g.nc == HS_MAX_CONTROLS) return false;
+      } else if (g.nt == 1 && g.nc == 0) {
+        // unitary, well within what factor_rotation asks for
+        const double tol = 2.5e-13;
+        const cplx o = std::conj(g.m[0]) * g.m[1] + std::conj(g.m[2]) * g.m[3];
+        if (!(std::fabs(std::norm(g.m[0]) + std::norm(g.m[2]) - 1.0) <= tol &&
+              std::fabs(std::norm(g.m[1]) + std::norm(g.m[3]) - 1.0) <= tol &&
+              std::norm(o) <= tol * tol))
+          return false;
+      } else if (!(g.nt == 1 && is_x(g.m)) && !(g.nt == 2 && g.nc == 0 && is_swap4(g.m))) {
+        return false;
+      }
+    }
+  return true;
+}
+
 // An op of a group before it is scheduled.
 struct WideRec {
   enum Kind { kRot, kNeg, kPhase, kCx, kSwap } kind;
@@ -905,17 +954,11 @@ struct WideRec {
   cplx c{1.0, 0.0};      // kPhase
   const Rot* rot = nullptr;
   bool z = false;        // kRot: its phase part is still to be applied
+  bool global = false;   // kPhase: a flush's global factor
   bool done = false;
   bool diag() const { return kind == kNeg || kind == kPhase; }
   bool uniform() const { return cthr == 0 && couter == 0; }
 };
-
-uint32_t elements_of(uint32_t mask) {  // elements whose register bits cover mask
-  uint32_t w = 0;
-  for (uint32_t e = 0; e < 32; ++e)
-    if ((e & mask) == mask) w |= 1u << e;
-  return w;
-}
 
 void wide_records(const SlotGate& sg, const Layout& L, const std::vector<int>& q2s,
                   std::vector<WideRec>* out) {
@@ -941,7 +984,8 @@ void wide_records(const SlotGate& sg, const Layout& L, const std::vector<int>& q
       out->push_back(x);
     }
     w.c = r.flG;
-    if (w.c != cplx(1.0, 0.0)) out->push_back(w);
+    w.global = true;
+    out->push_back(w);
     return;
   }
   const LoweredGate& g = r.g;
@@ -981,7 +1025,16 @@ void wide_records(const SlotGate& sg, const Layout& L, const std::vector<int>& q
 // rotation that is next on its bit and the register-only factors of modulus 1
 // join the table of the first step that needs one.  `reserve`: coefficients to
 // be left for the program's later groups.
-int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* G, int reserve) {
+//
+// Flips (Rot::flip) relabel the elements: element e holds the amplitude of
+// register index e ^ xm.  A rotation on a flipped bit has its pair's roles, so
+// its two shears, exchanged; its phase turns the other amplitude back instead,
+// up to a global factor that `gamma` collects for the next flush; diagonal ops
+// are written for e ^ xm (a condition "bit is 0" as the unconditional factor
+// times its inverse on the bit, a CZ as one and a Z).  The group's end stores
+// element e where e ^ xm belongs.
+int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* G, int reserve,
+               cplx* gamma) {
   const int n = int(rec.size()), size = 1 << kWideBits;
   G->first_step = uint16_t(P->nsteps);
   // dependencies as bit sets over the ops: the last non-diagonal op on a bit,
@@ -1048,6 +1101,16 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     done.add(i);
     --left;
   };
+  uint32_t xm = 0;
+  struct Piece {  // a factor of a run
+    uint32_t mask, cthr;
+    uint64_t couter;
+    cplx c;
+  };
+  std::vector<Piece> pieces;
+  auto is_pair = [&](int i) {
+    return rec[i].kind == WideRec::kNeg && rec[i].uniform() && __builtin_popcount(rec[i].mask) == 2;
+  };
   while (left > 0 || pend_any) {
     if (P->nsteps >= kWideMaxSteps) return set_error(HS_E_UNSUPPORTED, "too many steps in a pass");
     WideStep& S = P->steps[P->nsteps++];
@@ -1084,17 +1147,55 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     });
     touched |= moved;
     const bool last = touched == 0;  // diagonal ops alone are left
+    if (xm) {
+      // runs with several flipped bits, or more pieces than there is room for:
+      // undo those flips first (a step of plain X)
+      uint32_t undo = 0;
+      int extra = 0;
+      open.each([&](int i) {
+        if (is_sign(i) || is_pair(i) || !(rec[i].mask & xm) || !(last || (rec[i].mask & touched)))
+          return;
+        if (__builtin_popcount(rec[i].mask & xm) > 1 || rec[i].c == cplx(0.0, 0.0))
+          undo |= rec[i].mask & xm;
+        ++extra;
+      });
+      const int room = std::min(kWideMaxConds - P->nconds, kWideMaxOps - 8 - P->nwops) -
+                       (reserve / 2 + left);
+      if (extra > room) undo |= xm;
+      if (undo) {
+        S.apply = pend_any && (pend & undo);
+        if (S.apply) {
+          pend_any = false;
+          pend = 0;
+        }
+        for (int j = 0; j < kWideBits; ++j) {
+          if (!((undo >> j) & 1u)) continue;
+          WideOp& op = P->ops[P->nwops++];
+          std::memset(&op, 0, sizeof(op));
+          op.code = wk_cx;
+          op.reg = uint8_t(j);
+          op.elems = ~0u;
+          ++S.nperms;
+        }
+        xm &= ~undo;
+        continue;
+      }
+    }
     // ---- diagonal ops
     std::vector<int> run;
+    auto add_sign = [&](uint32_t bits, uint32_t cthr, uint64_t couter) {
+      WideSign& q = P->signs[P->nsigns++];
+      q.bits = bits;
+      q.cthr = cthr;
+      q.couter = couter;
+      ++S.nsigns;
+      pend_any = true;
+      pend |= bits & 31u;
+    };
     open.each([&](int i) {
       if (is_sign(i)) {
-        WideSign& q = P->signs[P->nsigns++];
-        q.bits = rec[i].mask ? rec[i].mask : 32u;
-        q.cthr = rec[i].cthr;
-        q.couter = rec[i].couter;
-        ++S.nsigns;
-        pend_any = true;
-        pend |= rec[i].mask;
+        add_sign(rec[i].mask == 0 || (rec[i].mask & xm) ? rec[i].mask | 32u : rec[i].mask,
+                 rec[i].cthr, rec[i].couter);
         finish(i);
       } else if (last || (rec[i].mask & touched)) {
         run.push_back(i);
@@ -1141,75 +1242,101 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
         finish(i);
       });
       S.table = uint16_t(P->ncoef);
-      for (int e = 0; e < size; ++e) push_amp_coef(f[e]);
+      const cplx first = f[xm];  // element 0's, left out of the table
+      *gamma *= first;
+      for (int e = 0; e < size; ++e)
+        push_amp_coef(xm ? f[uint32_t(e) ^ xm] * std::conj(first) : f[e]);
     }
+    // pairs on flipped bits leave a Z on the other bit
+    for (int i : run)
+      if (is_pair(i) && (rec[i].mask & xm)) {
+        const uint32_t a = rec[i].mask & (0u - rec[i].mask), b = rec[i].mask ^ a;
+        add_sign(((xm & a) ? b : 0u) | ((xm & b) ? a : 0u) | ((xm & a) && (xm & b) ? 32u : 0u), 0, 0);
+      }
     S.apply = pend_any && ((pend & moved) || (last && left == int(run.size())));
     if (S.apply) {
       pend_any = false;
       pend = 0;
     }
     // negations of register pairs, then runs, one per register mask
-    for (size_t k = 0; k < run.size();) {
-      const WideRec& x = rec[run[k]];
-      if (x.kind != WideRec::kNeg || !x.uniform() || __builtin_popcount(x.mask) != 2) {
-        ++k;
-        continue;
+    pieces.clear();
+    for (int i : run) {
+      const WideRec& x = rec[i];
+      if (is_pair(i)) {
+        WideOp& op = P->ops[P->nwops++];
+        std::memset(&op, 0, sizeof(op));
+        op.code = wk_neg;
+        op.reg = uint8_t(wide_pair(__builtin_ctz(x.mask), 31 - __builtin_clz(x.mask)));
+        ++S.nruns;
+      } else if (x.mask & xm) {  // one flipped bit: on 0 = everywhere, undone on 1
+        pieces.push_back({x.mask & ~xm, x.cthr, x.couter, x.c});
+        pieces.push_back({x.mask, x.cthr, x.couter, 1.0 / x.c});
+      } else {
+        cplx c = x.c;
+        if (x.global) {
+          c *= *gamma;
+          *gamma = 1.0;
+        }
+        if (c != cplx(1.0, 0.0)) pieces.push_back({x.mask, x.cthr, x.couter, c});
       }
-      WideOp& op = P->ops[P->nwops++];
-      std::memset(&op, 0, sizeof(op));
-      op.code = wk_neg;
-      op.reg = uint8_t(wide_pair(__builtin_ctz(x.mask), 31 - __builtin_clz(x.mask)));
-      ++S.nruns;
-      finish(run[k]);
-      run.erase(run.begin() + k);
+      finish(i);
     }
-    while (!run.empty()) {
+    for (size_t k = 0; k < pieces.size(); ++k) {
+      const uint32_t mask = pieces[k].mask;
+      if (mask > 31u) continue;  // taken by an earlier run
       WideOp& op = P->ops[P->nwops++];
       std::memset(&op, 0, sizeof(op));
       op.code = wk_run;
-      op.reg = uint8_t(rec[run[0]].mask);
+      op.reg = uint8_t(mask);
       op.first = uint16_t(P->nconds);
       cplx c = 1.0;
-      std::vector<int> rest;
-      for (int i : run) {
-        if (rec[i].mask != op.reg) {
-          rest.push_back(i);
-          continue;
-        }
-        if (rec[i].uniform()) {
-          c *= rec[i].c;
+      for (size_t l = k; l < pieces.size(); ++l) {
+        Piece& x = pieces[l];
+        if (x.mask != mask) continue;
+        if (x.cthr == 0 && x.couter == 0) {
+          c *= x.c;
         } else {
           WideCond& q = P->conds[P->nconds++];
-          q.cthr = rec[i].cthr;
-          q.couter = rec[i].couter;
-          q.coef = uint32_t(push_coef(rec[i].c));
+          q.cthr = x.cthr;
+          q.couter = x.couter;
+          q.coef = uint32_t(push_coef(x.c));
           ++op.n;
         }
-        finish(i);
+        x.mask = ~0u;
       }
       if (c != cplx(1.0, 0.0)) op.coef = uint16_t(push_coef(c));
       ++S.nruns;
-      run = rest;
     }
+    uint32_t flips = 0;
     for (int j = 0; j < kWideBits; ++j) {
       if (rot[j] < 0) continue;
       const Rot& r = *rec[rot[j]].rot;
-      S.forms |= uint16_t(r.form << (2 * j));
-      S.rot[j] = uint16_t(push_amp_coef(cplx(r.t, r.s)));
-      if (rec[rot[j]].z) {
-        S.zmask |= uint8_t(1u << j);
-        push_amp_coef(cplx(r.tz, r.sz));
+      const bool turned = (xm >> j) & 1u;  // the pair's roles are exchanged
+      if (!r.none) {
+        S.forms |= uint16_t((turned ? 3 - r.form : r.form) << (2 * j));
+        S.rot[j] = uint16_t(push_amp_coef(turned ? cplx(r.s, r.t) : cplx(r.t, r.s)));
+        if (rec[rot[j]].z) {
+          S.zmask |= uint8_t(1u << j);
+          push_amp_coef(turned ? cplx(-r.tz, -r.sz) : cplx(r.tz, r.sz));
+          if (turned) *gamma *= r.b1;
+        }
       }
+      if (r.flip) flips |= 1u << j;
       finish(rot[j]);
     }
+    xm ^= flips;
     for (int i : perms) {
       WideOp& op = P->ops[P->nwops++];
       std::memset(&op, 0, sizeof(op));
       if (rec[i].kind == WideRec::kCx) {
         op.code = wk_cx;
         op.reg = uint8_t(rec[i].j);
-        op.elems = elements_of(rec[i].mask & ~rec[i].target);
+        const uint32_t ctl = rec[i].mask & ~rec[i].target;
+        for (uint32_t e = 0; e < uint32_t(size); ++e)
+          if (((e ^ xm) & ctl) == ctl) op.elems |= 1u << e;
       } else {
+        const uint32_t a = (xm >> rec[i].j) & 1u, b = (xm >> rec[i].jb) & 1u;
+        if (a != b) xm ^= rec[i].mask;  // the flips change places too
         op.code = wk_swap;
         op.reg = uint8_t(wide_pair(rec[i].j, rec[i].jb));
       }
@@ -1219,6 +1346,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
       finish(i);
     }
   }
+  G->flip = uint8_t(xm);
   G->num_steps = uint16_t(P->nsteps - G->first_step);
   return HS_OK;
 }
@@ -1236,7 +1364,10 @@ void finish_wide(WideProgram* P, const std::vector<uint32_t>& regs, int dtype) {
   }
   for (int g = 0; g < P->ngroups; ++g) {
     WideGroup& G = P->groups[g];
-    for (int j = 0; j < kWideBits; ++j) G.dx[j] = off[G.reg_tbit[j]];
+    for (int j = 0; j < kWideBits; ++j) {
+      G.dx[j] = off[G.reg_tbit[j]];
+      if ((G.flip >> j) & 1u) G.tw[kWideFlipEntry] ^= G.dx[j];
+    }
     int b = 0;
     for (int tb = 0; tb < P->m; ++tb) {
       if ((regs[g] >> tb) & 1u) continue;
@@ -1246,7 +1377,11 @@ void finish_wide(WideProgram* P, const std::vector<uint32_t>& regs, int dtype) {
     }
   }
   const WideGroup& last = P->groups[P->ngroups - 1];
-  for (int j = 0; j < kWideBits; ++j) P->sreg[j] = slot[last.reg_tbit[j]];
+  for (int j = 0; j < kWideBits; ++j) {  // (a flipped bit's element 0 is the one with the bit set)
+    const bool f = (last.flip >> j) & 1u;
+    P->sreg[j] = f ? -int64_t(slot[last.reg_tbit[j]]) : int64_t(slot[last.reg_tbit[j]]);
+    if (f) P->sbase += slot[last.reg_tbit[j]];
+  }
   // chunk c = t + k * threads holds tile indices [c << sh, (c + 1) << sh)
   P->per_thr = ((1 << P->m) >> sh) >> thr_bits;
   for (int b = 0; b < thr_bits; ++b) {
@@ -1267,7 +1402,7 @@ void finish_wide(WideProgram* P, const std::vector<uint32_t>& regs, int dtype) {
 int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
                     const std::vector<SlotGate>& sgs, std::vector<int> remaining,
                     const std::vector<int>& tile, const std::vector<int>& tbit_of_slot,
-                    std::vector<PlannedPass>* passes) {
+                    cplx* gamma, std::vector<PlannedPass>* passes) {
   const int m = int(tile.size());
   WideProgram* P = nullptr;
   std::vector<uint32_t> regs_of;
@@ -1321,7 +1456,7 @@ int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
     int reserve = 2;
     for (int x : rest)
       reserve += sgs[x].rg->kind == RK_FLUSH ? 2 + 2 * int(sgs[x].rg->flq.size()) : 2;
-    HS_TRY(wide_steps(rec, dtype, P, &G, reserve));
+    HS_TRY(wide_steps(rec, dtype, P, &G, reserve, gamma));
     remaining.swap(rest);
   }
   finish_wide(P, regs_of, dtype);
@@ -1365,7 +1500,10 @@ int plan_chunks(int n, const std::vector<int>& q2s,
   // the scaled rotation forms and non-unitary diagonal gates)
   const double lim = dtype == HS_DTYPE_C64 ? 24.0 : 48.0;
   const bool wide = sink && use_wide(n, dtype);
-  rewrite(gates, fr, dtype == HS_DTYPE_C128, lim, wide, &rg);
+  const bool flips = wide && (tile_bits_hint <= 0 || tile_bits_hint >= kWideMinTileBits) &&
+                     all_wide(gates, *fr);
+  const double pivot = !flips ? 0.0 : dtype == HS_DTYPE_C128 ? kShearPivot : kFlipPivotC64;
+  rewrite(gates, fr, dtype == HS_DTYPE_C128 || flips, pivot, lim, wide, &rg);
   if (flush) {
     if (!fr->identity()) {
       rg.push_back(flush_gate(fr));
@@ -1480,6 +1618,7 @@ int plan_chunks(int n, const std::vector<int>& q2s,
       merged.size() < chunks.size())
     chunks.swap(merged);
   std::vector<PlannedPass> passes;
+  cplx gamma = 1.0;  // global factor the wide programs leave (wide_steps)
   for (const Chunk& c : chunks) {
     const std::vector<int>& chunk = c.gates;
     const bool wide_chunk = c.wide;
@@ -1510,7 +1649,7 @@ int plan_chunks(int n, const std::vector<int>& q2s,
       return HS_OK;
     };
     if (wide_chunk && m >= kWideMinTileBits) {
-      HS_TRY(plan_wide_chunk(n, dtype, q2s, sgs, chunk, tile, tbit_of_slot, &passes));
+      HS_TRY(plan_wide_chunk(n, dtype, q2s, sgs, chunk, tile, tbit_of_slot, &gamma, &passes));
       HS_TRY(hand_over());
       continue;
     }
@@ -1564,6 +1703,8 @@ int plan_chunks(int n, const std::vector<int>& q2s,
       Emitter E{P, &q2s};
       for (int x : members) {
         const SlotGate& sg = sgs[x];
+        if (sg.rg->kind == RK_ROT && sg.rg->rot.flip)
+          return set_error(HS_E_UNSUPPORTED, "a flipped rotation outside a wide program");
         if (sg.rg->kind == RK_ROT)
           emit_rot(sg, L, E);
         else if (sg.rg->kind == RK_FLUSH)
@@ -1576,6 +1717,17 @@ int plan_chunks(int n, const std::vector<int>& q2s,
       remaining = later;
     }
     if (sink) HS_TRY(hand_over());
+  }
+  if (gamma != cplx(1.0, 0.0) && !flush) {
+    fr->G *= gamma;
+  } else if (gamma != cplx(1.0, 0.0)) {
+    // left by rotations planned after the flush (their qubits had nothing
+    // pending): a flush of its own
+    std::vector<std::vector<LoweredGate>> nothing(1);
+    Frames g;
+    g.reset(n);
+    g.G = gamma;
+    return plan_chunks(n, q2s, nothing, &g, true, tile_bits_hint, dtype, nullptr, sink);
   }
   if (!sink)
     for (auto& P : *programs) finish_layout(&P, dtype);

@@ -167,7 +167,7 @@ struct Emu {
         for (int t = 0; t < nthr; ++t) {
           uint32_t tw = 0;
           for (int b = 0; b < kWideMaxThrBits; ++b)
-            if ((t >> b) & 1) tw ^= G.tw[b];
+            if ((t >> b) & 1) tw ^= G.tw[b];  // (t < 2^7: never the flips' entry)
           const uint32_t thr = tw & 0xffffu, a0 = tw >> 16;
           auto at = [&](int e) {
             uint32_t a = a0;
@@ -183,7 +183,7 @@ struct Emu {
             step(v, P.steps[s], thr, gbase, z);
           need(z == 0, "signs left at the end of a group");
           if (last) {
-            uint64_t p = gbase;
+            uint64_t p = gbase + P.sbase;
             for (int b = 0; b < bits; ++b)
               if ((t >> b) & 1) p += P.sthr[b];
             for (unsigned e = 0; e < (1u << kWideBits); ++e) {
@@ -194,7 +194,11 @@ struct Emu {
               sv[q] = v[e];
             }
           } else {
-            for (unsigned e = 0; e < (1u << kWideBits); ++e) buf[at(e)] = v[e];
+            for (unsigned e = 0; e < (1u << kWideBits); ++e) {
+              need((a0 ^ G.tw[kWideFlipEntry]) < tile_bytes, "flip offset out of range");
+              need((at(e) * ab ^ G.tw[kWideFlipEntry]) == at(e ^ G.flip) * ab, "flip offset");
+              buf[at(e ^ G.flip)] = v[e];
+            }
           }
         }
       }

@@ -143,6 +143,39 @@ def test_passes_take_gates_of_later_parts(emu, port):
         assert emu(n, parts, dtype=1, mode=2)[1]["passes"] >= len(parts)
 
 
+def test_flips_and_custom_gates(emu, port):
+    """Rotations beyond the pivot (X and Y among them) next to every gate that
+    meets a flipped bit, and frames that custom gates leave far from 1 between
+    calls: those calls do without flips."""
+    rng = np.random.default_rng(17)
+    n = 12
+    g = []
+    for _ in range(5):
+        for q in range(n):
+            g.append([Gate("X", (q,)), Gate("Y", (q,)), Gate("RY", (q,), params=(3.0,)),
+                      Gate("U3", (q,), params=(2.9, float(rng.uniform(0, 6)), 1.0))][int(rng.integers(4))])
+        for _ in range(8):
+            q = [int(v) for v in rng.permutation(n)[:4]]
+            g.append([Gate("Z", (q[0],), (q[1],)), Gate("Z", (q[0],), (q[1], q[2])),
+                      Gate("X", (q[0],), (q[1], q[2])), Gate("SWAP", (q[0], q[1])),
+                      Gate("RZZ", (q[0], q[1]), params=(0.7,)),
+                      Gate("C1", (q[0],), (q[1], q[2], q[3]), params=(1.0, 0.0, 0.0, 1j))][int(rng.integers(6))])
+    want = port.run(n, to_records(g))
+    for split, k in ((partition.partition_acyclic, 12), (partition.partition_dfs, 6)):
+        parts = partition.parts_to_gates(g, split(g, k))
+        for mode in (0, 1, 2):
+            got, st = emu(n, parts, mode=mode)
+            assert st["wide"] == st["passes"]
+            assert np.abs(got - want).max() <= 1e-12
+            got, _ = emu(n, parts, dtype=1, mode=mode)
+            assert np.abs(got - want).max() <= 1e-5
+    # a first call whose custom diagonal leaves a factor of 1e4 pending
+    parts = [[Gate("H", (q,)) for q in range(n)] + [Gate("C1", (3,), params=(1.0, 0.0, 0.0, 1e4))], g]
+    want = port.run(n, to_records([x for p in parts for x in p]))
+    got, _ = emu(n, parts, mode=0)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
 def test_other_gates_keep_the_general_form(emu):
     """Gates outside the wide form (dense controlled, two-qubit dense, custom
     non-unitary diagonals, controlled swaps) and small states are not taken."""
