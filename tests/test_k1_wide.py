@@ -121,7 +121,14 @@ def test_program_limits(emu, port):
         a, b = (int(x) for x in rng.choice(n, 2, replace=False))
         many.append(Gate("U1", (a,), (b,), params=(u()[0],)) if i % 2 else Gate("Z", (a,), (b,)))
     many += [Gate("U3", (q,), params=u()) for q in range(n)]
-    for gates in (deep, many):
+    swaps = [g for i in range(140) for g in (Gate("SWAP", tuple(int(x) for x in rng.choice(n, 2, replace=False))),
+                                             Gate("RY", (i % n,), params=(3.0,)))]
+    # phases and pairs on bits that flips keep turning over
+    turned = [g for i in range(120) for g in (
+        Gate("RY", (i % 5,), params=(3.0,)), Gate("Z", (i % 5,), ((i + 1) % 5,)),
+        Gate("C1", (i % 5,), ((i + 1) % 5, (i + 2) % 5), params=(1.0, 0.0, 0.0, 1j)),
+        Gate("U1", (i % 5,), (5 + i % 7,), params=(0.1 + i,)))]
+    for gates in (deep, many, swaps, turned):
         want = port.run(n, to_records(gates))
         for mode in (0, 1, 2):
             got, st = emu(n, [gates], mode=mode)
