@@ -506,7 +506,7 @@ def config1_form(args, abi, peak_gbs, pg, device):
                         f"complex128",
             "circuit_s": t, "passes_per_step": passes, "value": len(gates) * float(1 << n) / t,
             "unit": UNIT,
-            "roofline": {"bound": "hbm", "kernel": "k1_part", "avg_launch_ms": k1_ms,
+            "roofline": {"bound": "hbm", "kernel": "k1_wide", "avg_launch_ms": k1_ms,
                          "achieved": bpp / (k1_ms / 1e3) / 1e9, "peak": peak_gbs, "unit": "GB/s",
                          "frac": bpp / (k1_ms / 1e3) / 1e9 / peak_gbs},
             "high_qubit_parts": {"part_on_top_qubits_ms": ms_hi, "part_on_low_qubits_ms": ms_lo,
@@ -771,7 +771,7 @@ def main():
             "norm": norm,
             "roofline": {"bound": "hbm", "achieved": k1_gbs, "peak": peak_gbs, "unit": "GB/s",
                          "frac": k1_gbs / peak_gbs, "traffic": traffic, "peak_source": peak_src,
-                         "kernel": "k1_part", "algorithmic_bytes_per_launch": bytes_per_pass,
+                         "kernel": "k1_wide", "algorithmic_bytes_per_launch": bytes_per_pass,
                          "avg_launch_ms": k1_avg_ms, "fp64": fp64},
             "qubit_bounded_parts": alt,
             "fused": fused,

@@ -262,7 +262,9 @@ __device__ __forceinline__ void apply_deferred(V (&v)[1 << R], const Deferred& d
 // instantiation when it holds nothing else, because a switch over every op
 // kind in the loop makes the compiler reconcile the register copies of all
 // cases at its join (measured: ~50 register moves per op and 160 instead of
-// ~110 registers per thread).
+// ~110 registers per thread).  States of ten qubits and more run such programs
+// in the wide form (kernels_wide.cu) unless tiles below 2^10 or 8 amplitudes
+// per thread were asked for.
 template <int R, bool FULL, bool FAST, typename V>
 __device__ __forceinline__ void run_op(V (&v)[1 << R], const DevOp& op, const double2* s_coef,
                                        uint32_t thr, uint64_t gbase, Deferred& dfr,

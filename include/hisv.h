@@ -208,10 +208,10 @@ int hs_plan_stats(int num_qubits, int dtype, const hs_gate* gates, int num_gates
 
 /* Tile-size override for K1 (0 = automatic).  Returns the previous value. */
 int hs_set_tile_qubits(int m);
-/* Amplitudes per thread of K1 passes: 2^r with r = 4 (default; complex128
- * tiles of 2^10 in CTAs of 64 threads, or 2^11 in CTAs of 128) or 3 (CTAs
- * twice as wide, register groups of three qubits).  Returns the previous
- * value. */
+/* Amplitudes per thread of K1 passes.  r = 4 (default): 32 for passes of
+ * rotations, diagonal gates, controlled X and swaps on ten qubits and more, 16
+ * for the others; r = 3: 8 for every pass (wider CTAs, register groups of
+ * three qubits).  Returns the previous value. */
 int hs_set_k1_reg_bits(int r);
 
 /* ---- precision form (complex64 state, fused unitaries on the tensor cores) --
