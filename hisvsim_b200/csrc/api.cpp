@@ -448,14 +448,20 @@ int hs_part_run_carry(hs_state* st, hs_frames* fr, const hs_gate* gates, int num
   if (num_gates == 0) return HS_OK;
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gates, num_gates, &lg));
-  return run_lowered(st, lg, &fr->fr, false, S(stream));
+  Frames next = fr->fr;  // (an error leaves the factors as they were)
+  HS_TRY(run_lowered(st, lg, &next, false, S(stream)));
+  fr->fr = std::move(next);
+  return HS_OK;
 }
 
 int hs_frames_flush(hs_state* st, hs_frames* fr, void* stream) {
   HS_TRY(check_state(st));
   if (!fr || fr->n != st->n) return set_error(HS_E_INVALID, "frames missing or of another size");
   if (fr->fr.identity()) return HS_OK;
-  return run_lowered(st, {}, &fr->fr, true, S(stream));
+  Frames next = fr->fr;
+  HS_TRY(run_lowered(st, {}, &next, true, S(stream)));
+  fr->fr = std::move(next);
+  return HS_OK;
 }
 
 int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,

@@ -135,16 +135,24 @@ constexpr double kFlipPivotC64 = 0.6;
 // complex64 states keep form 0.  False when W is not of the form above to
 // 1e-12 (custom C1 matrices need not be).
 // `pivot` > 0: cosines below it are turned (Rot::flip).
+
+// Whether W (its second column scaled to a unit vector) is of that form to `tol`.
+// A lower left entry of exactly 0 is not: the gate is diagonal, or its upper
+// right entry is the rounding residue of a product that should have been
+// (custom C1 matrices), and it is applied as the matrix it is.
+bool rotates(const cplx& w0, const cplx& w1, const cplx& w2, const cplx& w3, double tol) {
+  const double c = std::abs(w0), s = std::abs(w2);
+  return s != 0.0 && std::fabs(c * c + s * s - 1.0) <= tol &&
+         std::norm(std::conj(w0) * w1 + std::conj(w2) * w3) <= tol * tol;
+}
+
 bool factor_rotation(const cplx* W, bool scaled, double pivot, Rot* R) {
   R->flip = R->none = false;
   const double c = std::abs(W[0]), s = std::abs(W[2]);
   const double rho = std::hypot(std::abs(W[1]), std::abs(W[3]));
-  const double tol = 1e-12;
   if (!(rho > 0.0) || !std::isfinite(rho)) return false;
   const cplx w1 = W[1] / rho, w3 = W[3] / rho;
-  if (!(std::fabs(c * c + s * s - 1.0) <= tol) ||
-      !(std::norm(std::conj(W[0]) * w1 + std::conj(W[2]) * w3) <= tol * tol))
-    return false;
+  if (!rotates(W[0], w1, W[2], w3, 1e-12)) return false;
   if (c < pivot) {  // W = X V = X diag(g0, g1) M diag(1, b1) = diag(g1, g0) X M diag(1, b1)
     if (c == 0.0) {
       *R = Rot{false, 0.0, 0.0, cplx(1.0), 1, 0.0, 0.0, W[1], W[2], true, true};
@@ -158,20 +166,18 @@ bool factor_rotation(const cplx* W, bool scaled, double pivot, Rot* R) {
   }
   cplx a0, a1, b1;
   double cc = c, ss = s;
-  if (c > 0.0 && s > 0.0) {
+  if (c > 0.0) {
     a0 = W[0] / c;
     a1 = W[2] / s;
     // (a0, a1 are of modulus 1: dividing by them is multiplying by the conjugate)
     b1 = c >= s ? w3 * std::conj(a1) : -w1 * std::conj(a0);
     b1 /= std::abs(b1);
-  } else if (c == 0.0) {  // anti-diagonal
+  } else {  // anti-diagonal
     a0 = -w1;
     a1 = W[2];
     b1 = 1.0;
     cc = 0.0;
     ss = 1.0;
-  } else {
-    return false;  // diagonal: handled by the caller
   }
   // the norms of the rows are 1 to 1e-12; keep the phases unit-modulus (by the
   // exact modulus: the square root of a norm this close to 1 rounds to 1 and
@@ -929,12 +935,10 @@ bool all_wide(const std::vector<std::vector<LoweredGate>>& parts, const Frames& 
           if (std::fabs(std::norm(g.m[(g.nt == 1 ? 3 : 5) * i]) - 1.0) > 2e-12) return false;
         if (g.nt == 2 && g.nc == HS_MAX_CONTROLS) return false;
       } else if (g.nt == 1 && g.nc == 0) {
-        // unitary, well within what factor_rotation asks for
+        // a rotation, well within what factor_rotation asks for
         const double tol = 2.5e-13;
-        const cplx o = std::conj(g.m[0]) * g.m[1] + std::conj(g.m[2]) * g.m[3];
-        if (!(std::fabs(std::norm(g.m[0]) + std::norm(g.m[2]) - 1.0) <= tol &&
-              std::fabs(std::norm(g.m[1]) + std::norm(g.m[3]) - 1.0) <= tol &&
-              std::norm(o) <= tol * tol))
+        if (!(std::fabs(std::norm(g.m[1]) + std::norm(g.m[3]) - 1.0) <= tol &&
+              rotates(g.m[0], g.m[1], g.m[2], g.m[3], tol)))
           return false;
       } else if (!(g.nt == 1 && is_x(g.m)) && !(g.nt == 2 && g.nc == 0 && is_swap4(g.m))) {
         return false;

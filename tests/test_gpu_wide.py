@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from hisvsim_b200 import abi, circuits, partition
-from hisvsim_b200.gates import part_offsets, to_records
+from hisvsim_b200.gates import Gate, part_offsets, to_records
 from test_k1_wide import _mixed
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +36,24 @@ def test_wide_passes_match_oracle(port, n, hint, dtype, tol):
         assert np.abs(st.amplitudes() - want).max() <= tol
     finally:
         abi.set_tile_qubits(prev)
+
+
+@pytest.mark.parametrize("dtype,tol", [(abi.C128, 1e-12), (abi.C64, 1e-5)])
+@pytest.mark.parametrize("m", [(1, 2e-17, 0, 1), (1, 0, 2e-17, 1), (1, 2e-13, 0, 1j), (0, 1, 1, 2e-17)])
+def test_gates_diagonal_to_rounding(port, m, dtype, tol):
+    """Custom gates with a rounding residue off (or on) the diagonal, among gates that flip."""
+    n = 12
+    near = Gate("C1", (2,), params=m)
+    gates = ([Gate("H", (q,)) for q in range(n)] + [Gate("X", (0,)), Gate("RY", (1,), params=(3.0,)), near]
+             + circuits.random_layered(n, 3, 5) + [near])
+    want = port.run(n, to_records(gates))
+    rec, offs = part_offsets([gates[:n + 3], gates[n + 3:n + 40], gates[n + 40:]])
+    st = abi.State(n, dtype)
+    st.run_parts(rec, offs)
+    assert np.abs(st.amplitudes() - want).max() <= tol
+    st.set_basis(0)
+    fr = abi.Frames(n)
+    for p in range(len(offs) - 1):
+        st.run_part_carry(fr, rec[offs[p]:offs[p + 1]])
+    st.flush(fr)
+    assert np.abs(st.amplitudes() - want).max() <= tol

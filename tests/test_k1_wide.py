@@ -193,3 +193,19 @@ def test_other_gates_keep_the_general_form(emu):
         assert st["passes"] == 1 and st["wide"] == 0
     _, st = emu(9, [[Gate("H", (q,)) for q in range(9)]])
     assert st["passes"] == 1 and st["wide"] == 0
+
+
+def test_gates_diagonal_to_rounding_are_not_refused(emu):
+    """A custom gate with one off-diagonal entry of exactly 0 and the other a
+    rounding residue, next to gates that flip: applied as a matrix where it is no
+    rotation (lower left 0), and its call does without flips."""
+    n = 12
+    base = [Gate("H", (q,)) for q in range(n)] + [Gate("X", (0,)), Gate("RY", (1,), params=(3.0,))]
+    for m, wide in (((1, 2e-17, 0, 1), False), ((1, 0, 2e-17, 1), True),
+                    ((1, 2e-13, 0, 1j), False), ((5e-324, 1, 1, 0), True), ((0, 1, 1, 2e-17), True)):
+        gate = Gate("C1", (2,), params=m)
+        for parts in ([base + [gate]], [[gate] + base], [base, [gate], base]):
+            for dtype in (0, 1):
+                for mode in (0, 1, 2):
+                    _, st = emu(n, parts, dtype=dtype, mode=mode)
+                    assert (st["wide"] == st["passes"]) == wide
