@@ -88,6 +88,11 @@ TimedRegion::~TimedRegion() {
 namespace {
 
 cudaStream_t S(void* stream) { return static_cast<cudaStream_t>(stream); }
+// the stream of a call's work on `st`
+cudaStream_t S(const hs_state* st, void* stream) {
+  if (stream) st->elsewhere = true;
+  return S(stream);
+}
 
 int check_state(const hs_state* st) {
   if (!st || !st->amp) return set_error(HS_E_INVALID, "null or destroyed state");
@@ -96,10 +101,11 @@ int check_state(const hs_state* st) {
 
 // Device memory of small states, kept when they are destroyed: mapping and
 // unmapping it costs 0.6 ms (at times several) per state, forty times the
-// planning of a small part, for programs that make a state per circuit.  A
-// block changes hands only when the device has finished everything (the wait
-// that cudaFree implies), whatever streams used it.  At most kKeptBytes per
-// device in blocks of up to kKeptBlock; given back when an allocation fails.
+// planning of a small part, for programs that make a state per circuit.  Only
+// states whose work all ran on the default stream are kept, once that stream has
+// finished: a wait for the whole device would end any other thread's stream
+// capture, which freeing the memory does not.  At most kKeptBytes per device in
+// blocks of up to kKeptBlock; given back when an allocation fails.
 constexpr size_t kKeptBlock = 16ull << 20, kKeptBytes = 32ull << 20;
 std::mutex g_kept_mu;
 struct KeptBlock {
@@ -137,10 +143,14 @@ cudaError_t state_alloc(void** p, size_t bytes) {
   return cudaMalloc(p, bytes);
 }
 
-void state_free(void* p, size_t bytes, int dev) {
+void state_free(hs_state* st) {
+  void* const p = st->amp;
+  const size_t bytes = amp_bytes(st->dtype) << st->n;
+  const int dev = st->dev;
   int cur = -1;
-  if (dev >= 0 && dev < 64 && bytes <= kKeptBlock && cudaGetDevice(&cur) == cudaSuccess &&
-      cur == dev && cudaDeviceSynchronize() == cudaSuccess) {
+  if (!st->elsewhere && dev >= 0 && dev < 64 && bytes <= kKeptBlock &&
+      cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
+      cudaStreamSynchronize(nullptr) == cudaSuccess) {
     std::lock_guard<std::mutex> lk(g_kept_mu);
     if (g_kept_bytes[dev] + bytes <= kKeptBytes) {
       g_kept[dev].push_back({p, bytes});
@@ -318,7 +328,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
 
 int hs_state_destroy(hs_state* st) {
   if (!st) return HS_OK;
-  if (st->amp) state_free(st->amp, amp_bytes(st->dtype) << st->n, st->dev);
+  if (st->amp) state_free(st);
   st->amp = nullptr;
   if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev);
   delete st;
@@ -339,6 +349,7 @@ int hs_state_dtype(const hs_state* st, int* dtype) {
 
 int hs_state_device_ptr(const hs_state* st, void** dptr) {
   HS_TRY(check_state(st));
+  st->elsewhere = true;  // the caller's own work on it is not known
   *dptr = st->amp;
   return HS_OK;
 }
@@ -353,7 +364,7 @@ int hs_state_set_basis(hs_state* st, uint64_t x, void* stream) {
   HS_TRY(check_state(st));
   if (st->n < 64 && (x >> st->n)) return set_error(HS_E_INVALID, "basis index out of range");
   for (int q = 0; q < st->n; ++q) st->q2s[q] = st->s2q[q] = q;
-  return set_basis_kernel(st->amp, st->dtype, st->n, x, S(stream));
+  return set_basis_kernel(st->amp, st->dtype, st->n, x, S(st, stream));
 }
 
 int hs_state_copy_to_host(hs_state* st, void* host, uint64_t first, uint64_t count,
@@ -363,8 +374,8 @@ int hs_state_copy_to_host(hs_state* st, void* host, uint64_t first, uint64_t cou
   if (first > size || count > size - first) return set_error(HS_E_INVALID, "range outside state");
   const size_t b = amp_bytes(st->dtype);
   HS_CUDA(cudaMemcpyAsync(host, static_cast<char*>(st->amp) + first * b, count * b,
-                          cudaMemcpyDeviceToHost, S(stream)));
-  HS_CUDA(cudaStreamSynchronize(S(stream)));
+                          cudaMemcpyDeviceToHost, S(st, stream)));
+  HS_CUDA(cudaStreamSynchronize(S(st, stream)));
   return HS_OK;
 }
 
@@ -375,8 +386,8 @@ int hs_state_copy_from_host(hs_state* st, const void* host, uint64_t first, uint
   if (first > size || count > size - first) return set_error(HS_E_INVALID, "range outside state");
   const size_t b = amp_bytes(st->dtype);
   HS_CUDA(cudaMemcpyAsync(static_cast<char*>(st->amp) + first * b, host, count * b,
-                          cudaMemcpyHostToDevice, S(stream)));
-  HS_CUDA(cudaStreamSynchronize(S(stream)));
+                          cudaMemcpyHostToDevice, S(st, stream)));
+  HS_CUDA(cudaStreamSynchronize(S(st, stream)));
   return HS_OK;
 }
 
@@ -387,15 +398,16 @@ int hs_state_canonicalize(hs_state* st, void* stream) {
   bool ident = true;
   for (int p = 0; p < st->n; ++p) ident &= pi[p] == p;
   if (ident) return HS_OK;
-  return permute_positions(st, pi, S(stream));
+  return permute_positions(st, pi, S(st, stream));
 }
 
 int hs_state_convert(const hs_state* src, hs_state* dst, void* stream) {
   HS_TRY(check_state(src));
   HS_TRY(check_state(dst));
   if (src->n != dst->n) return set_error(HS_E_INVALID, "qubit counts differ");
+  S(src, stream);
   HS_TRY(convert_kernel(src->amp, src->dtype, dst->amp, dst->dtype, 1ull << src->n,
-                        S(stream)));
+                        S(dst, stream)));
   dst->q2s = src->q2s;
   dst->s2q = src->s2q;
   return HS_OK;
@@ -406,7 +418,7 @@ int hs_gate_apply(hs_state* st, const hs_gate* gate, void* stream) {
   if (!gate) return set_error(HS_E_INVALID, "null gate");
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gate, 1, &lg));
-  return run_part(st, lg, S(stream));
+  return run_part(st, lg, S(st, stream));
 }
 
 int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream) {
@@ -415,7 +427,7 @@ int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream)
   if (num_gates == 0) return HS_OK;
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gates, num_gates, &lg));
-  return run_part(st, lg, S(stream));
+  return run_part(st, lg, S(st, stream));
 }
 
 int hs_frames_create(int num_qubits, hs_frames** out) {
@@ -449,7 +461,7 @@ int hs_part_run_carry(hs_state* st, hs_frames* fr, const hs_gate* gates, int num
   std::vector<LoweredGate> lg;
   HS_TRY(lower_all(st, gates, num_gates, &lg));
   Frames next = fr->fr;  // (an error leaves the factors as they were)
-  HS_TRY(run_lowered(st, lg, &next, false, S(stream)));
+  HS_TRY(run_lowered(st, lg, &next, false, S(st, stream)));
   fr->fr = std::move(next);
   return HS_OK;
 }
@@ -459,7 +471,7 @@ int hs_frames_flush(hs_state* st, hs_frames* fr, void* stream) {
   if (!fr || fr->n != st->n) return set_error(HS_E_INVALID, "frames missing or of another size");
   if (fr->fr.identity()) return HS_OK;
   Frames next = fr->fr;
-  HS_TRY(run_lowered(st, {}, &next, true, S(stream)));
+  HS_TRY(run_lowered(st, {}, &next, true, S(st, stream)));
   fr->fr = std::move(next);
   return HS_OK;
 }
@@ -484,8 +496,8 @@ int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets
   fr.reset(st->n);
   return plan_parts(st->n, st->q2s, all, &fr, true, g_tile_hint.load(), st->dtype,
                     [&](PlannedPass& p) {
-                      TimedRegion tr(S(stream));
-                      return launch_pass(st, p, S(stream));
+                      TimedRegion tr(S(st, stream));
+                      return launch_pass(st, p, S(st, stream));
                     });
 }
 
@@ -512,7 +524,7 @@ int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_o
   int rc = HS_OK;
   for (auto& e : ev)
     if (cudaEventCreate(&e) != cudaSuccess) rc = set_error(HS_E_CUDA, "event create");
-  const cudaStream_t s = S(stream);
+  const cudaStream_t s = S(st, stream);
   if (rc == HS_OK && cudaEventRecord(ev[0], s) != cudaSuccess)
     rc = set_error(HS_E_CUDA, "event record");
   for (int p = 0; p < num_parts && rc == HS_OK; ++p) {
@@ -584,8 +596,8 @@ int hs_permute_bits(hs_state* st, const int32_t* pairs, int num_pairs, void* str
     pi[b] = a;
   }
   if (num_pairs == 0) return HS_OK;
-  TimedRegion tr(S(stream));
-  HS_TRY(launch_permute(st->amp, st->dtype, st->n, pairs, num_pairs, S(stream)));
+  TimedRegion tr(S(st, stream));
+  HS_TRY(launch_permute(st->amp, st->dtype, st->n, pairs, num_pairs, S(st, stream)));
   count_pass(0);
   std::vector<int> s2q(st->n);
   for (int p = 0; p < st->n; ++p) s2q[pi[p]] = st->s2q[p];
@@ -611,8 +623,8 @@ int hs_gather_qubits(hs_state* st, const int32_t* proc_qubits, int num, void* st
     if (is_proc[st->s2q[p]]) order.push_back(p);
   std::vector<int> pi(st->n);
   for (int j = 0; j < st->n; ++j) pi[order[j]] = j;
-  TimedRegion tr(S(stream));
-  return permute_positions(st, pi, S(stream));
+  TimedRegion tr(S(st, stream));
+  return permute_positions(st, pi, S(st, stream));
 }
 
 int hs_project(hs_state* st, const int32_t* qubits, const int32_t* values, int count,
@@ -637,7 +649,7 @@ int hs_project(hs_state* st, const int32_t* qubits, const int32_t* values, int c
     if (!used[q]) slots.push_back(st->q2s[q]);
   hs_state* ns = nullptr;
   HS_TRY(hs_state_create(st->n - count, st->dtype, &ns));
-  const cudaStream_t s = S(stream);
+  const cudaStream_t s = S(st, stream);
   double p = 0;
   int rc = project_kernel(st->amp, ns->amp, st->dtype, ns->n, slots.data(), offset, s);
   if (rc == HS_OK) rc = reduce_norm2(ns->amp, ns->dtype, ns->n, &p, s);

@@ -182,6 +182,7 @@ int hs_fused_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_o
     return set_error(HS_E_INVALID, "unknown precision %d", precision);
   if (num_parts <= 0) return HS_OK;
   cudaStream_t s = S(stream);
+  if (s) st->elsewhere = true;
   std::vector<PartLocal> parts;
   DevBuf d_a;
   HS_TRY(compose_all(st->n, st->q2s, st->s2q, gates, part_offsets, num_parts, s, &parts, &d_a,
@@ -224,6 +225,7 @@ int hs_fused_apply(hs_state* st, const double* u, const int32_t* qubits, int pre
     parts[0].qubits[j] = q;
   }
   const cudaStream_t s = S(stream);
+  if (s) st->elsewhere = true;
   DevBuf d_u, d_a, d_err;
   d_u.s = d_a.s = d_err.s = s;
   HS_CUDA(cudaMallocAsync(&d_u.p, sizeof(double2) * kFusedDim * kFusedDim, s));

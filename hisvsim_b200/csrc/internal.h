@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <complex>
 #include <functional>
 #include <memory>
@@ -564,5 +565,7 @@ struct hs_state {
   int dtype = HS_DTYPE_C128;
   void* amp = nullptr;  // device, slot-ordered
   int dev = 0;          // the device it was created on
+  // its device pointer was handed out, or a call ran on another stream than the default one
+  mutable std::atomic<bool> elsewhere{false};
   std::vector<int> q2s, s2q;
 };

@@ -61,3 +61,43 @@ def test_kept_memory_is_bounded():
         [s.close() for s in states]
     # 32 MiB of states and the granularity of their mappings
     assert before - torch.cuda.mem_get_info()[0] <= 96 << 20
+
+
+def test_states_come_and_go_beside_a_capture():
+    """A thread makes, uses and destroys states while another captures a stream
+    (thread-local mode, as hs_batch does): the capture stays valid."""
+    import torch
+
+    x = torch.zeros(1024, device="cuda")
+    side = torch.cuda.Stream()
+    rec = to_records(circuits.random_layered(10, 2, 1))
+    abi.State(10).close()
+    err = []
+
+    def states():
+        try:
+            abi.set_device(0)
+            for n in (4, 10, 12):
+                for stream in (None, side.cuda_stream):
+                    st = abi.State(n)
+                    if n == 10:
+                        st.run_part(rec, stream=stream)
+                    st.close()
+        except Exception as e:  # noqa: BLE001
+            err.append(e)
+
+    g = torch.cuda.CUDAGraph()
+    cap = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(cap):
+        g.capture_begin(capture_error_mode="thread_local")
+        x.add_(1.0)
+        t = threading.Thread(target=states)
+        t.start()
+        t.join()
+        x.add_(1.0)
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    assert not err
+    assert bool((x == 2.0).all())
