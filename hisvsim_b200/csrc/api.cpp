@@ -11,6 +11,8 @@
 #include <random>
 #include <set>
 
+#include <cuda.h>
+
 #include "bounds.cuh"
 #include "internal.h"
 
@@ -85,6 +87,32 @@ TimedRegion::~TimedRegion() {
   }
 }
 
+uint64_t context_id() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<GetId>(f);
+  }();
+  unsigned long long id = 0;
+  return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  return alloc_releasing(
+      cudaErrorMemoryAllocation, [&] { return cudaMalloc(p, bytes); }, release_kept);
+}
+
+cudaError_t device_malloc_async(void** p, size_t bytes, cudaStream_t s) {
+  return alloc_releasing(
+      cudaErrorMemoryAllocation, [&] { return cudaMallocAsync(p, bytes, s); }, release_kept);
+}
+
 namespace {
 
 cudaStream_t S(void* stream) { return static_cast<cudaStream_t>(stream); }
@@ -105,61 +133,45 @@ int check_state(const hs_state* st) {
 // states whose work all ran on the default stream are kept, once that stream has
 // finished: a wait for the whole device would end any other thread's stream
 // capture, which freeing the memory does not.  At most kKeptBytes per device in
-// blocks of up to kKeptBlock; given back when an allocation fails.
+// blocks of up to kKeptBlock; given back when an allocation of the library fails.
 constexpr size_t kKeptBlock = 16ull << 20, kKeptBytes = 32ull << 20;
-std::mutex g_kept_mu;
-struct KeptBlock {
-  void* p;
-  size_t bytes;
-};
-std::vector<KeptBlock> g_kept[64];
-size_t g_kept_bytes[64];
+
+KeptBlocks<kKeptBytes>& kept_states(int dev) {
+  static auto* const pools = new KeptBlocks<kKeptBytes>[64];  // (not destroyed at exit: states may be)
+  return pools[dev & 63];
+}
 
 cudaError_t state_alloc(void** p, size_t bytes) {
   int dev = 0;
   const cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 64 && bytes <= kKeptBlock) {
-    std::lock_guard<std::mutex> lk(g_kept_mu);
-    auto& kept = g_kept[dev];
-    for (size_t i = 0; i < kept.size(); ++i)
-      if (kept[i].bytes == bytes) {
-        *p = kept[i].p;
-        g_kept_bytes[dev] -= bytes;
-        kept.erase(kept.begin() + i);
-        return cudaSuccess;
-      }
-  }
-  const cudaError_t first = cudaMalloc(p, bytes);
-  if (first != cudaErrorMemoryAllocation || dev >= 64) return first;
-  cudaGetLastError();
-  {
-    std::lock_guard<std::mutex> lk(g_kept_mu);
-    if (g_kept[dev].empty()) return first;
-    for (const KeptBlock& b : g_kept[dev]) cudaFree(b.p);
-    g_kept[dev].clear();
-    g_kept_bytes[dev] = 0;
-  }
-  return cudaMalloc(p, bytes);
+  if (bytes <= kKeptBlock && (*p = kept_states(dev).take(context_id(), bytes))) return cudaSuccess;
+  return device_malloc(p, bytes);
 }
 
-void state_free(hs_state* st) {
-  void* const p = st->amp;
+void state_free(const hs_state* st) {
   const size_t bytes = amp_bytes(st->dtype) << st->n;
-  const int dev = st->dev;
   int cur = -1;
-  if (!st->elsewhere && dev >= 0 && dev < 64 && bytes <= kKeptBlock &&
-      cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
-      cudaStreamSynchronize(nullptr) == cudaSuccess) {
-    std::lock_guard<std::mutex> lk(g_kept_mu);
-    if (g_kept_bytes[dev] + bytes <= kKeptBytes) {
-      g_kept[dev].push_back({p, bytes});
-      g_kept_bytes[dev] += bytes;
-      return;
-    }
+  if (!st->elsewhere && bytes <= kKeptBlock && cudaGetDevice(&cur) == cudaSuccess &&
+      cur == st->dev && cudaStreamSynchronize(nullptr) == cudaSuccess && st->ctx == context_id()) {
+    for (void* p : kept_states(cur).put(st->ctx, st->amp, bytes)) cudaFree(p);
+    return;
   }
-  cudaFree(p);
+  cudaFree(st->amp);
 }
+
+}  // namespace
+
+bool release_kept() {
+  cudaGetLastError();  // (the failed allocation's)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::vector<void*> blocks = kept_states(dev).drain(context_id());
+  for (void* p : blocks) cudaFree(p);
+  return scratch_release(dev, context_id()) || !blocks.empty();
+}
+
+namespace {
 
 // Apply a permutation of bit positions to the data: the bit at position p
 // moves to position pi[p].  Done as two in-place involution passes of K2:
@@ -322,6 +334,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
     return rc;
   }
   if (cudaGetDevice(&st->dev) == cudaSuccess) ++g_live_states[st->dev & 63];
+  st->ctx = context_id();
   *out = st;
   return HS_OK;
 }
@@ -330,7 +343,7 @@ int hs_state_destroy(hs_state* st) {
   if (!st) return HS_OK;
   if (st->amp) state_free(st);
   st->amp = nullptr;
-  if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev);
+  if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev, st->ctx);
   delete st;
   return HS_OK;
 }

@@ -282,7 +282,7 @@ int build_plan(hs_batch* b) {
     cut.resize((cut.size() + 15) & ~size_t(15));
   }
   b->threads = max_m > 11 ? 256 : 128;
-  HS_CUDA(cudaMalloc(&b->d_cut, cut.size()));
+  HS_CUDA(device_malloc(&b->d_cut, cut.size()));
   HS_CUDA(cudaMemcpy(b->d_cut, cut.data(), cut.size(), cudaMemcpyHostToDevice));
   for (int i = 0; i < b->ninst; ++i) inst[i].cut = b->d_cut + cut_off[i];
   // work items: per step level, per instance, the step's tiles in chunks
@@ -309,10 +309,10 @@ int build_plan(hs_batch* b) {
   b->items = items;
   b->total = total;
   b->ncounters = nc;
-  HS_CUDA(cudaMalloc(&b->d_inst, sizeof(BatchInstance) * inst.size()));
-  HS_CUDA(cudaMalloc(&b->d_items, sizeof(BatchItem) * items.size()));
-  HS_CUDA(cudaMalloc(&b->d_counters, sizeof(uint32_t) * nc));
-  HS_CUDA(cudaMalloc(&b->d_partial, sizeof(double) * size_t(b->ninst) * 256));
+  HS_CUDA(device_malloc(&b->d_inst, sizeof(BatchInstance) * inst.size()));
+  HS_CUDA(device_malloc(&b->d_items, sizeof(BatchItem) * items.size()));
+  HS_CUDA(device_malloc(&b->d_counters, sizeof(uint32_t) * nc));
+  HS_CUDA(device_malloc(&b->d_partial, sizeof(double) * size_t(b->ninst) * 256));
   HS_CUDA(cudaMemcpy(b->d_inst, inst.data(), sizeof(BatchInstance) * inst.size(),
                      cudaMemcpyHostToDevice));
   HS_CUDA(cudaMemcpy(b->d_items, items.data(), sizeof(BatchItem) * items.size(),
@@ -411,18 +411,18 @@ int hs_batch_create_qaoa(int num_instances, const int32_t* num_qubits, const int
     hs_batch_destroy(b);
     return code;
   };
-  if (cudaMalloc(&b->pool, amps * sizeof(float2)) != cudaSuccess) {
+  if (device_malloc(&b->pool, amps * sizeof(float2)) != cudaSuccess) {
     cudaGetLastError();
     delete b;
     return set_error(HS_E_NOMEM, "batch states: %llu amplitudes", (unsigned long long)amps);
   }
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-      cudaMalloc(&b->d_par, sizeof(BatchParams) * num_instances) != cudaSuccess ||
-      cudaMalloc(&b->d_head, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&b->d_err, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&b->d_limit, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&b->d_expect, sizeof(double) * num_instances) != cudaSuccess ||
+      device_malloc(&b->d_par, sizeof(BatchParams) * num_instances) != cudaSuccess ||
+      device_malloc(&b->d_head, sizeof(unsigned long long)) != cudaSuccess ||
+      device_malloc(&b->d_err, sizeof(int)) != cudaSuccess ||
+      device_malloc(&b->d_limit, sizeof(uint32_t)) != cudaSuccess ||
+      device_malloc(&b->d_expect, sizeof(double) * num_instances) != cudaSuccess ||
       cudaMallocHost(&b->h_expect, sizeof(double) * num_instances) != cudaSuccess ||
       cudaMallocHost(&b->h_err, sizeof(int)) != cudaSuccess)
     return fail(set_error(HS_E_NOMEM, "batch buffers"));

@@ -81,10 +81,10 @@ int compose_all(int n, const std::vector<int>& q2s, const std::vector<int>& s2q,
   DevBuf d_g, d_o;
   d_g.s = d_o.s = d_a->s = s;
   if (d_u) d_u->s = s;
-  HS_CUDA(cudaMallocAsync(&d_g.p, sizeof(FusedGate) * std::max<size_t>(1, flat.size()), s));
-  HS_CUDA(cudaMallocAsync(&d_o.p, sizeof(int32_t) * foffs.size(), s));
-  HS_CUDA(cudaMallocAsync(&d_a->p, size_t(kFusedABytes) * nparts, s));
-  if (d_u) HS_CUDA(cudaMallocAsync(&d_u->p, sizeof(double2) * kFusedDim * kFusedDim * nparts, s));
+  HS_CUDA(device_malloc_async(&d_g.p, sizeof(FusedGate) * std::max<size_t>(1, flat.size()), s));
+  HS_CUDA(device_malloc_async(&d_o.p, sizeof(int32_t) * foffs.size(), s));
+  HS_CUDA(device_malloc_async(&d_a->p, size_t(kFusedABytes) * nparts, s));
+  if (d_u) HS_CUDA(device_malloc_async(&d_u->p, sizeof(double2) * kFusedDim * kFusedDim * nparts, s));
   if (!flat.empty())
     HS_CUDA(cudaMemcpyAsync(d_g.p, flat.data(), sizeof(FusedGate) * flat.size(),
                             cudaMemcpyHostToDevice, s));
@@ -191,7 +191,7 @@ int hs_fused_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_o
   HS_TRY(plan_fused(st->n, st->q2s, parts, precision, &passes));
   DevBuf d_err;
   d_err.s = s;
-  HS_CUDA(cudaMallocAsync(&d_err.p, sizeof(int), s));
+  HS_CUDA(device_malloc_async(&d_err.p, sizeof(int), s));
   HS_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
   {
     TimedRegion tr(s);
@@ -228,9 +228,9 @@ int hs_fused_apply(hs_state* st, const double* u, const int32_t* qubits, int pre
   if (s) st->elsewhere = true;
   DevBuf d_u, d_a, d_err;
   d_u.s = d_a.s = d_err.s = s;
-  HS_CUDA(cudaMallocAsync(&d_u.p, sizeof(double2) * kFusedDim * kFusedDim, s));
-  HS_CUDA(cudaMallocAsync(&d_a.p, kFusedABytes, s));
-  HS_CUDA(cudaMallocAsync(&d_err.p, sizeof(int), s));
+  HS_CUDA(device_malloc_async(&d_u.p, sizeof(double2) * kFusedDim * kFusedDim, s));
+  HS_CUDA(device_malloc_async(&d_a.p, kFusedABytes, s));
+  HS_CUDA(device_malloc_async(&d_err.p, sizeof(int), s));
   HS_CUDA(cudaMemcpyAsync(d_u.p, u, sizeof(double2) * kFusedDim * kFusedDim,
                           cudaMemcpyHostToDevice, s));
   HS_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
@@ -299,7 +299,7 @@ int hs_compare_host(hs_state* a, const void* host_b, int bdtype, double out[4]) 
   const size_t bb = amp_bytes(bdtype), ab = amp_bytes(a->dtype);
   const uint64_t chunk = std::min<uint64_t>(size, 1ull << 26);
   DevBuf stage;
-  HS_CUDA(cudaMallocAsync(&stage.p, chunk * bb, nullptr));
+  HS_CUDA(device_malloc_async(&stage.p, chunk * bb, nullptr));
   double acc[4] = {0, 0, 0, 0};
   for (uint64_t first = 0; first < size; first += chunk) {
     HS_CUDA(cudaMemcpy(stage.p, static_cast<const char*>(host_b) + first * bb, chunk * bb,

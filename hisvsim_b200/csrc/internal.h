@@ -11,6 +11,8 @@
 #include <string>
 #include <vector>
 
+#include "kept_blocks.h"
+
 #include "hisv.h"
 
 namespace hisv {
@@ -469,6 +471,19 @@ int launch_batch_init(const BatchInstance* d_inst, int ninst, cudaStream_t s);
 int launch_batch_expect(const BatchInstance* d_inst, int ninst, int max_n, double* d_partial,
                         double* d_out, cudaStream_t s);
 
+// ---- device memory (api.cpp) -------------------------------------------------
+// id of the calling thread's context (unique in the process), 0 = none yet
+uint64_t context_id();
+// frees the blocks kept on the current device; whether there were any
+bool release_kept();
+// cudaMalloc and cudaMallocAsync that give those back before they fail
+cudaError_t device_malloc(void** p, size_t bytes);
+cudaError_t device_malloc_async(void** p, size_t bytes, cudaStream_t s);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+  return device_malloc(reinterpret_cast<void**>(p), bytes);
+}
+
 // ---- launchers (kernels_*.cu) ----------------------------------------------
 int launch_part(void* amp, int dtype, const PartProgram& prog, cudaStream_t s);
 int launch_wide(void* amp, int dtype, const WideProgram& prog, cudaStream_t s);
@@ -484,8 +499,9 @@ int reduce_zz(const void* amp, int dtype, int n, const int32_t* slot_pairs, int 
               double* out, cudaStream_t s);
 int reduce_chunks(const void* amp, int dtype, int n, int chunk_bits, double* host_out,
                   cudaStream_t s);
-// frees the reductions' kept scratch blocks of device `dev` (its last state is gone)
-void scratch_release(int dev);
+// frees the reductions' idle scratch blocks of device `dev` and context `ctx`;
+// whether there were any
+bool scratch_release(int dev, uint64_t ctx);
 // a chunk of amplitudes with samples: its first amplitude, the mass before it,
 // its samples [s0, s0 + ns) of the sorted sample points
 struct MeasureChunk {
@@ -564,7 +580,8 @@ struct hs_state {
   int n = 0;
   int dtype = HS_DTYPE_C128;
   void* amp = nullptr;  // device, slot-ordered
-  int dev = 0;          // the device it was created on
+  int dev = 0;          // the device and the context (context_id) it was created on
+  uint64_t ctx = 0;
   // its device pointer was handed out, or a call ran on another stream than the default one
   mutable std::atomic<bool> elsewhere{false};
   std::vector<int> q2s, s2q;

@@ -1,7 +1,6 @@
 // K2 (in-place bit-swap permutation), K3 (FP64 reductions) and small
 // elementwise kernels (basis-state set, dtype conversion).
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "bounds.cuh"
@@ -18,39 +17,32 @@ int num_sms() { return device_sms(); }
 // whenever it changes hands, whatever the threads and streams.  Allocating from
 // a stream-ordered pool instead costs 0.45 ms per call that synchronises,
 // whatever the size of the state.  The blocks are freed with the device's last
-// state (scratch_release); larger requests are allocated for the call.
+// state (scratch_release) and when an allocation fails; larger requests are
+// allocated for the call.
 constexpr size_t kScratchBlock = 1ull << 20;
 constexpr size_t kScratchKept = 4;
 
-std::mutex g_scratch_mu;
-std::vector<void*> g_scratch[64];
+using KeptScratch = KeptBlocks<kScratchKept * kScratchBlock>;
+KeptScratch& kept_scratch(int dev) {
+  static auto* const pools = new KeptScratch[64];  // (not destroyed at exit)
+  return pools[dev & 63];
+}
 
 class Scratch {
  public:
   ~Scratch() {
     if (!p_) return;
-    if (idle_ && block_) {
-      std::lock_guard<std::mutex> lk(g_scratch_mu);
-      if (g_scratch[dev_].size() < kScratchKept) {
-        g_scratch[dev_].push_back(p_);
-        return;
-      }
-    }
-    cudaFree(p_);
+    if (idle_ && block_)
+      for (void* p : kept_scratch(dev_).put(ctx_, p_, kScratchBlock)) cudaFree(p);
+    else
+      cudaFree(p_);
   }
   int get(size_t bytes) {
     HS_CUDA(cudaGetDevice(&dev_));
-    block_ = bytes <= kScratchBlock && dev_ >= 0 && dev_ < 64;
-    if (block_) {
-      std::lock_guard<std::mutex> lk(g_scratch_mu);
-      g_scratch[dev_].reserve(kScratchKept);
-      if (!g_scratch[dev_].empty()) {
-        p_ = g_scratch[dev_].back();
-        g_scratch[dev_].pop_back();
-        return HS_OK;
-      }
-    }
-    HS_CUDA(cudaMalloc(&p_, block_ ? kScratchBlock : bytes));
+    block_ = bytes <= kScratchBlock;
+    if (!block_ || !(p_ = kept_scratch(dev_).take(context_id(), kScratchBlock)))
+      HS_CUDA(device_malloc(&p_, block_ ? kScratchBlock : bytes));
+    ctx_ = context_id();
     return HS_OK;
   }
   // waits for the call's work; what is left behind may then be handed on
@@ -65,6 +57,7 @@ class Scratch {
  private:
   void* p_ = nullptr;
   int dev_ = 0;
+  uint64_t ctx_ = 0;
   bool block_ = false, idle_ = false;
 };
 
@@ -504,11 +497,10 @@ int run_compare(const void* a, const void* b, uint64_t size, double out[4], cuda
 
 }  // namespace
 
-void scratch_release(int dev) {
-  if (dev < 0 || dev >= 64) return;
-  std::lock_guard<std::mutex> lk(g_scratch_mu);
-  for (void* p : g_scratch[dev]) cudaFree(p);
-  g_scratch[dev].clear();
+bool scratch_release(int dev, uint64_t ctx) {
+  const std::vector<void*> blocks = kept_scratch(dev).drain(ctx);
+  for (void* p : blocks) cudaFree(p);
+  return !blocks.empty();
 }
 
 int reduce_compare(const void* a, int adtype, const void* b, int bdtype, int n, double out[4],
@@ -896,7 +888,7 @@ int fp64_probe(double* tflops) {
   HS_CUDA(cudaGetDevice(&dev));
   HS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   double* d = nullptr;
-  HS_CUDA(cudaMalloc(&d, sizeof(double)));
+  HS_CUDA(device_malloc(&d, sizeof(double)));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

@@ -74,7 +74,7 @@ class CallBuffers {
       }
     }
     if (!base_) {
-      HS_CUDA(cudaMalloc(&base_, bytes));
+      HS_CUDA(device_malloc(&base_, bytes));
       bytes_ = bytes;
     }
     next_ = base_;
@@ -130,10 +130,10 @@ int hs_mlp_create(int in_dim, uint64_t seed, hs_mlp** out) {
       cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return fail(set_error(HS_E_CUDA, "device query"));
   const size_t pb = sizeof(float) * size_t(m->P);
-  if (cudaMalloc(&m->d_params, pb) != cudaSuccess || cudaMalloc(&m->d_m, pb) != cudaSuccess ||
-      cudaMalloc(&m->d_v, pb) != cudaSuccess || cudaMalloc(&m->d_grad, pb) != cudaSuccess ||
-      cudaMalloc(&m->d_partial, pb * size_t(m->sms)) != cudaSuccess ||
-      cudaMalloc(&m->d_lpart, sizeof(float) * size_t(m->sms)) != cudaSuccess) {
+  if (device_malloc(&m->d_params, pb) != cudaSuccess || device_malloc(&m->d_m, pb) != cudaSuccess ||
+      device_malloc(&m->d_v, pb) != cudaSuccess || device_malloc(&m->d_grad, pb) != cudaSuccess ||
+      device_malloc(&m->d_partial, pb * size_t(m->sms)) != cudaSuccess ||
+      device_malloc(&m->d_lpart, sizeof(float) * size_t(m->sms)) != cudaSuccess) {
     cudaGetLastError();
     return fail(set_error(HS_E_NOMEM, "model buffers"));
   }

@@ -101,3 +101,51 @@ def test_states_come_and_go_beside_a_capture():
     torch.cuda.synchronize()
     assert not err
     assert bool((x == 2.0).all())
+
+
+def test_kept_memory_of_many_states_is_bounded():
+    """Eight states of 16 MiB destroyed together leave 32 MiB and the granularity
+    of their mappings."""
+    import torch
+
+    torch.cuda.init()
+    abi.State(4).close()
+    before = torch.cuda.mem_get_info()[0]
+    for n in (20, 19, 20):
+        states = [abi.State(n) for _ in range(8)]
+        [s.close() for s in states]
+    assert before - torch.cuda.mem_get_info()[0] <= 48 << 20
+
+
+_RESET = """
+import ctypes, glob, os, sys
+import numpy as np, torch
+from hisvsim_b200 import abi
+rt = ctypes.CDLL(glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "cuda_runtime", "lib", "libcudart.so.*"))[0])
+for n in (4, 12, 20):
+    st = abi.State(n)
+    st.norm2()
+    st.close()
+assert rt.cudaDeviceReset() == 0
+try:  # states need the library's kernels in the new context; its memory must be new either way
+    for n in (4, 12, 20):
+        st = abi.State(n)
+        a = st.raw()
+        assert a[0] == 1 and not a[1:].any()
+        assert abs(st.norm2() - 1) < 1e-12
+        st.close()
+    print("usable")
+except abi.HisvError as e:
+    print("refused", e)
+"""
+
+
+def test_reset_device_leaves_no_stale_blocks():
+    """After a device reset no block of the old context is handed out."""
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", _RESET], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.startswith(("usable", "refused"))
+    assert "illegal" not in r.stdout
