@@ -412,12 +412,15 @@ void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double pivot, do
   out->push_back(x);
 }
 
+// some parts of a call, in order
+using Parts = std::vector<const std::vector<LoweredGate>*>;
+
 // every part in turn; the gates keep their part's number
-void rewrite(const std::vector<std::vector<LoweredGate>>& parts, Frames* F, bool scaled,
-             double pivot, double lim, bool split, std::vector<RGate>* out) {
+void rewrite(const Parts& parts, Frames* F, bool scaled, double pivot, double lim, bool split,
+             std::vector<RGate>* out) {
   for (size_t p = 0; p < parts.size(); ++p) {
     const size_t first = out->size();
-    for (const auto& g : parts[p]) rewrite_gate(g, F, scaled, pivot, lim, split, out);
+    for (const auto& g : *parts[p]) rewrite_gate(g, F, scaled, pivot, lim, split, out);
     for (size_t i = first; i < out->size(); ++i) (*out)[i].part = int(p);
   }
 }
@@ -881,6 +884,10 @@ bool use_wide(int n, int dtype) {
   return k1_reg_bits(dtype) == kRegBits && n >= kWideMinTileBits;
 }
 
+// Whether gates of later parts may move into earlier passes.  Complex64 calls
+// keep a pass per part, as hs_parts_run_timed does.
+bool moves_gates(int dtype) { return dtype == HS_DTYPE_C128; }
+
 // Gates a wide program can hold: rotations, flushes, phases, X under any
 // controls, and the plain swap.
 bool wide_gate(const SlotGate& s) {
@@ -924,11 +931,11 @@ struct RecSet {
 // Whether every gate of a call ends up in wide programs, which alone hold
 // rotations with a flip: the kinds wide_gate takes, and pending factors (from
 // earlier calls, custom gates among them) that factor_rotation can take in.
-bool all_wide(const std::vector<std::vector<LoweredGate>>& parts, const Frames& F) {
+bool all_wide(const Parts& parts, const Frames& F) {
   for (const cplx& r : F.r)
     if (!(std::norm(r) > 1e-6 && std::norm(r) < 1e6)) return false;
-  for (const auto& gates : parts)
-    for (const LoweredGate& g : gates) {
+  for (const auto* gates : parts)
+    for (const LoweredGate& g : *gates) {
       if (g.nt == 0) continue;
       if (is_diagonal(g)) {
         for (int i = 0; i < (g.nt == 1 ? 2 : 4); ++i)
@@ -1481,31 +1488,29 @@ struct ChunkRoom {
   }
 };
 
-// The planner of both program kinds: into `programs` (PartPrograms only) or,
-// with `sink`, as PartPrograms and WidePrograms, handed over pass by pass.
-// A pass takes what fits of the first part left (in order, up to the first gate
-// that does not fit).  Given a sink, a pass of wide gates also takes, where that
-// saves passes, every gate of the parts after it that fits the tile and has to
-// follow no gate left behind: a part bounded by the qubits its gates touch
-// leaves room in the tile, which holds targets alone, and parts so used up cost
-// no pass of their own (27 qubits, parts of 9 touched qubits: 9 passes instead
-// of 13; 20 random layers of 20 qubits in parts of 10: 9 instead of 26).
-int plan_chunks(int n, const std::vector<int>& q2s,
-                const std::vector<std::vector<LoweredGate>>& gates, Frames* fr, bool flush,
-                int tile_bits_hint, int dtype, std::vector<PartProgram>* programs,
+// The planner of both program kinds, for some parts of a call: into `programs`
+// (PartPrograms only) or, with `sink`, as PartPrograms and WidePrograms, handed
+// over pass by pass.  A pass takes what fits of the first part left (in order, up
+// to the first gate that does not fit).  Given a sink, a pass of wide gates also
+// takes, where that saves passes, every gate of the parts after it that fits the
+// tile and has to follow no gate left behind: a part bounded by the qubits its
+// gates touch leaves room in the tile, which holds targets alone, and parts so
+// used up cost no pass of their own (27 qubits, parts of 9 touched qubits: 9
+// passes instead of 13; 20 random layers of 20 qubits in parts of 10: 9 instead
+// of 26).  `flips`: rotations beyond the pivot become flips (all_wide).
+int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* fr, bool flush,
+                int tile_bits_hint, int dtype, bool flips, std::vector<PartProgram>* programs,
                 const PassSink* sink) {
   if (n < 1 || n > 63) return set_error(HS_E_INVALID, "bad qubit count %d", n);
   if (int(fr->r.size()) != n) fr->reset(n);
   std::vector<RGate> rg;
   size_t count = 2;
-  for (const auto& g : gates) count += g.size();
+  for (const auto* g : gates) count += g->size();
   rg.reserve(count);
   // keep the carried scale within a few dozen binary orders (it moves with
   // the scaled rotation forms and non-unitary diagonal gates)
   const double lim = dtype == HS_DTYPE_C64 ? 24.0 : 48.0;
   const bool wide = sink && use_wide(n, dtype);
-  const bool flips = wide && (tile_bits_hint <= 0 || tile_bits_hint >= kWideMinTileBits) &&
-                     all_wide(gates, *fr);
   const double pivot = !flips ? 0.0 : dtype == HS_DTYPE_C128 ? kShearPivot : kFlipPivotC64;
   rewrite(gates, fr, dtype == HS_DTYPE_C128 || flips, pivot, lim, wide, &rg);
   if (flush) {
@@ -1570,28 +1575,42 @@ int plan_chunks(int n, const std::vector<int>& q2s,
     uint64_t tset = 0;
     bool wide = false;
   };
-  auto cut = [&](bool merge, std::vector<Chunk>* out) -> bool {
-    std::vector<int> left, rest;
-    for (size_t x = 0; x < sgs.size(); ++x) left.push_back(int(x));
+  // the next gate joins the chunk if it is of the same part and fits
+  auto join = [&](Chunk* c, ChunkRoom* room, int x, int part) -> bool {
+    const SlotGate& g = sgs[x];
+    if (g.rg->part != part || low_union_size(c->tset | g.tmask, low_need) > max_tile ||
+        !room->add(g))
+      return false;
+    c->tset |= g.tmask;
+    c->gates.push_back(x);
+    c->wide = c->wide && wide_gate(g);
+    return true;
+  };
+  std::vector<Chunk> chunks, merged;
+  for (int x = 0; x < int(sgs.size());) {
+    chunks.emplace_back();
+    Chunk& c = chunks.back();
+    c.wide = wide;
+    ChunkRoom room;
+    const int part = sgs[x].rg->part;
+    while (x < int(sgs.size()) && join(&c, &room, x, part)) ++x;
+    if (c.gates.empty()) return set_error(HS_E_INVALID, "gate does not fit a tile");
+  }
+  // The same with gates moved forward.  Every chunk walks the gates that are left,
+  // which plan_parts bounds.
+  auto cut_merged = [&](std::vector<Chunk>* out) {
+    std::vector<int> left(sgs.size()), rest;
+    for (size_t x = 0; x < sgs.size(); ++x) left[x] = int(x);
     while (!left.empty()) {
       out->emplace_back();
       Chunk& c = out->back();
       ChunkRoom room;
       const int part = sgs[left[0]].rg->part;
-      c.wide = wide;
+      c.wide = true;
       size_t i = 0;
-      for (; i < left.size(); ++i) {
-        const SlotGate& g = sgs[left[i]];
-        if (g.rg->part != part || low_union_size(c.tset | g.tmask, low_need) > max_tile ||
-            !room.add(g))
-          break;
-        c.tset |= g.tmask;
-        c.gates.push_back(left[i]);
-        c.wide = c.wide && wide_gate(g);
-      }
-      if (c.gates.empty()) return false;
+      while (i < left.size() && join(&c, &room, left[i], part)) ++i;
       rest.clear();
-      if (merge && c.wide && low_union_size(c.tset, low_min) <= max_tile) {
+      if (c.wide && low_union_size(c.tset, low_min) <= max_tile) {
         uint64_t held_t = 0, held_d = 0;  // slots of gates left behind, as in take_group_roles
         const uint64_t every = (1ull << n) - 1ull;
         for (; i < left.size() && held_t != every; ++i) {
@@ -1610,17 +1629,13 @@ int plan_chunks(int n, const std::vector<int>& q2s,
       rest.insert(rest.end(), left.begin() + i, left.end());
       left.swap(rest);
     }
-    return true;
   };
-  std::vector<Chunk> chunks, merged;
-  if (!cut(false, &chunks)) return set_error(HS_E_INVALID, "gate does not fit a tile");
   // moving gates between passes pays where it saves passes: as many passes with
-  // other gates in them only change places of work and widen tiles.  Complex64
-  // calls keep a pass per part: hs_parts_run_timed, which times the parts one by
-  // one, gives the same bits there.
-  if (wide && dtype == HS_DTYPE_C128 && gates.size() > 1 && cut(true, &merged) &&
-      merged.size() < chunks.size())
-    chunks.swap(merged);
+  // other gates in them only change places of work and widen tiles
+  if (wide && moves_gates(dtype) && gates.size() > 1) {
+    cut_merged(&merged);
+    if (merged.size() < chunks.size()) chunks.swap(merged);
+  }
   std::vector<PlannedPass> passes;
   cplx gamma = 1.0;  // global factor the wide programs leave (wide_steps)
   for (const Chunk& c : chunks) {
@@ -1727,11 +1742,10 @@ int plan_chunks(int n, const std::vector<int>& q2s,
   } else if (gamma != cplx(1.0, 0.0)) {
     // left by rotations planned after the flush (their qubits had nothing
     // pending): a flush of its own
-    std::vector<std::vector<LoweredGate>> nothing(1);
     Frames g;
     g.reset(n);
     g.G = gamma;
-    return plan_chunks(n, q2s, nothing, &g, true, tile_bits_hint, dtype, nullptr, sink);
+    return plan_chunks(n, q2s, {}, &g, true, tile_bits_hint, dtype, false, nullptr, sink);
   }
   if (!sink)
     for (auto& P : *programs) finish_layout(&P, dtype);
@@ -1744,13 +1758,48 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
                Frames* fr, bool flush, int tile_bits_hint, int dtype,
                std::vector<PartProgram>* programs) {
   programs->clear();
-  return plan_chunks(n, q2s, {gates}, fr, flush, tile_bits_hint, dtype, programs, nullptr);
+  return plan_chunks(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, false, programs, nullptr);
 }
+
+namespace {
+
+// The parts of a call, window by window: a window's passes are on the device
+// before the next window is rewritten, and what a chunk walks stays bounded, so
+// planning is linear in the gates.  Where gates may move a window takes whole
+// parts up to kWindowGates gates (one part at least): half a millisecond of planning ahead of
+// its first pass, and at most one pass more than over the whole call per some
+// thirty; elsewhere it is one part.
+constexpr size_t kWindowGates = 1024;
+
+int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr, bool flush,
+              int tile_bits_hint, int dtype, const PassSink& sink) {
+  if (int(fr->r.size()) != n) fr->reset(n);
+  const bool wide = use_wide(n, dtype);
+  const bool flips = wide && (tile_bits_hint <= 0 || tile_bits_hint >= kWideMinTileBits) &&
+                     all_wide(parts, *fr);
+  const size_t most = wide && moves_gates(dtype) ? kWindowGates : 0;
+  size_t i = 0;
+  do {
+    Parts window;
+    for (size_t count = 0; i < parts.size(); ++i) {
+      count += parts[i]->size();
+      if (!window.empty() && count > most) break;
+      window.push_back(parts[i]);
+    }
+    HS_TRY(plan_chunks(n, q2s, window, fr, flush && i == parts.size(), tile_bits_hint, dtype, flips,
+                       nullptr, &sink));
+  } while (i < parts.size());
+  return HS_OK;
+}
+
+}  // namespace
 
 int plan_parts(int n, const std::vector<int>& q2s,
                const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
                int tile_bits_hint, int dtype, const PassSink& sink) {
-  return plan_chunks(n, q2s, parts, fr, flush, tile_bits_hint, dtype, nullptr, &sink);
+  Parts all;
+  for (const auto& p : parts) all.push_back(&p);
+  return plan_call(n, q2s, all, fr, flush, tile_bits_hint, dtype, sink);
 }
 
 int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
@@ -1761,7 +1810,7 @@ int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
     passes->push_back(std::move(p));
     return HS_OK;
   };
-  return plan_chunks(n, q2s, {gates}, fr, flush, tile_bits_hint, dtype, nullptr, &sink);
+  return plan_call(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, sink);
 }
 
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,

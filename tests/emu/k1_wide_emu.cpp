@@ -7,6 +7,7 @@
 // store.  Every offset is range-checked.  Passes of chunks that
 // do not qualify for a wide program are counted, not run.  Nothing in the
 // product loads this file.
+#include <chrono>
 #include <cmath>
 #include <complex>
 #include <cstdarg>
@@ -274,4 +275,30 @@ int wide_parts_run(int n, int dtype, const hs_gate* gates, const int32_t* offs, 
   if (stats) std::memcpy(stats, st, sizeof(st));
   return HS_OK;
 }
+}
+
+// Plans parts as one call without running them: {passes}, seconds {to the first pass, in all}.
+extern "C" int wide_plan_time(int n, int dtype, const hs_gate* gates, const int32_t* offs,
+                              int nparts, int32_t* passes, double* seconds) {
+  std::vector<std::vector<LoweredGate>> parts(nparts);
+  for (int p = 0; p < nparts; ++p) {
+    parts[p].resize(offs[p + 1] - offs[p]);
+    for (int i = offs[p]; i < offs[p + 1]; ++i) {
+      const int rc = lower_gate(gates[i], n, &parts[p][i - offs[p]]);
+      if (rc != HS_OK) return rc;
+    }
+  }
+  std::vector<int> q2s(n);
+  for (int q = 0; q < n; ++q) q2s[q] = q;
+  Frames fr;
+  fr.reset(n);
+  *passes = 0;
+  const auto t0 = std::chrono::steady_clock::now();
+  auto now = [&] { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); };
+  const int rc = plan_parts(n, q2s, parts, &fr, true, 0, dtype, [&](PlannedPass&) {
+    if (++*passes == 1) seconds[0] = now();
+    return HS_OK;
+  });
+  seconds[1] = now();
+  return rc;
 }
