@@ -507,7 +507,7 @@ int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets
   // and applied by the last pass; each pass is launched as soon as it is planned
   Frames fr;
   fr.reset(st->n);
-  return plan_parts(st->n, st->q2s, all, &fr, true, g_tile_hint.load(), st->dtype,
+  return plan_parts(st->n, st->q2s, all, &fr, true, g_tile_hint.load(), st->dtype, true,
                     [&](PlannedPass& p) {
                       TimedRegion tr(S(st, stream));
                       return launch_pass(st, p, S(st, stream));
@@ -524,15 +524,18 @@ int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_o
       return set_error(HS_E_INVALID, "part offsets must be non-decreasing");
   // plan every part before the first launch, so that the device never waits
   // for the host between two parts and each event pair brackets one part only
+  std::vector<std::vector<LoweredGate>> all(num_parts);
+  for (int p = 0; p < num_parts; ++p)
+    HS_TRY(lower_all(st, gates + part_offsets[p], part_offsets[p + 1] - part_offsets[p],
+                     &all[p]));
   std::vector<std::vector<PlannedPass>> progs(num_parts);
   Frames fr;
   fr.reset(st->n);
-  for (int p = 0; p < num_parts; ++p) {
-    std::vector<LoweredGate> lg;
-    HS_TRY(lower_all(st, gates + part_offsets[p], part_offsets[p + 1] - part_offsets[p], &lg));
-    HS_TRY(plan_passes(st->n, st->q2s, lg, &fr, p == num_parts - 1, g_tile_hint.load(),
-                       st->dtype, &progs[p]));
-  }
+  HS_TRY(plan_parts(st->n, st->q2s, all, &fr, true, g_tile_hint.load(), st->dtype, false,
+                    [&](PlannedPass& p) {
+                      progs[p.of_part].push_back(std::move(p));
+                      return HS_OK;
+                    }));
   std::vector<cudaEvent_t> ev(num_parts + 1, nullptr);
   int rc = HS_OK;
   for (auto& e : ev)

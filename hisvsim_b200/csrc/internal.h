@@ -299,6 +299,7 @@ static_assert(sizeof(WideProgram) <= 32700, "kernel parameter space");
 struct PlannedPass {
   std::unique_ptr<PartProgram> part;
   std::unique_ptr<WideProgram> wide;
+  int of_part = 0;  // plan_parts
   int nops() const { return wide ? wide->nops : part->nops; }
   size_t bytes() const { return wide ? sizeof(WideProgram) : sizeof(PartProgram); }
 };
@@ -333,11 +334,12 @@ int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
                 Frames* fr, bool flush, int tile_bits_hint, int dtype,
                 std::vector<PlannedPass>* passes);
 // The parts of one call, handed to `sink` pass by pass as they are planned (an
-// error it returns ends the planning).  A pass may take gates of later parts.
+// error it returns ends the planning).  With `merge` a pass may take gates of
+// later parts; without, PlannedPass::of_part is the part it belongs to.
 using PassSink = std::function<int(PlannedPass&)>;
 int plan_parts(int n, const std::vector<int>& q2s,
                const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
-               int tile_bits_hint, int dtype, const PassSink& sink);
+               int tile_bits_hint, int dtype, bool merge, const PassSink& sink);
 // one self-contained part: fresh frames, flushed at the end
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
               int tile_bits_hint, int dtype, std::vector<PartProgram>* programs);

@@ -885,7 +885,8 @@ bool use_wide(int n, int dtype) {
 }
 
 // Whether gates of later parts may move into earlier passes.  Complex64 calls
-// keep a pass per part, as hs_parts_run_timed does.
+// keep their parts' passes: hs_parts_run_timed, which times the parts one by one,
+// gives the same bits there.
 bool moves_gates(int dtype) { return dtype == HS_DTYPE_C128; }
 
 // Gates a wide program can hold: rotations, flushes, phases, X under any
@@ -1765,29 +1766,35 @@ namespace {
 
 // The parts of a call, window by window: a window's passes are on the device
 // before the next window is rewritten, and what a chunk walks stays bounded, so
-// planning is linear in the gates.  Where gates may move a window takes whole
-// parts up to kWindowGates gates (one part at least): half a millisecond of planning ahead of
-// its first pass, and at most one pass more than over the whole call per some
-// thirty; elsewhere it is one part.
+// planning is linear in the gates.  Where gates may move (`merge`) a window takes
+// whole parts up to kWindowGates gates (one part at least): half a millisecond of
+// planning ahead of its first pass, and at most one pass more than over the whole
+// call per some thirty; elsewhere it is one part.
 constexpr size_t kWindowGates = 1024;
 
 int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr, bool flush,
-              int tile_bits_hint, int dtype, const PassSink& sink) {
+              int tile_bits_hint, int dtype, bool merge, const PassSink& sink) {
   if (int(fr->r.size()) != n) fr->reset(n);
   const bool wide = use_wide(n, dtype);
   const bool flips = wide && (tile_bits_hint <= 0 || tile_bits_hint >= kWideMinTileBits) &&
                      all_wide(parts, *fr);
-  const size_t most = wide && moves_gates(dtype) ? kWindowGates : 0;
+  const size_t most = wide && merge && moves_gates(dtype) ? kWindowGates : 0;
   size_t i = 0;
+  int first = 0;
+  const PassSink tagged = [&](PlannedPass& p) {
+    p.of_part = first;
+    return sink(p);
+  };
   do {
     Parts window;
+    first = int(i);
     for (size_t count = 0; i < parts.size(); ++i) {
       count += parts[i]->size();
       if (!window.empty() && count > most) break;
       window.push_back(parts[i]);
     }
     HS_TRY(plan_chunks(n, q2s, window, fr, flush && i == parts.size(), tile_bits_hint, dtype, flips,
-                       nullptr, &sink));
+                       nullptr, &tagged));
   } while (i < parts.size());
   return HS_OK;
 }
@@ -1796,10 +1803,10 @@ int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr
 
 int plan_parts(int n, const std::vector<int>& q2s,
                const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
-               int tile_bits_hint, int dtype, const PassSink& sink) {
+               int tile_bits_hint, int dtype, bool merge, const PassSink& sink) {
   Parts all;
   for (const auto& p : parts) all.push_back(&p);
-  return plan_call(n, q2s, all, fr, flush, tile_bits_hint, dtype, sink);
+  return plan_call(n, q2s, all, fr, flush, tile_bits_hint, dtype, merge, sink);
 }
 
 int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,
@@ -1810,7 +1817,7 @@ int plan_passes(int n, const std::vector<int>& q2s, const std::vector<LoweredGat
     passes->push_back(std::move(p));
     return HS_OK;
   };
-  return plan_call(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, sink);
+  return plan_call(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, false, sink);
 }
 
 int plan_part(int n, const std::vector<int>& q2s, const std::vector<LoweredGate>& gates,

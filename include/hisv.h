@@ -173,9 +173,12 @@ int hs_part_run(hs_state* st, const hs_gate* gates, int num_gates, void* stream)
 int hs_parts_run(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,
                  int num_parts, void* stream);
 
-/* hs_parts_run with every part planned first and then launched back to back,
- * part_ms[p] = device time of part p (CUDA events between consecutive parts;
- * synchronises).  The harvest of part timings for the cost model. */
+/* The parts of hs_parts_run, every one planned first and then launched back to
+ * back, part_ms[p] = device time of part p (CUDA events between consecutive
+ * parts; synchronises).  Each part keeps its own passes: complex64 states get the
+ * bits of hs_parts_run, complex128 states, where that call moves gates between
+ * parts, its amplitudes to rounding.  The harvest of part timings for the cost
+ * model. */
 int hs_parts_run_timed(hs_state* st, const hs_gate* gates, const int32_t* part_offsets,
                        int num_parts, float* part_ms, void* stream);
 

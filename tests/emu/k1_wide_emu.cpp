@@ -214,7 +214,8 @@ extern "C" {
 const char* wide_last_error() { return g_err; }
 
 // Plan parts (mode 0: one by one, frames carried and flushed by the last; 1:
-// each on its own; 2: as one call, gates moving into earlier parts' passes) on a
+// each on its own; 2: as one call, gates moving into earlier parts' passes; 3: as
+// one call, every part with its own passes, as hs_parts_run_timed) on a
 // state whose qubit q sits in slot q2s[q], run the wide passes on `amps` (slot order,
 // 2^n complex128, in/out; complex64 rounds).  stats: {passes, wide passes,
 // groups, steps, tables}.
@@ -254,8 +255,8 @@ int wide_parts_run(int n, int dtype, const hs_gate* gates, const int32_t* offs, 
       if (rc != HS_OK) return rc;
     }
   }
-  if (mode == 2) {
-    const int rc = plan_parts(n, q2s, parts, &fr, true, tile_hint, dtype, sink);
+  if (mode >= 2) {
+    const int rc = plan_parts(n, q2s, parts, &fr, true, tile_hint, dtype, mode == 2, sink);
     if (rc != HS_OK) return rc;
   } else {
     for (int p = 0; p < nparts; ++p) {
@@ -295,7 +296,7 @@ extern "C" int wide_plan_time(int n, int dtype, const hs_gate* gates, const int3
   *passes = 0;
   const auto t0 = std::chrono::steady_clock::now();
   auto now = [&] { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); };
-  const int rc = plan_parts(n, q2s, parts, &fr, true, 0, dtype, [&](PlannedPass&) {
+  const int rc = plan_parts(n, q2s, parts, &fr, true, 0, dtype, true, [&](PlannedPass&) {
     if (++*passes == 1) seconds[0] = now();
     return HS_OK;
   });

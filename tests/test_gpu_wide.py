@@ -57,3 +57,22 @@ def test_gates_diagonal_to_rounding(port, m, dtype, tol):
         st.run_part_carry(fr, rec[offs[p]:offs[p + 1]])
     st.flush(fr)
     assert np.abs(st.amplitudes() - want).max() <= tol
+
+
+@pytest.mark.parametrize("odd", [None, Gate("H", (0,), (1,)), Gate("RXX", (3, 1), params=(0.3,))])
+def test_timed_parts_match_the_plain_call(port, odd):
+    """run_parts_timed: the bits of run_parts in complex64, also where one part holds a
+    gate outside the wide form; its amplitudes in complex128."""
+    n = 12
+    parts = [[Gate("H", (q,)) for q in range(n)] + [Gate("RY", (q,), params=(3.0,)) for q in range(n)],
+             ([odd] if odd else []) + [Gate("U3", (2,), params=(2.5, 0.3, 1.0))], _mixed(n, 2, 6)]
+    rec, offs = part_offsets(parts)
+    want = port.run(n, rec)
+    for dtype, tol in ((abi.C64, 1e-5), (abi.C128, 1e-12)):
+        a, b = abi.State(n, dtype), abi.State(n, dtype)
+        a.run_parts(rec, offs)
+        ms = b.run_parts_timed(rec, offs)
+        assert len(ms) == len(parts)
+        x, y = a.amplitudes(), b.amplitudes()
+        assert dtype != abi.C64 or np.array_equal(x, y)
+        assert max(np.abs(x - want).max(), np.abs(y - want).max()) <= tol

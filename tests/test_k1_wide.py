@@ -235,3 +235,19 @@ def test_long_calls_are_planned_as_they_run(emu, dtype):
     assert first <= total / 5
     assert total <= 16 * short
     assert many <= 9 * few
+
+
+def test_timed_calls_plan_as_plain_ones(emu, port):
+    """hs_parts_run_timed's passes (mode 3): in complex64 those of hs_parts_run, a part
+    outside the wide form among them (the emulator leaves such passes out in both);
+    in complex128 the same amplitudes to rounding."""
+    n = 11
+    for odd in ([], [Gate("H", (0,), (1,))], [Gate("RXX", (0, 1), params=(0.3,))]):
+        parts = [[Gate("H", (q,)) for q in range(n)] + [Gate("RY", (q,), params=(3.0,)) for q in range(n)],
+                 odd + [Gate("U3", (2,), params=(2.5, 0.3, 1.0))], _mixed(n, 1, 6)]
+        plain, a = emu(n, parts, dtype=1, mode=2)
+        timed, b = emu(n, parts, dtype=1, mode=3)
+        assert a == b and np.array_equal(plain, timed)
+        if not odd:
+            want = port.run(n, to_records([g for p in parts for g in p]))
+            assert np.abs(emu(n, parts, mode=3)[0] - want).max() <= 1e-12
