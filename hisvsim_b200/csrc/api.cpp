@@ -149,15 +149,16 @@ cudaError_t state_alloc(void** p, size_t bytes) {
   return device_malloc(p, bytes);
 }
 
-void state_free(const hs_state* st) {
+// whether the state's work has ended (freeing its memory waits for it)
+bool state_free(const hs_state* st) {
   const size_t bytes = amp_bytes(st->dtype) << st->n;
   int cur = -1;
   if (!st->elsewhere && bytes <= kKeptBlock && cudaGetDevice(&cur) == cudaSuccess &&
       cur == st->dev && cudaStreamSynchronize(nullptr) == cudaSuccess && st->ctx == context_id()) {
     for (void* p : kept_states(cur).put(st->ctx, st->amp, bytes)) cudaFree(p);
-    return;
+    return true;
   }
-  cudaFree(st->amp);
+  return cudaFree(st->amp) == cudaSuccess;
 }
 
 }  // namespace
@@ -214,7 +215,7 @@ int permute_positions(hs_state* st, const std::vector<int>& pi, cudaStream_t s) 
 }
 
 int launch_pass(hs_state* st, const PlannedPass& p, cudaStream_t s) {
-  HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, s)
+  HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, st->ticket, s)
                 : launch_part(st->amp, st->dtype, *p.part, s));
   count_pass(p.nops());
   g_param_bytes += (long long)p.bytes();
@@ -323,13 +324,16 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
   st->q2s.resize(num_qubits);
   st->s2q.resize(num_qubits);
   for (int q = 0; q < num_qubits; ++q) st->q2s[q] = st->s2q[q] = q;
-  int rc = set_basis_kernel(st->amp, dtype, num_qubits, 0, nullptr);
+  st->ticket_id = ticket_take();
+  st->ticket = ticket_address(st->ticket_id);
+  int rc = set_basis_kernel(st->amp, dtype, num_qubits, 0, st->ticket, nullptr);
   if (rc == HS_OK) {
     e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) rc = set_error(HS_E_CUDA, "init: %s", cudaGetErrorString(e));
   }
   if (rc != HS_OK) {
     cudaFree(st->amp);
+    ticket_give(st->ticket_id);
     delete st;
     return rc;
   }
@@ -341,7 +345,7 @@ int hs_state_create(int num_qubits, int dtype, hs_state** out) {
 
 int hs_state_destroy(hs_state* st) {
   if (!st) return HS_OK;
-  if (st->amp) state_free(st);
+  if (st->amp && state_free(st)) ticket_give(st->ticket_id);
   st->amp = nullptr;
   if (--g_live_states[st->dev & 63] == 0) scratch_release(st->dev, st->ctx);
   delete st;
@@ -377,7 +381,7 @@ int hs_state_set_basis(hs_state* st, uint64_t x, void* stream) {
   HS_TRY(check_state(st));
   if (st->n < 64 && (x >> st->n)) return set_error(HS_E_INVALID, "basis index out of range");
   for (int q = 0; q < st->n; ++q) st->q2s[q] = st->s2q[q] = q;
-  return set_basis_kernel(st->amp, st->dtype, st->n, x, S(st, stream));
+  return set_basis_kernel(st->amp, st->dtype, st->n, x, st->ticket, S(st, stream));
 }
 
 int hs_state_copy_to_host(hs_state* st, void* host, uint64_t first, uint64_t count,

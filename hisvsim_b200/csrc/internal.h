@@ -488,7 +488,12 @@ cudaError_t device_malloc(T** p, size_t bytes) {
 
 // ---- launchers (kernels_*.cu) ----------------------------------------------
 int launch_part(void* amp, int dtype, const PartProgram& prog, cudaStream_t s);
-int launch_wide(void* amp, int dtype, const WideProgram& prog, cudaStream_t s);
+// `ticket`: the state's tile counter (device; null = none), left at 0
+int launch_wide(void* amp, int dtype, const WideProgram& prog, uint32_t* ticket, cudaStream_t s);
+// a free tile counter (-1: none left), and its device address
+int ticket_take();
+void ticket_give(int i);
+uint32_t* ticket_address(int i);
 int launch_permute(void* amp, int dtype, int n, const int32_t* pairs, int npairs,
                    cudaStream_t s);
 int reduce_norm2(const void* amp, int dtype, int n, double* out, cudaStream_t s);
@@ -516,7 +521,8 @@ struct MeasureChunk {
 int sample_chunks(const void* amp, int dtype, int chunk_bits,
                   const std::vector<MeasureChunk>& chunks, const std::vector<double>& u,
                   uint64_t* pos, cudaStream_t s);
-int set_basis_kernel(void* amp, int dtype, int n, uint64_t index, cudaStream_t s);
+// (resets the state's tile counter, null = none, as well)
+int set_basis_kernel(void* amp, int dtype, int n, uint64_t index, uint32_t* ticket, cudaStream_t s);
 // out[j] = in[offset | deposit(j, old_slots)] for j < 2^out_bits
 int project_kernel(const void* in, void* out, int dtype, int out_bits, const int* old_slots,
                    uint64_t offset, cudaStream_t s);
@@ -584,6 +590,8 @@ struct hs_state {
   void* amp = nullptr;  // device, slot-ordered
   int dev = 0;          // the device and the context (context_id) it was created on
   uint64_t ctx = 0;
+  int ticket_id = -1;   // its tile counter (launch_wide)
+  uint32_t* ticket = nullptr;
   // its device pointer was handed out, or a call ran on another stream than the default one
   mutable std::atomic<bool> elsewhere{false};
   std::vector<int> q2s, s2q;

@@ -409,8 +409,9 @@ __global__ void __launch_bounds__(kRedThreads) k3_chunks(const V* __restrict__ a
 }
 
 template <typename V>
-__global__ void k_set_basis(V* __restrict__ sv, uint64_t size, uint64_t index) {
+__global__ void k_set_basis(V* __restrict__ sv, uint64_t size, uint64_t index, uint32_t* ticket) {
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+  if (ticket && blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < size; i += stride) {
     V v;
     v.x = i == index ? 1 : 0;
@@ -912,14 +913,15 @@ int fp64_probe(double* tflops) {
   return HS_OK;
 }
 
-int set_basis_kernel(void* amp, int dtype, int n, uint64_t index, cudaStream_t s) {
+int set_basis_kernel(void* amp, int dtype, int n, uint64_t index, uint32_t* ticket,
+                     cudaStream_t s) {
   const uint64_t size = 1ull << n;
   if (dtype == HS_DTYPE_C128)
     k_set_basis<double2><<<grid_for(size, 256), 256, 0, s>>>(static_cast<double2*>(amp), size,
-                                                             index);
+                                                             index, ticket);
   else
     k_set_basis<float2><<<grid_for(size, 256), 256, 0, s>>>(static_cast<float2*>(amp), size,
-                                                            index);
+                                                            index, ticket);
   HS_CUDA(cudaGetLastError());
   return HS_OK;
 }

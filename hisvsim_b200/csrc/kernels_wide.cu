@@ -5,6 +5,8 @@
 // register group runs, exchanged through shared memory between groups, stored
 // straight from the last group's registers -- for the same entry points.
 #include <atomic>
+#include <mutex>
+#include <vector>
 
 #include "bounds.cuh"
 #include "internal.h"
@@ -272,11 +274,25 @@ __device__ __forceinline__ uint64_t deposit(uint64_t x, const Runs& r) {
   return out;
 }
 
+// The tile after the present one, and the number drawn for the one after that.
+struct NextTile {
+  uint64_t base;
+  uint32_t tile, drawn;
+};
+
+// Tiles are handed out in order, by a counter of the state's (`ticket`, 0 between
+// launches: a launch counts to its number of tiles and wraps).  The tiles in
+// flight are then always neighbours, and the sectors and DRAM pages that
+// neighbouring tiles share are read and written once.  With every CTA on a fixed
+// stride of tiles the CTAs drift apart and meet their neighbours' sectors after
+// they left the L2: complex128, 33 qubits in frontier parts of 12, 7 layers, 1661
+// ms against 812; 30 qubits in parts of 9, where whole lines are read, 145
+// against 125.  A state without a counter keeps the stride.
 // OPS: the program has other ops than rotations, signs, tables and negations
 template <bool OPS, typename V>
 __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
-    k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+    k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P, uint32_t* ticket) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];  // the tile, then a NextTile
   const uint32_t t = threadIdx.x;
   const uint32_t tile_bytes = uint32_t(sizeof(V)) << P.m;
   const uint64_t size = 1ull << P.n;  // amplitudes of the state (bounds checks)
@@ -299,19 +315,20 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
         cp_async16(sb + (ct ^ P.cslot[k]), base + P.gchunk[k]);
     cp_async_commit();
   };
-  uint64_t tile = blockIdx.x;
-  uint64_t gbase = tile < P.ntiles ? deposit(tile, P.outer) : 0;
-  // the next tile's offset by one addition in the scattered outer bits (the
-  // carries run through the other bits, which are set)
-  const uint64_t omask = deposit(P.ntiles - 1, P.outer);
-  const uint64_t ostep = deposit(uint64_t(gridDim.x), P.outer);
-  if (tile < P.ntiles) issue(gbase);
+  uint32_t tile = blockIdx.x;
+  const uint32_t ntiles = uint32_t(P.ntiles);
+  uint64_t gbase = deposit(tile, P.outer);
+  NextTile& N = *reinterpret_cast<NextTile*>(smem_raw + (sizeof(V) << P.m));
+  // one number per tile: a launch draws ntiles in all
+  auto draw = [&](uint32_t after) {
+    if (t == 0) N.drawn = ticket ? gridDim.x + atomicInc(ticket, ntiles - 1) : after + gridDim.x;
+  };
+  issue(gbase);
+  draw(tile);
   cp_async_wait();
   __syncthreads();
   V v[E];
-  for (; tile < P.ntiles; tile += gridDim.x) {
-    const uint64_t next = tile + gridDim.x;
-    const uint64_t gnext = next < P.ntiles ? (((gbase | ~omask) + ostep) & omask) : 0;
+  while (tile < ntiles) {
     for (int g = 0; g < P.ngroups; ++g) {
       const WideGroup& G = P.groups[g];
       const bool last = g == P.ngroups - 1;
@@ -334,8 +351,12 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
       if (last) {
         // every thread holds its registers of the last group: the buffer takes
         // the next tile while this one is finished and stored
+        if (t == 0) {
+          N.tile = N.drawn;
+          N.base = deposit(N.drawn, P.outer);
+        }
         __syncthreads();
-        if (next < P.ntiles) issue(gnext);
+        if (N.tile < ntiles) issue(N.base);
       }
       uint32_t z = 0;  // pending signs (WideSign)
       for (int s = G.first_step, s_end = s + G.num_steps; s < s_end; ++s) {
@@ -393,6 +414,9 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
           }
           if (HS_IN_BOUNDS(uint64_t(p - sv) < size, kBoundsK1)) __stcs(p, v[e]);
         }
+        tile = N.tile;
+        gbase = N.base;
+        if (tile < ntiles) draw(tile);  // (while the copies are awaited)
         cp_async_wait();  // the next tile's copies (the only ones in flight)
       } else {
         const uint32_t a1 = a0 ^ G.tw[kWideFlipEntry];
@@ -403,16 +427,15 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
       }
       __syncthreads();
     }
-    gbase = gnext;
   }
 }
 
 template <bool OPS, typename V>
-int launch(V* sv, const WideProgram& P, cudaStream_t s) {
+int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   constexpr auto kernel = k1_wide<OPS, V>;
   HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
   const int threads = 1 << (P.m - kWideBits);
-  const size_t smem = sizeof(V) << P.m;
+  const size_t smem = (sizeof(V) << P.m) + sizeof(NextTile);
   // resident CTAs per SM, looked up once per device and tile size (the call
   // costs as much host time as the launch of a small pass)
   static std::atomic<int> resident[64][kWideMaxTileBits + 1];
@@ -425,26 +448,19 @@ int launch(V* sv, const WideProgram& P, cudaStream_t s) {
     if (per_sm < 1) return set_error(HS_E_UNSUPPORTED, "K1 tile does not fit an SM (m=%d)", P.m);
     cached.store(per_sm, std::memory_order_relaxed);
   }
-  // Tiles whose runs are 16 bytes or less read sectors that their neighbours share,
-  // from the L2 if those come soon: on states beyond 8 GiB two CTAs per SM keep
-  // fewer tiles in flight (passes of 12 targets, complex128 30 qubits 27.5 -> 20.8
-  // ms, complex64 34 qubits 356 -> 169 ms; 28 qubits 2.2 -> 2.7 ms, and with runs
-  // of 32 bytes and more the full occupancy is as fast or faster).
-  int run = 0;
-  while (run < P.m && P.tile_slot[run] == run) ++run;
-  if ((sizeof(V) << run) <= 16 && (sizeof(V) << P.n) > (8ull << 30)) per_sm = per_sm < 2 ? per_sm : 2;
   const uint64_t want = uint64_t(device_sms()) * uint64_t(per_sm);
   const int grid = int(P.ntiles < want ? P.ntiles : want);
-  kernel<<<grid, threads, smem, s>>>(sv, P);
+  // (a launch with a CTA per tile hands none out)
+  kernel<<<grid, threads, smem, s>>>(sv, P, uint64_t(grid) < P.ntiles ? ticket : nullptr);
   HS_CUDA(cudaGetLastError());
   return HS_OK;
 }
 
 template <typename V>
-int launch_typed(V* sv, const WideProgram& P, cudaStream_t s) {
+int launch_typed(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   bool ops = false;
   for (int i = 0; i < P.nwops; ++i) ops |= P.ops[i].code != wk_neg;
-  return ops ? launch<true>(sv, P, s) : launch<false>(sv, P, s);
+  return ops ? launch<true>(sv, P, ticket, s) : launch<false>(sv, P, ticket, s);
 }
 
 }  // namespace
@@ -453,9 +469,45 @@ int launch_typed(V* sv, const WideProgram& P, cudaStream_t s) {
 HS_BOUNDS_TAKE(bounds_take_wide)
 #endif
 
-int launch_wide(void* amp, int dtype, const WideProgram& P, cudaStream_t s) {
-  if (dtype == HS_DTYPE_C128) return launch_typed(static_cast<double2*>(amp), P, s);
-  return launch_typed(static_cast<float2*>(amp), P, s);
+int launch_wide(void* amp, int dtype, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
+  if (dtype == HS_DTYPE_C128) return launch_typed(static_cast<double2*>(amp), P, ticket, s);
+  return launch_typed(static_cast<float2*>(amp), P, ticket, s);
+}
+
+// The states' tile counters: one 32-byte sector each of a fixed array, so that a
+// launch needs no memory of its own and none is reset between launches.  (Calls
+// on one state are ordered among themselves; states share no counter.)
+namespace {
+constexpr int kTickets = 4096, kTicketStride = 8;
+__device__ uint32_t g_tickets[kTickets * kTicketStride];
+std::mutex g_ticket_mu;
+std::vector<int> g_ticket_free;
+int g_ticket_next = 0;
+}  // namespace
+
+int ticket_take() {
+  std::lock_guard<std::mutex> lk(g_ticket_mu);
+  if (!g_ticket_free.empty()) {
+    const int i = g_ticket_free.back();
+    g_ticket_free.pop_back();
+    return i;
+  }
+  return g_ticket_next < kTickets ? g_ticket_next++ : -1;
+}
+
+void ticket_give(int i) {
+  if (i < 0) return;
+  std::lock_guard<std::mutex> lk(g_ticket_mu);
+  g_ticket_free.push_back(i);
+}
+
+uint32_t* ticket_address(int i) {
+  void* p = nullptr;
+  if (i < 0 || cudaGetSymbolAddress(&p, g_tickets) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return static_cast<uint32_t*>(p) + size_t(i) * kTicketStride;
 }
 
 }  // namespace hisv

@@ -76,3 +76,62 @@ def test_timed_parts_match_the_plain_call(port, odd):
         x, y = a.amplitudes(), b.amplitudes()
         assert dtype != abi.C64 or np.array_equal(x, y)
         assert max(np.abs(x - want).max(), np.abs(y - want).max()) <= tol
+
+
+@pytest.mark.parametrize("dtype,tol", [(abi.C128, 1e-12), (abi.C64, 1e-5)])
+@pytest.mark.parametrize("hint,n", [(10, 22), (11, 21), (12, 22), (0, 22)])
+def test_more_tiles_than_ctas(port, dtype, tol, hint, n):
+    """Tiles drawn from the state's counter: it is back at 0 after every pass (a second
+    run gives the same bits), two states at once on two streams have their own, and a
+    captured run replays."""
+    import torch
+
+    gates = circuits.random_u3_cz(n, 2, n) + [Gate("X", (0,), (n - 1,)), Gate("SWAP", (1, n - 2))]
+    rec, offs = part_offsets(partition.parts_to_gates(gates, partition.partition_frontier(gates, 10)))
+    want = port.run(n, to_records(gates))
+    prev = abi.set_tile_qubits(hint)
+    try:
+        st = [abi.State(n, dtype) for _ in range(2)]
+        st[0].run_parts(rec, offs)
+        first = st[0].amplitudes()
+        assert np.abs(first - want).max() <= tol
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        for s, x in zip(st, streams):
+            s.set_basis(0, stream=x.cuda_stream)
+        for _ in range(2):
+            for s, x in zip(st, streams):
+                s.set_basis(0, stream=x.cuda_stream)
+                s.run_parts(rec, offs, stream=x.cuda_stream)
+        torch.cuda.synchronize()
+        assert all(np.array_equal(s.amplitudes(), first) for s in st)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(streams[0]):
+            g.capture_begin(capture_error_mode="thread_local")
+            st[0].set_basis(0, stream=streams[0].cuda_stream)
+            st[0].run_parts(rec, offs, stream=streams[0].cuda_stream)
+            g.capture_end()
+        for _ in range(3):
+            st[0].load(np.zeros(1 << n, st[0].np_dtype))
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(st[0].amplitudes(), first)
+    finally:
+        abi.set_tile_qubits(prev)
+
+
+def test_passes_without_low_slots_are_not_slower_than_the_general_form():
+    """29 qubits, complex128, passes whose 12 targets leave no low slot (runs of 16
+    bytes): the wide form is the one taken, so the general form (8 amplitudes per
+    thread) does not run the same pass faster."""
+    n = 29
+    st = abi.State(n)
+    for qs in ([3, 5, 7, 12, 13, 14, 15, 16, 17, 24, 27, 28], [7, 12, 13, 14, 15, 17, 18, 19, 20, 23, 26, 28]):
+        rec, offs = part_offsets([[Gate("U3", (q,), params=(0.3 + q, 0.1, 0.2)) for q in qs for _ in range(2)]])
+        ms = {}
+        for r in (3, 4):
+            prev = abi.set_k1_reg_bits(r)
+            try:
+                ms[r] = min(float(st.run_parts_timed(rec, offs)[0]) for _ in range(4))
+            finally:
+                abi.set_k1_reg_bits(prev)
+        assert ms[4] <= ms[3], ms
