@@ -773,26 +773,28 @@ int hs_measure(hs_state* st, const int32_t* qubits, int num_qubits, uint32_t num
   std::vector<double> u(num_samples);
   for (auto& x : u) x = dis(gen);
   std::sort(u.begin(), u.end());
-  const int cb = std::min(st->n, 16);
+  const int cb = std::min(st->n, 16);  // (offsets within a chunk take 16 bits)
   std::vector<double> chunk(size_t(1) << (st->n - cb));
   HS_TRY(reduce_chunks(st->amp, st->dtype, st->n, cb, chunk.data(), nullptr));
   // the chunk of every sample, from the chunks' masses; the device finds the
   // amplitude within it
-  std::vector<MeasureChunk> touched;
+  uint32_t placed = 0;
+  const std::vector<MeasureChunk> touched = place_samples(chunk, cb, u, kSamplesPerBlock, &placed);
+  std::vector<uint16_t> off(num_samples);  // within the sample's chunk
+  HS_TRY(sample_chunks(st->amp, st->dtype, cb, touched, u, off.data(), nullptr));
   uint32_t k = 0;
-  double cum = 0;
-  for (size_t c = 0; c < chunk.size() && k < num_samples; ++c) {
-    const uint32_t s0 = k;
-    while (k < num_samples && u[k] < cum + chunk[c]) ++k;
-    if (k > s0) touched.push_back({uint64_t(c) << cb, cum, s0, k - s0});
-    cum += chunk[c];
-  }
-  const uint32_t placed = k;
-  std::vector<uint64_t> pos(num_samples);
-  HS_TRY(sample_chunks(st->amp, st->dtype, cb, touched, u, pos.data(), nullptr));
-  for (k = 0; k < placed; ++k)
-    for (int j = 0; j < num_qubits; ++j)
-      out[size_t(k) * num_qubits + j] = int32_t((pos[k] >> slots[j]) & 1);
+  uint64_t last = ~0ull;
+  for (const MeasureChunk& c : touched)
+    for (uint32_t i = 0; i < c.ns; ++i, ++k) {
+      const uint64_t pos = c.first + off[k];
+      int32_t* row = out + size_t(k) * num_qubits;
+      if (pos == last) {  // (the points are sorted: on small states most repeat)
+        std::memcpy(row, row - num_qubits, sizeof(int32_t) * num_qubits);
+        continue;
+      }
+      for (int j = 0; j < num_qubits; ++j) row[j] = int32_t((pos >> slots[j]) & 1);
+      last = pos;
+    }
   // samples beyond the accumulated mass read as all ones (state_vector.hpp:969-978)
   for (; k < num_samples; ++k)
     for (int j = 0; j < num_qubits; ++j) out[size_t(k) * num_qubits + j] = 1;

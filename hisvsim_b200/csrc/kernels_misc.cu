@@ -322,18 +322,18 @@ __global__ void __launch_bounds__(kRedThreads)
 struct SampleChunk {
   uint64_t first;      // first amplitude of the chunk
   double base;         // mass before it
-  uint32_t s0, ns;     // its samples in u / pos
+  uint32_t s0, ns;     // its samples in u / off
 };
 
-// One block per chunk with samples.  The chunk (2^chunk_bits amplitudes) is cut
-// into up to 256 runs; the warps sum the runs, one warp scans the run sums, and
-// each sample's warp then walks its run in steps of 32 amplitudes.  A sample
-// that the rounding of the sums leaves beyond the chunk takes the chunk's last
-// amplitude of non-zero probability.
+// One block per work item: a chunk and up to kSamplesPerBlock of its samples.  The
+// chunk (2^chunk_bits amplitudes) is cut into up to 256 runs; the warps sum the
+// runs, one thread scans the run sums, and each sample's warp then walks its run
+// in steps of 32 amplitudes.  A sample that the rounding of the sums leaves beyond
+// the chunk takes the chunk's last amplitude of non-zero probability.
 template <typename V>
 __global__ void __launch_bounds__(kRedThreads)
     k3_sample(const V* __restrict__ a, int chunk_bits, const SampleChunk* __restrict__ chunks,
-              const double* __restrict__ u, uint64_t* __restrict__ pos) {
+              const double* __restrict__ u, uint16_t* __restrict__ off) {
   __shared__ double run[kRedThreads];  // sums, then the mass up to and including each run
   const SampleChunk C = chunks[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kRedThreads / 32;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kRedThreads)
       const uint32_t some = __ballot_sync(0xffffffffu, i >= 0 && prob(i < 0 ? 0 : i) > 0.0);
       if (some) last = i1 - 1 - __clz(int(some));
     }
-    if (lane == 0) pos[C.s0 + k] = C.first + uint64_t(found >= 0 ? found : last >= 0 ? last : 0);
+    if (lane == 0) off[C.s0 + k] = uint16_t(found >= 0 ? found : last >= 0 ? last : 0);
   }
 }
 
@@ -783,16 +783,17 @@ int reduce_zz(const void* amp, int dtype, int n, const int32_t* slot_pairs, int 
 
 int sample_chunks(const void* amp, int dtype, int chunk_bits,
                   const std::vector<MeasureChunk>& chunks, const std::vector<double>& u,
-                  uint64_t* pos, cudaStream_t s) {
+                  uint16_t* off, cudaStream_t s) {
   static_assert(sizeof(SampleChunk) == sizeof(MeasureChunk), "chunk layout");
   if (chunks.empty()) return HS_OK;
   const size_t cb = sizeof(SampleChunk) * chunks.size(), ub = sizeof(double) * u.size();
-  Scratch sc;  // [chunks | u | positions]
-  HS_TRY(sc.get(cb + 2 * ub));
+  const size_t ob = sizeof(uint16_t) * u.size();
+  Scratch sc;  // [chunks | u | offsets]
+  HS_TRY(sc.get(cb + ub + ob));
   char* scratch = sc.bytes();
   auto* dc = reinterpret_cast<SampleChunk*>(scratch);
   auto* du = reinterpret_cast<double*>(scratch + cb);
-  auto* dp = reinterpret_cast<uint64_t*>(scratch + cb + ub);
+  auto* dp = reinterpret_cast<uint16_t*>(scratch + cb + ub);
   cudaError_t e[5];
   e[0] = cudaMemcpyAsync(dc, chunks.data(), cb, cudaMemcpyHostToDevice, s);
   e[1] = cudaMemcpyAsync(du, u.data(), ub, cudaMemcpyHostToDevice, s);
@@ -803,7 +804,7 @@ int sample_chunks(const void* amp, int dtype, int chunk_bits,
     k3_sample<float2><<<unsigned(chunks.size()), kRedThreads, 0, s>>>(
         static_cast<const float2*>(amp), chunk_bits, dc, du, dp);
   e[2] = cudaGetLastError();
-  e[3] = cudaMemcpyAsync(pos, dp, ub, cudaMemcpyDeviceToHost, s);
+  e[3] = cudaMemcpyAsync(off, dp, ob, cudaMemcpyDeviceToHost, s);
   e[4] = sc.finish(s);
   for (cudaError_t x : e)
     if (x != cudaSuccess) return set_error(HS_E_CUDA, "samples: %s", cudaGetErrorString(x));

@@ -55,3 +55,19 @@ def test_samples_follow_the_distribution(n, samples, zeros, dtype):
     assert np.all(p[idx] > 0)
     assert np.all(cum[idx] >= u - 1e-12)
     assert np.all(cum[idx] - p[idx] <= u + 1e-12)
+
+
+@pytest.mark.parametrize("n,samples", [(1, 300), (10, 5000), (16, 5000), (17, 3001)])
+def test_many_samples_of_a_small_state(n, samples):
+    """More samples than one block searches: the points of the seed, as in
+    test_samples_follow_the_distribution."""
+    st, p = _state(n, abi.C128, 90 + n, n > 2)
+    seed = 77 + n
+    got = st.measure(list(range(n)), samples, seed)
+    idx = (got.astype(np.int64) << np.arange(n)).sum(axis=1)
+    raw = np.random.RandomState(seed)._bit_generator.random_raw(2 * samples).astype(np.float64)
+    u = np.sort((raw[0::2] + raw[1::2] * 2.0 ** 32) / 2.0 ** 64)
+    cum = np.cumsum(p)
+    assert np.all(p[idx] > 0)
+    assert np.all(cum[idx] >= u - 1e-12)
+    assert np.all(cum[idx] - p[idx] <= u + 1e-12)
