@@ -29,8 +29,10 @@ def port():
 
 @pytest.fixture(scope="session")
 def ref():
-    from oracle.oracle import RefOracle
+    from oracle.oracle import REF_LIB, RefOracle
 
+    if not os.path.exists(REF_LIB):
+        pytest.skip(f"{REF_LIB} missing: `make -C oracle ref` builds it from the reference's checkout")
     return RefOracle()
 
 
