@@ -253,7 +253,11 @@ def run_reference_arm(args):
     gate_vals, parts_vals = [], []
     r = None
     for i in range(args.warmup + args.steps):
-        r = cpu_sample(args, threads)
+        try:
+            r = cpu_sample(args, threads)
+        except FileNotFoundError as e:
+            print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+            return
         if i >= args.warmup:
             gate_vals.append(r["per_gate"]["value"])
             parts_vals.append(r["parts"]["value"])

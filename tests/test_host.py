@@ -314,3 +314,22 @@ def test_bench_partitions(monkeypatch):
         assert len({q for i in p for q in gates[i].qubits}) <= 9
     fused = bench.partitioner(args)(gates, 6)
     assert all(len({q for i in p for q in gates[i].qubits}) <= 6 for p in fused)
+
+
+def test_reference_arm_says_why_it_is_unavailable(monkeypatch, capsys):
+    """bench.py --impl reference without the reference's library: one line, no error."""
+    import json
+    import sys
+
+    import bench
+    from oracle import oracle
+
+    class Missing:
+        def __init__(self):
+            raise FileNotFoundError("libhisv_ref.so missing")
+
+    monkeypatch.setattr(oracle, "RefOracle", Missing)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--steps", "1", "--warmup", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "libhisv_ref.so" in line["unavailable"]
