@@ -274,11 +274,21 @@ __device__ __forceinline__ uint64_t deposit(uint64_t x, const Runs& r) {
   return out;
 }
 
-// The tile after the present one, and the number drawn for the one after that.
+// A tile: its number and its offset.
 struct NextTile {
   uint64_t base;
-  uint32_t tile, drawn;
+  uint64_t tile;
 };
+
+// deposit by a whole warp, a run per lane (a loop over the runs costs 0.6 us, on
+// the path of a tile of 10)
+__device__ __forceinline__ uint64_t warp_deposit(uint32_t x, const Runs& r) {
+  const int i = int(threadIdx.x & 31u);
+  uint64_t v = 0;
+  if (i < r.n) v = ((uint64_t(x) >> r.src[i]) & ((1ull << r.len[i]) - 1ull)) << r.dst[i];
+  return uint64_t(__reduce_or_sync(0xffffffffu, uint32_t(v >> 32))) << 32 |
+         __reduce_or_sync(0xffffffffu, uint32_t(v));
+}
 
 // Tiles are handed out in order, by a counter of the state's (`ticket`, 0 between
 // launches: a launch counts to its number of tiles and wraps).  The tiles in
@@ -286,13 +296,13 @@ struct NextTile {
 // neighbouring tiles share are read and written once.  With every CTA on a fixed
 // stride of tiles the CTAs drift apart and meet their neighbours' sectors after
 // they left the L2: complex128, 33 qubits in frontier parts of 12, 7 layers, 1661
-// ms against 812; 30 qubits in parts of 9, where whole lines are read, 145
-// against 125.  A state without a counter keeps the stride.
+// ms against 815; 30 qubits in parts of 9, where whole lines are read, 145
+// against 122.  A state without a counter keeps the stride (as do small launches).
 // OPS: the program has other ops than rotations, signs, tables and negations
 template <bool OPS, typename V>
 __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
     k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P, uint32_t* ticket) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];  // the tile, then a NextTile
+  extern __shared__ __align__(128) unsigned char smem_raw[];  // the tile, then two NextTile
   const uint32_t t = threadIdx.x;
   const uint32_t tile_bytes = uint32_t(sizeof(V)) << P.m;
   const uint64_t size = 1ull << P.n;  // amplitudes of the state (bounds checks)
@@ -318,13 +328,25 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
   uint32_t tile = blockIdx.x;
   const uint32_t ntiles = uint32_t(P.ntiles);
   uint64_t gbase = deposit(tile, P.outer);
-  NextTile& N = *reinterpret_cast<NextTile*>(smem_raw + (sizeof(V) << P.m));
-  // one number per tile: a launch draws ntiles in all
-  auto draw = [&](uint32_t after) {
-    if (t == 0) N.drawn = ticket ? gridDim.x + atomicInc(ticket, ntiles - 1) : after + gridDim.x;
+  // the tile after the present one, known a tile ahead: written by warp 0 into one
+  // entry while the other is read.  One number per tile: a launch draws ntiles in all
+  NextTile* N = reinterpret_cast<NextTile*>(smem_raw + (sizeof(V) << P.m));
+  auto draw = [&](NextTile* to, uint32_t after) {
+    if (t >= 32u) return;
+    uint32_t x = after;
+    if (ticket) {
+      if (t == 0) x = atomicInc(ticket, ntiles - 1);
+      x = __shfl_sync(0xffffffffu, x, 0);
+    }
+    x += gridDim.x;
+    const uint64_t base = warp_deposit(x, P.outer);
+    if (t == 0) {
+      to->tile = x;
+      to->base = base;
+    }
   };
   issue(gbase);
-  draw(tile);
+  draw(N, tile);
   cp_async_wait();
   __syncthreads();
   V v[E];
@@ -351,12 +373,8 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
       if (last) {
         // every thread holds its registers of the last group: the buffer takes
         // the next tile while this one is finished and stored
-        if (t == 0) {
-          N.tile = N.drawn;
-          N.base = deposit(N.drawn, P.outer);
-        }
         __syncthreads();
-        if (N.tile < ntiles) issue(N.base);
+        if (N->tile < ntiles) issue(N->base);
       }
       uint32_t z = 0;  // pending signs (WideSign)
       for (int s = G.first_step, s_end = s + G.num_steps; s < s_end; ++s) {
@@ -414,9 +432,11 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
           }
           if (HS_IN_BOUNDS(uint64_t(p - sv) < size, kBoundsK1)) __stcs(p, v[e]);
         }
-        tile = N.tile;
-        gbase = N.base;
-        if (tile < ntiles) draw(tile);  // (while the copies are awaited)
+        tile = uint32_t(N->tile);
+        gbase = N->base;
+        // the other entry, while the copies are awaited
+        N = reinterpret_cast<NextTile*>(reinterpret_cast<uintptr_t>(N) ^ sizeof(NextTile));
+        if (tile < ntiles) draw(N, tile);
         cp_async_wait();  // the next tile's copies (the only ones in flight)
       } else {
         const uint32_t a1 = a0 ^ G.tw[kWideFlipEntry];
@@ -435,7 +455,7 @@ int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   constexpr auto kernel = k1_wide<OPS, V>;
   HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
   const int threads = 1 << (P.m - kWideBits);
-  const size_t smem = (sizeof(V) << P.m) + sizeof(NextTile);
+  const size_t smem = (sizeof(V) << P.m) + 2 * sizeof(NextTile);
   // resident CTAs per SM, looked up once per device and tile size (the call
   // costs as much host time as the launch of a small pass)
   static std::atomic<int> resident[64][kWideMaxTileBits + 1];
@@ -450,8 +470,11 @@ int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   }
   const uint64_t want = uint64_t(device_sms()) * uint64_t(per_sm);
   const int grid = int(P.ntiles < want ? P.ntiles : want);
-  // (a launch with a CTA per tile hands none out)
-  kernel<<<grid, threads, smem, s>>>(sv, P, uint64_t(grid) < P.ntiles ? ticket : nullptr);
+  // Few tiles per CTA keep the stride: it spreads the last ones evenly, while
+  // numbers drawn a tile ahead go to whichever CTAs start first, several on one SM
+  // (1.4 tiles per CTA, complex64 22 qubits: 233 us with the stride, 276 in order;
+  // 2.3, complex128 22 qubits: 322, 328; 4.6, 23 qubits: 631, 609).
+  kernel<<<grid, threads, smem, s>>>(sv, P, P.ntiles >= 4 * uint64_t(grid) ? ticket : nullptr);
   HS_CUDA(cudaGetLastError());
   return HS_OK;
 }

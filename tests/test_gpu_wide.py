@@ -78,17 +78,24 @@ def test_timed_parts_match_the_plain_call(port, odd):
         assert max(np.abs(x - want).max(), np.abs(y - want).max()) <= tol
 
 
+@pytest.fixture(scope="module")
+def many_tiles(port):
+    """A circuit on 24 qubits: four tiles per CTA and more at every tile size."""
+    n = 24
+    gates = circuits.random_u3_cz(n, 1, n) + [Gate("X", (0,), (n - 1,)), Gate("SWAP", (1, n - 2))]
+    rec, offs = part_offsets(partition.parts_to_gates(gates, partition.partition_frontier(gates, 10)))
+    return n, rec, offs, port.run(n, to_records(gates))
+
+
 @pytest.mark.parametrize("dtype,tol", [(abi.C128, 1e-12), (abi.C64, 1e-5)])
-@pytest.mark.parametrize("hint,n", [(10, 22), (11, 21), (12, 22), (0, 22)])
-def test_more_tiles_than_ctas(port, dtype, tol, hint, n):
+@pytest.mark.parametrize("hint", [0, 10, 11, 12])
+def test_many_tiles_per_cta(many_tiles, dtype, tol, hint):
     """Tiles drawn from the state's counter: it is back at 0 after every pass (a second
     run gives the same bits), two states at once on two streams have their own, and a
     captured run replays."""
     import torch
 
-    gates = circuits.random_u3_cz(n, 2, n) + [Gate("X", (0,), (n - 1,)), Gate("SWAP", (1, n - 2))]
-    rec, offs = part_offsets(partition.parts_to_gates(gates, partition.partition_frontier(gates, 10)))
-    want = port.run(n, to_records(gates))
+    n, rec, offs, want = many_tiles
     prev = abi.set_tile_qubits(hint)
     try:
         st = [abi.State(n, dtype) for _ in range(2)]
