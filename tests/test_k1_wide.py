@@ -251,3 +251,24 @@ def test_timed_calls_plan_as_plain_ones(emu, port):
         if not odd:
             want = port.run(n, to_records([g for p in parts for g in p]))
             assert np.abs(emu(n, parts, mode=3)[0] - want).max() <= 1e-12
+
+
+@pytest.mark.parametrize("dtype,tol", [(0, 1e-12), (1, 1e-4)])
+def test_calls_of_several_windows(emu, port, dtype, tol):
+    """More gates than one planning window holds: parts that end at, before and beyond
+    its border, one longer than a window, empty ones, frames carried across."""
+    n = 11
+    gates = circuits.random_layered(n, 150, 8) + _mixed(n, 6, 9)
+    want = port.run(n, to_records(gates))
+    for sizes in ([25], [1024], [1023, 1, 2], [7, 0, 1100, 30], [len(gates)]):
+        parts, i = [], 0
+        while i < len(gates):
+            k = sizes[len(parts) % len(sizes)]
+            parts.append(gates[i:i + k])
+            i += k
+        got, st = emu(n, parts, dtype=dtype, mode=2)
+        assert st["wide"] == st["passes"]
+        assert np.abs(got - want).max() <= tol
+        if dtype == 1:
+            timed, _ = emu(n, parts, dtype=dtype, mode=3)
+            assert np.array_equal(got, timed)
