@@ -453,23 +453,23 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
 template <bool OPS, typename V>
 int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   constexpr auto kernel = k1_wide<OPS, V>;
-  HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
   const int threads = 1 << (P.m - kWideBits);
   const size_t smem = (sizeof(V) << P.m) + 2 * sizeof(NextTile);
-  // resident CTAs per SM, looked up once per device and tile size (the call
-  // costs as much host time as the launch of a small pass)
+  // CTAs that are resident at once, looked up once per device and tile size (the
+  // calls cost as much host time as the launch of a small pass)
   static std::atomic<int> resident[64][kWideMaxTileBits + 1];
   int dev = 0;
   HS_CUDA(cudaGetDevice(&dev));
   std::atomic<int>& cached = resident[dev & 63][P.m];
-  int per_sm = cached.load(std::memory_order_relaxed);
-  if (per_sm < 1) {
-    HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1) return set_error(HS_E_UNSUPPORTED, "K1 tile does not fit an SM (m=%d)", P.m);
-    cached.store(per_sm, std::memory_order_relaxed);
+  int most = cached.load(std::memory_order_relaxed);
+  if (most < 1) {
+    HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
+    HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kernel, threads, smem));
+    if (most < 1) return set_error(HS_E_UNSUPPORTED, "K1 tile does not fit an SM (m=%d)", P.m);
+    most *= device_sms();
+    cached.store(most, std::memory_order_relaxed);
   }
-  const uint64_t want = uint64_t(device_sms()) * uint64_t(per_sm);
-  const int grid = int(P.ntiles < want ? P.ntiles : want);
+  const int grid = P.ntiles < uint64_t(most) ? int(P.ntiles) : most;
   // Few tiles per CTA keep the stride: it spreads the last ones evenly, while
   // numbers drawn a tile ahead go to whichever CTAs start first, several on one SM
   // (1.4 tiles per CTA, complex64 22 qubits: 233 us with the stride, 276 in order;

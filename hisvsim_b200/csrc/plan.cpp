@@ -759,11 +759,18 @@ void choose_fold(uint8_t* fold, int m, int rbits, const std::vector<uint32_t>& r
   for (int k = 3; k < nslot; ++k) fold[k] = uint8_t(1u << (k % 3));
   if (lane_bits < 1 || nslot <= 3) return;
   // constraints: the lane tile bits of each group
-  std::vector<std::vector<int>> cons;
+  struct Lanes {
+    int n;
+    int bit[4];
+    const int* begin() const { return bit; }
+    const int* end() const { return bit + n; }
+  };
+  std::vector<Lanes> cons;
+  cons.reserve(regs.size());
   for (uint32_t reg : regs) {
-    std::vector<int> lb;
-    for (int b = 0; b < m && int(lb.size()) < lane_bits; ++b)
-      if (!((reg >> b) & 1u)) lb.push_back(b);
+    Lanes lb{};
+    for (int b = 0; b < m && lb.n < lane_bits; ++b)
+      if (!((reg >> b) & 1u)) lb.bit[lb.n++] = b;
     cons.push_back(lb);
   }
   auto vec = [&](const uint8_t* F, int tbit) -> uint32_t {
@@ -774,10 +781,10 @@ void choose_fold(uint8_t* fold, int m, int rbits, const std::vector<uint32_t>& r
   // the lanes' images must have full rank: min(lanes, 3 slot bits + the
   // in-slot bit when a lane bit is one) -- complex64 lanes that share the
   // in-slot half can at best hit every bank pair twice
-  auto independent = [&](const uint8_t* F, const std::vector<int>& lb) {
+  auto independent = [&](const uint8_t* F, const Lanes& lb) {
     int dims = 3;
     for (int b : lb) dims += b < sh;
-    const int want = std::min(int(lb.size()), dims);
+    const int want = std::min(lb.n, dims);
     uint32_t basis[8];
     int rank = 0;
     for (int b : lb) {
@@ -789,7 +796,7 @@ void choose_fold(uint8_t* fold, int m, int rbits, const std::vector<uint32_t>& r
     return rank >= want;
   };
   // the highest slot bit each constraint involves (checked once it is set)
-  auto top = [&](const std::vector<int>& lb) {
+  auto top = [&](const Lanes& lb) {
     int t = -1;
     for (int b : lb) t = std::max(t, b - sh);
     return t;
@@ -902,7 +909,7 @@ bool wide_gate(const SlotGate& s) {
 // A set of a group's ops.
 constexpr int kRecWords = 3;
 struct RecSet {
-  uint64_t w[kRecWords] = {};
+  uint64_t w[kRecWords];  // (RecSet{} is the empty one)
   void add(int i) { w[i >> 6] |= 1ull << (i & 63); }
   RecSet& operator|=(const RecSet& o) {
     for (int k = 0; k < kRecWords; ++k) w[k] |= o.w[k];
@@ -1054,8 +1061,8 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
   // follows from them)
   if (n > kRecWords * 64) return set_error(HS_E_UNSUPPORTED, "%d ops in a group", n);
   RecSet preds[kRecWords * 64], done{}, diag{}, perm{};
-  std::vector<int> queue[kWideBits];  // the non-diagonal ops of each bit, in order
-  size_t head[kWideBits] = {};
+  uint8_t queue[kWideBits][kRecWords * 64];  // the non-diagonal ops of each bit, in order
+  int queued[kWideBits] = {}, head[kWideBits] = {};
   {
     int last[kWideBits];
     RecSet since[kWideBits] = {};
@@ -1068,7 +1075,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
         if ((rec[b].target >> j) & 1u) {
           p |= since[j];
           last[j] = b;
-          queue[j].push_back(b);
+          queue[j][queued[j]++] = uint8_t(b);
           since[j] = RecSet{};
         } else {
           since[j].add(b);
@@ -1097,7 +1104,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
   auto available = [&](int i) { return preds[i].within(done); };
   // a non-diagonal op may run in this step: what it follows is done, or is a
   // diagonal op that may run at the start of the step (`open`)
-  RecSet open;
+  RecSet open{};
   auto ready = [&](int i) { return preds[i].within(done | open); };
   // a conditional sign of the thread or of one register bit
   auto is_sign = [&](int i) {
@@ -1120,6 +1127,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     cplx c;
   };
   std::vector<Piece> pieces;
+  std::vector<int> perms, run;
   auto is_pair = [&](int i) {
     return rec[i].kind == WideRec::kNeg && rec[i].uniform() && __builtin_popcount(rec[i].mask) == 2;
   };
@@ -1136,11 +1144,11 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     // ---- the step's non-diagonal ops
     int rot[kWideBits];
     uint32_t touched = 0, moved = 0;  // register bits acted on; by controlled X and swaps
-    std::vector<int> perms;
+    perms.clear();
     for (int j = 0; j < kWideBits; ++j) {
       rot[j] = -1;
-      while (head[j] < queue[j].size() && rec[queue[j][head[j]]].done) ++head[j];
-      if (head[j] == queue[j].size()) continue;
+      while (head[j] < queued[j] && rec[queue[j][head[j]]].done) ++head[j];
+      if (head[j] == queued[j]) continue;
       const int i = queue[j][head[j]];  // (a later op on the bit has to follow it)
       if (rec[i].kind == WideRec::kRot && ready(i)) {
         rot[j] = i;
@@ -1194,7 +1202,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
       }
     }
     // ---- diagonal ops
-    std::vector<int> run;
+    run.clear();
     auto add_sign = [&](uint32_t bits, uint32_t cthr, uint64_t couter) {
       WideSign& q = P->signs[P->nsigns++];
       q.bits = bits;
@@ -1217,7 +1225,7 @@ int wide_steps(std::vector<WideRec>& rec, int dtype, WideProgram* P, WideGroup* 
     int zs[kWideBits], nz = 0;
     bool need = false;
     for (int j = 0; j < kWideBits; ++j) {
-      if (head[j] == queue[j].size()) continue;
+      if (head[j] == queued[j]) continue;
       const int i = queue[j][head[j]];
       // (nothing non-diagonal on the bit is ahead of it)
       if (rec[i].kind == WideRec::kRot && rec[i].z) {
@@ -1433,6 +1441,7 @@ int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
     build_runs(tile, &P->tile);
     for (int b = 0; b < m; ++b) P->tile_slot[b] = uint8_t(tile[b]);
     std::vector<int> outer;
+    outer.reserve(n);
     for (int s = 0; s < n; ++s)
       if (tbit_of_slot[s] < 0) outer.push_back(s);
     build_runs(outer, &P->outer);
@@ -1440,6 +1449,8 @@ int plan_wide_chunk(int n, int dtype, const std::vector<int>& q2s,
   new_program();
   std::vector<int> members, rest;
   std::vector<WideRec> rec;
+  members.reserve(remaining.size());
+  rec.reserve(remaining.size() + 2);
   while (!remaining.empty()) {
     uint32_t rmask = 0;
     members.clear();
@@ -1655,6 +1666,7 @@ int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* 
                                               low_union_size(tset, low_min)));
     for (int s = 0; s < n && __builtin_popcountll(tset) < m; ++s) tset |= 1ull << s;
     std::vector<int> tile;
+    tile.reserve(m);
     for (int s = 0; s < n; ++s)
       if ((tset >> s) & 1ull) tile.push_back(s);
     const int R = std::min(rbits, m);
@@ -1805,6 +1817,7 @@ int plan_parts(int n, const std::vector<int>& q2s,
                const std::vector<std::vector<LoweredGate>>& parts, Frames* fr, bool flush,
                int tile_bits_hint, int dtype, bool merge, const PassSink& sink) {
   Parts all;
+  all.reserve(parts.size());
   for (const auto& p : parts) all.push_back(&p);
   return plan_call(n, q2s, all, fr, flush, tile_bits_hint, dtype, merge, sink);
 }
