@@ -766,8 +766,8 @@ def main():
                        "partitioner": args.partitioner + (
                            " (limit on non-diagonal targets)" if args.partitioner == "frontier"
                            else ""),
-                       "tile_qubits": args.tile_qubits or "automatic (2^10 tiles, 16 amplitudes "
-                                                          "per thread for complex128)",
+                       "tile_qubits": args.tile_qubits or "automatic (tiles of 2^10 to 2^12, 32 "
+                                                          "amplitudes per thread)",
                        "passes_per_step": passes, "state_bytes": (1 << n) * 16,
                        "l2": "state >> L2 (126 MB), no flush", "parallelism": f"replicas{world}"},
             "circuit_s": t_step, "hbm_GBps": passes * bytes_per_pass / t_step / 1e9,

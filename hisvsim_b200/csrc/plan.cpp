@@ -1779,10 +1779,13 @@ namespace {
 // The parts of a call, window by window: a window's passes are on the device
 // before the next window is rewritten, and what a chunk walks stays bounded, so
 // planning is linear in the gates.  Where gates may move (`merge`) a window takes
-// whole parts up to kWindowGates gates (one part at least): half a millisecond of
-// planning ahead of its first pass, and at most one pass more than over the whole
-// call per some thirty; elsewhere it is one part.
-constexpr size_t kWindowGates = 1024;
+// whole parts up to window_gates (one part at least); elsewhere it is one part.
+// No gate moves across a window's border, which costs a pass or two there: on
+// large states, where a pass takes longer than planning hundreds of gates, windows
+// are larger (33 qubits, 1960 gates in parts of touched qubits: 54 passes in
+// windows of 1024 gates, 51 in one).  Up to 22 qubits half a millisecond of
+// planning is ahead of a call's first pass.
+size_t window_gates(int n) { return size_t(1024) << std::clamp(n - 22, 0, 4); }
 
 int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr, bool flush,
               int tile_bits_hint, int dtype, bool merge, const PassSink& sink) {
@@ -1790,7 +1793,7 @@ int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr
   const bool wide = use_wide(n, dtype);
   const bool flips = wide && (tile_bits_hint <= 0 || tile_bits_hint >= kWideMinTileBits) &&
                      all_wide(parts, *fr);
-  const size_t most = wide && merge && moves_gates(dtype) ? kWindowGates : 0;
+  const size_t most = wide && merge && moves_gates(dtype) ? window_gates(n) : 0;
   size_t i = 0;
   int first = 0;
   const PassSink tagged = [&](PlannedPass& p) {

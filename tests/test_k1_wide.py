@@ -272,3 +272,18 @@ def test_calls_of_several_windows(emu, port, dtype, tol):
         if dtype == 1:
             timed, _ = emu(n, parts, dtype=dtype, mode=3)
             assert np.array_equal(got, timed)
+
+
+def test_windows_grow_with_the_state(emu):
+    """A call of 1960 gates on 33 qubits is one window (fewer passes than its halves
+    planned apart)."""
+    def passes(n, parts):
+        rec, offs = part_offsets(parts)
+        k, sec = ctypes.c_int32(), (ctypes.c_double * 2)()
+        assert emu.lib.wide_plan_time(n, 0, rec.ctypes.data, offs.ctypes.data, len(offs) - 1,
+                                      ctypes.byref(k), sec) == 0
+        return k.value
+    gates = circuits.random_u3_cz(33, 40, 1)
+    parts = partition.parts_to_gates(gates, partition.partition_frontier(gates, 9))
+    cut = next(i for i in range(len(parts)) if sum(map(len, parts[:i + 1])) > 1024)
+    assert passes(33, parts) < passes(33, parts[:cut]) + passes(33, parts[cut:])
