@@ -131,8 +131,8 @@ constexpr double kFlipPivotC64 = 0.6;
 //   form 2 (scaled, rho > 1): M = diag(1 / c, c rho) [[1, t], [0, 1]] [[1, 0], [s, 1]],
 //     s = sg / (c rho), t = -sg c rho (rho shrinks to c^2 rho).
 // Forms 1 and 2 take 4 FMA per pair instead of 6 and leave a real scale on
-// the qubit's two values, which complex128 frames carry (`scaled`);
-// complex64 states keep form 0.  False when W is not of the form above to
+// the qubit's two values, which the frames carry (`scaled`: complex128, and
+// complex64 calls with flips; other complex64 calls keep form 0).  False when W is not of the form above to
 // 1e-12 (custom C1 matrices need not be).
 // `pivot` > 0: cosines below it are turned (Rot::flip).
 
@@ -329,7 +329,7 @@ bool out_of_range(cplx G, double lim) {
   return !(g <= top && g * top >= 1.0);
 }
 
-// `scaled`: rotations may leave real scales in the frames (complex128);
+// `scaled`: rotations may leave real scales in the frames (factor_rotation);
 // `lim`: the global factor's scale is flushed once it leaves 2^+-lim; `split`:
 // diagonal gates become phases (split_diagonal), for wide programs.
 void rewrite_gate(const LoweredGate& g, Frames* F, bool scaled, double pivot, double lim,
