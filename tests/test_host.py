@@ -333,3 +333,22 @@ def test_reference_arm_says_why_it_is_unavailable(monkeypatch, capsys):
     bench.main()
     line = json.loads(capsys.readouterr().out)
     assert line["impl"] == "reference" and "libhisv_ref.so" in line["unavailable"]
+
+
+def test_build_does_without_the_reference(monkeypatch, tmp_path):
+    """__graft_entry__.build() where the reference's directory holds no sources: the
+    library and the port oracle are built, the reference's harness is not asked for."""
+    import subprocess
+    import sys
+
+    if ROOT not in sys.path:
+        sys.path.insert(0, ROOT)
+    import __graft_entry__ as entry
+    from hisvsim_b200 import build
+
+    calls = []
+    monkeypatch.setenv("HISV_REFERENCE", str(tmp_path))
+    monkeypatch.setattr(build, "build_all", lambda verbose=False: calls.append("all"))
+    monkeypatch.setattr(subprocess, "run", lambda cmd, **kw: calls.append(cmd[-1]))
+    entry.build()
+    assert calls == ["all", "port"]
