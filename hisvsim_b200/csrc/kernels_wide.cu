@@ -6,6 +6,7 @@
 // straight from the last group's registers -- for the same entry points.
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "bounds.cuh"
@@ -297,9 +298,10 @@ __device__ __forceinline__ uint64_t warp_deposit(uint32_t x, const Runs& r) {
 // stride of tiles the CTAs drift apart and meet their neighbours' sectors after
 // they left the L2: complex128, 33 qubits in frontier parts of 12, 7 layers, 1661
 // ms against 815; 30 qubits in parts of 9, where whole lines are read, 145
-// against 122.  A state without a counter keeps the stride (as do small launches).
+// against 122.  Small launches, and states without a counter, keep the stride
+// (ORDERED = false; launch below).
 // OPS: the program has other ops than rotations, signs, tables and negations
-template <bool OPS, typename V>
+template <bool OPS, bool ORDERED, typename V>
 __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
     k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P, uint32_t* ticket) {
   extern __shared__ __align__(128) unsigned char smem_raw[];  // the tile, then two NextTile
@@ -325,32 +327,35 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
         cp_async16(sb + (ct ^ P.cslot[k]), base + P.gchunk[k]);
     cp_async_commit();
   };
-  uint32_t tile = blockIdx.x;
-  const uint32_t ntiles = uint32_t(P.ntiles);
-  uint64_t gbase = deposit(tile, P.outer);
-  // the tile after the present one, known a tile ahead: written by warp 0 into one
-  // entry while the other is read.  One number per tile: a launch draws ntiles in all
+  std::conditional_t<ORDERED, uint32_t, uint64_t> tile = blockIdx.x;
+  uint64_t gbase = tile < P.ntiles ? deposit(tile, P.outer) : 0;
+  // ORDERED: the tile after the present one, known a tile ahead: written by warp 0
+  // into one entry while the other is read.  One number per tile: a launch draws
+  // ntiles in all
   NextTile* N = reinterpret_cast<NextTile*>(smem_raw + (sizeof(V) << P.m));
-  auto draw = [&](NextTile* to, uint32_t after) {
+  auto draw = [&](NextTile* to) {
     if (t >= 32u) return;
-    uint32_t x = after;
-    if (ticket) {
-      if (t == 0) x = atomicInc(ticket, ntiles - 1);
-      x = __shfl_sync(0xffffffffu, x, 0);
-    }
-    x += gridDim.x;
+    uint32_t x = 0;
+    if (t == 0) x = atomicInc(ticket, uint32_t(P.ntiles - 1));
+    x = gridDim.x + __shfl_sync(0xffffffffu, x, 0);
     const uint64_t base = warp_deposit(x, P.outer);
     if (t == 0) {
       to->tile = x;
       to->base = base;
     }
   };
-  issue(gbase);
-  draw(N, tile);
+  // the stride: the next tile's offset by one addition in the scattered outer bits
+  // (the carries run through the other bits, which are set)
+  const uint64_t omask = ORDERED ? 0 : deposit(P.ntiles - 1, P.outer);
+  const uint64_t ostep = ORDERED ? 0 : deposit(uint64_t(gridDim.x), P.outer);
+  if (tile < P.ntiles) issue(gbase);
+  if constexpr (ORDERED) draw(N);
   cp_async_wait();
   __syncthreads();
   V v[E];
-  while (tile < ntiles) {
+  while (tile < P.ntiles) {
+    const uint64_t next = tile + gridDim.x;
+    const uint64_t gnext = !ORDERED && next < P.ntiles ? (((gbase | ~omask) + ostep) & omask) : 0;
     for (int g = 0; g < P.ngroups; ++g) {
       const WideGroup& G = P.groups[g];
       const bool last = g == P.ngroups - 1;
@@ -374,7 +379,11 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
         // every thread holds its registers of the last group: the buffer takes
         // the next tile while this one is finished and stored
         __syncthreads();
-        if (N->tile < ntiles) issue(N->base);
+        if constexpr (ORDERED) {
+          if (N->tile < P.ntiles) issue(N->base);
+        } else {
+          if (next < P.ntiles) issue(gnext);
+        }
       }
       uint32_t z = 0;  // pending signs (WideSign)
       for (int s = G.first_step, s_end = s + G.num_steps; s < s_end; ++s) {
@@ -432,11 +441,13 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
           }
           if (HS_IN_BOUNDS(uint64_t(p - sv) < size, kBoundsK1)) __stcs(p, v[e]);
         }
-        tile = uint32_t(N->tile);
-        gbase = N->base;
-        // the other entry, while the copies are awaited
-        N = reinterpret_cast<NextTile*>(reinterpret_cast<uintptr_t>(N) ^ sizeof(NextTile));
-        if (tile < ntiles) draw(N, tile);
+        if constexpr (ORDERED) {
+          tile = uint32_t(N->tile);
+          gbase = N->base;
+          // the other entry, while the copies are awaited
+          N = reinterpret_cast<NextTile*>(reinterpret_cast<uintptr_t>(N) ^ sizeof(NextTile));
+          if (tile < P.ntiles) draw(N);
+        }
         cp_async_wait();  // the next tile's copies (the only ones in flight)
       } else {
         const uint32_t a1 = a0 ^ G.tw[kWideFlipEntry];
@@ -447,34 +458,50 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
       }
       __syncthreads();
     }
+    if constexpr (!ORDERED) {
+      tile += gridDim.x;
+      gbase = gnext;
+    }
   }
+}
+
+// CTAs of the kernel that are resident at once, looked up once per device and tile
+// size (the calls cost as much host time as the launch of a small pass)
+template <bool OPS, bool ORDERED, typename V>
+int resident_ctas(int m, size_t smem, int* most) {
+  static std::atomic<int> resident[64][kWideMaxTileBits + 1];
+  int dev = 0;
+  HS_CUDA(cudaGetDevice(&dev));
+  std::atomic<int>& cached = resident[dev & 63][m];
+  *most = cached.load(std::memory_order_relaxed);
+  if (*most >= 1) return HS_OK;
+  constexpr auto kernel = k1_wide<OPS, ORDERED, V>;
+  HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
+  HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(most, kernel, 1 << (m - kWideBits), smem));
+  if (*most < 1) return set_error(HS_E_UNSUPPORTED, "K1 tile does not fit an SM (m=%d)", m);
+  *most *= device_sms();
+  cached.store(*most, std::memory_order_relaxed);
+  return HS_OK;
 }
 
 template <bool OPS, typename V>
 int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
-  constexpr auto kernel = k1_wide<OPS, V>;
   const int threads = 1 << (P.m - kWideBits);
-  const size_t smem = (sizeof(V) << P.m) + 2 * sizeof(NextTile);
-  // CTAs that are resident at once, looked up once per device and tile size (the
-  // calls cost as much host time as the launch of a small pass)
-  static std::atomic<int> resident[64][kWideMaxTileBits + 1];
-  int dev = 0;
-  HS_CUDA(cudaGetDevice(&dev));
-  std::atomic<int>& cached = resident[dev & 63][P.m];
-  int most = cached.load(std::memory_order_relaxed);
-  if (most < 1) {
-    HS_TRY(smem_optin(reinterpret_cast<const void*>(kernel)));
-    HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kernel, threads, smem));
-    if (most < 1) return set_error(HS_E_UNSUPPORTED, "K1 tile does not fit an SM (m=%d)", P.m);
-    most *= device_sms();
-    cached.store(most, std::memory_order_relaxed);
-  }
-  const int grid = P.ntiles < uint64_t(most) ? int(P.ntiles) : most;
+  const size_t tile = sizeof(V) << P.m;
+  int most = 0;
+  HS_TRY((resident_ctas<OPS, false, V>(P.m, tile, &most)));
   // Few tiles per CTA keep the stride: it spreads the last ones evenly, while
   // numbers drawn a tile ahead go to whichever CTAs start first, several on one SM
   // (1.4 tiles per CTA, complex64 22 qubits: 233 us with the stride, 276 in order;
   // 2.3, complex128 22 qubits: 322, 328; 4.6, 23 qubits: 631, 609).
-  kernel<<<grid, threads, smem, s>>>(sv, P, P.ntiles >= 4 * uint64_t(grid) ? ticket : nullptr);
+  if (ticket && P.ntiles >= 4 * uint64_t(most)) {
+    const size_t smem = tile + 2 * sizeof(NextTile);
+    HS_TRY((resident_ctas<OPS, true, V>(P.m, smem, &most)));
+    k1_wide<OPS, true, V><<<most, threads, smem, s>>>(sv, P, ticket);
+  } else {
+    const int grid = P.ntiles < uint64_t(most) ? int(P.ntiles) : most;
+    k1_wide<OPS, false, V><<<grid, threads, tile, s>>>(sv, P, nullptr);
+  }
   HS_CUDA(cudaGetLastError());
   return HS_OK;
 }
