@@ -1500,6 +1500,12 @@ struct ChunkRoom {
   }
 };
 
+// Lists that a call's windows share.
+struct PlanLists {
+  std::vector<RGate> rg;
+  std::vector<SlotGate> sgs;
+};
+
 // The planner of both program kinds, for some parts of a call: into `programs`
 // (PartPrograms only) or, with `sink`, as PartPrograms and WidePrograms, handed
 // over pass by pass.  A pass takes what fits of the first part left (in order, up
@@ -1511,11 +1517,12 @@ struct ChunkRoom {
 // passes instead of 13; 20 random layers of 20 qubits in parts of 10: 9 instead
 // of 26).  `flips`: rotations beyond the pivot become flips (all_wide).
 int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* fr, bool flush,
-                int tile_bits_hint, int dtype, bool flips, std::vector<PartProgram>* programs,
-                const PassSink* sink) {
+                int tile_bits_hint, int dtype, bool flips, PlanLists* lists,
+                std::vector<PartProgram>* programs, const PassSink* sink) {
   if (n < 1 || n > 63) return set_error(HS_E_INVALID, "bad qubit count %d", n);
   if (int(fr->r.size()) != n) fr->reset(n);
-  std::vector<RGate> rg;
+  std::vector<RGate>& rg = lists->rg;
+  rg.clear();
   size_t count = 2;
   for (const auto* g : gates) count += g->size();
   rg.reserve(count);
@@ -1549,7 +1556,8 @@ int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* 
   // line is fetched as well and often evicted before its own tile reads it
   // -- 3.7% slower at 33 qubits)
   const int low_min = std::min(n, 3);
-  std::vector<SlotGate> sgs;
+  std::vector<SlotGate>& sgs = lists->sgs;
+  sgs.clear();
   sgs.reserve(rg.size());
   for (const auto& r : rg) {
     SlotGate s;
@@ -1603,6 +1611,7 @@ int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* 
     chunks.emplace_back();
     Chunk& c = chunks.back();
     c.wide = wide;
+    c.gates.reserve(std::min<size_t>(sgs.size() - size_t(x), 64));
     ChunkRoom room;
     const int part = sgs[x].rg->part;
     while (x < int(sgs.size()) && join(&c, &room, x, part)) ++x;
@@ -1758,7 +1767,7 @@ int plan_chunks(int n, const std::vector<int>& q2s, const Parts& gates, Frames* 
     Frames g;
     g.reset(n);
     g.G = gamma;
-    return plan_chunks(n, q2s, {}, &g, true, tile_bits_hint, dtype, false, nullptr, sink);
+    return plan_chunks(n, q2s, {}, &g, true, tile_bits_hint, dtype, false, lists, nullptr, sink);
   }
   if (!sink)
     for (auto& P : *programs) finish_layout(&P, dtype);
@@ -1771,7 +1780,9 @@ int plan_gates(int n, const std::vector<int>& q2s, const std::vector<LoweredGate
                Frames* fr, bool flush, int tile_bits_hint, int dtype,
                std::vector<PartProgram>* programs) {
   programs->clear();
-  return plan_chunks(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, false, programs, nullptr);
+  PlanLists lists;
+  return plan_chunks(n, q2s, {&gates}, fr, flush, tile_bits_hint, dtype, false, &lists, programs,
+                     nullptr);
 }
 
 namespace {
@@ -1800,8 +1811,10 @@ int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr
     p.of_part = first;
     return sink(p);
   };
+  PlanLists lists;
+  Parts window;
   do {
-    Parts window;
+    window.clear();
     first = int(i);
     for (size_t count = 0; i < parts.size(); ++i) {
       count += parts[i]->size();
@@ -1809,7 +1822,7 @@ int plan_call(int n, const std::vector<int>& q2s, const Parts& parts, Frames* fr
       window.push_back(parts[i]);
     }
     HS_TRY(plan_chunks(n, q2s, window, fr, flush && i == parts.size(), tile_bits_hint, dtype, flips,
-                       nullptr, &tagged));
+                       &lists, nullptr, &tagged));
   } while (i < parts.size());
   return HS_OK;
 }
