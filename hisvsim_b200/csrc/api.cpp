@@ -234,7 +234,8 @@ int permute_positions(hs_state* st, const std::vector<int>& pi, cudaStream_t s) 
 }
 
 int launch_pass(hs_state* st, const PlannedPass& p, cudaStream_t s) {
-  HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, st->ticket, s)
+  if (p.wide) p.wide->ticket = st->ticket;
+  HS_TRY(p.wide ? launch_wide(st->amp, st->dtype, *p.wide, s)
                 : launch_part(st->amp, st->dtype, *p.part, s));
   count_pass(p.nops());
   g_param_bytes += (long long)p.bytes();

@@ -272,6 +272,7 @@ struct WideProgram {
   int32_t nsteps, nsigns, nconds, nwops;
   int32_t per_thr;          // chunks a thread copies
   uint64_t ntiles;
+  uint32_t* ticket;         // the state's tile counter, set for the launch (launch_wide)
   Runs tile, outer;
   uint8_t tile_slot[16];
   uint8_t fold[16];         // shared-memory layout, as in PartProgram
@@ -488,8 +489,8 @@ cudaError_t device_malloc(T** p, size_t bytes) {
 
 // ---- launchers (kernels_*.cu) ----------------------------------------------
 int launch_part(void* amp, int dtype, const PartProgram& prog, cudaStream_t s);
-// `ticket`: the state's tile counter (device; null = none), left at 0
-int launch_wide(void* amp, int dtype, const WideProgram& prog, uint32_t* ticket, cudaStream_t s);
+// prog.ticket: the state's tile counter (device; null = none), left at 0
+int launch_wide(void* amp, int dtype, const WideProgram& prog, cudaStream_t s);
 // a free tile counter (-1: none left), and its device address
 int ticket_take();
 void ticket_give(int i);

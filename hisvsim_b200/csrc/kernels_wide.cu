@@ -5,9 +5,7 @@
 // register group runs, exchanged through shared memory between groups, stored
 // straight from the last group's registers -- for the same entry points.
 #include <atomic>
-#include <mutex>
 #include <type_traits>
-#include <vector>
 
 #include "bounds.cuh"
 #include "internal.h"
@@ -291,7 +289,7 @@ __device__ __forceinline__ uint64_t warp_deposit(uint32_t x, const Runs& r) {
          __reduce_or_sync(0xffffffffu, uint32_t(v));
 }
 
-// Tiles are handed out in order, by a counter of the state's (`ticket`, 0 between
+// Tiles are handed out in order, by a counter of the state's (P.ticket, 0 between
 // launches: a launch counts to its number of tiles and wraps).  The tiles in
 // flight are then always neighbours, and the sectors and DRAM pages that
 // neighbouring tiles share are read and written once.  With every CTA on a fixed
@@ -303,7 +301,7 @@ __device__ __forceinline__ uint64_t warp_deposit(uint32_t x, const Runs& r) {
 // OPS: the program has other ops than rotations, signs, tables and negations
 template <bool OPS, bool ORDERED, typename V>
 __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
-    k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P, uint32_t* ticket) {
+    k1_wide(V* __restrict__ sv, const __grid_constant__ WideProgram P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];  // the tile, then two NextTile
   const uint32_t t = threadIdx.x;
   const uint32_t tile_bytes = uint32_t(sizeof(V)) << P.m;
@@ -336,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, WideTraits<V>::blocks)
   auto draw = [&](NextTile* to) {
     if (t >= 32u) return;
     uint32_t x = 0;
-    if (t == 0) x = atomicInc(ticket, uint32_t(P.ntiles - 1));
+    if (t == 0) x = atomicInc(P.ticket, uint32_t(P.ntiles - 1));
     x = gridDim.x + __shfl_sync(0xffffffffu, x, 0);
     const uint64_t base = warp_deposit(x, P.outer);
     if (t == 0) {
@@ -485,7 +483,7 @@ int resident_ctas(int m, size_t smem, int* most) {
 }
 
 template <bool OPS, typename V>
-int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
+int launch(V* sv, const WideProgram& P, cudaStream_t s) {
   const int threads = 1 << (P.m - kWideBits);
   const size_t tile = sizeof(V) << P.m;
   int most = 0;
@@ -494,23 +492,23 @@ int launch(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
   // numbers drawn a tile ahead go to whichever CTAs start first, several on one SM
   // (1.4 tiles per CTA, complex64 22 qubits: 233 us with the stride, 276 in order;
   // 2.3, complex128 22 qubits: 322, 328; 4.6, 23 qubits: 631, 609).
-  if (ticket && P.ntiles >= 4 * uint64_t(most)) {
+  if (P.ticket && P.ntiles >= 4 * uint64_t(most)) {
     const size_t smem = tile + 2 * sizeof(NextTile);
     HS_TRY((resident_ctas<OPS, true, V>(P.m, smem, &most)));
-    k1_wide<OPS, true, V><<<most, threads, smem, s>>>(sv, P, ticket);
+    k1_wide<OPS, true, V><<<most, threads, smem, s>>>(sv, P);
   } else {
     const int grid = P.ntiles < uint64_t(most) ? int(P.ntiles) : most;
-    k1_wide<OPS, false, V><<<grid, threads, tile, s>>>(sv, P, nullptr);
+    k1_wide<OPS, false, V><<<grid, threads, tile, s>>>(sv, P);
   }
   HS_CUDA(cudaGetLastError());
   return HS_OK;
 }
 
 template <typename V>
-int launch_typed(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
+int launch_typed(V* sv, const WideProgram& P, cudaStream_t s) {
   bool ops = false;
   for (int i = 0; i < P.nwops; ++i) ops |= P.ops[i].code != wk_neg;
-  return ops ? launch<true>(sv, P, ticket, s) : launch<false>(sv, P, ticket, s);
+  return ops ? launch<true>(sv, P, s) : launch<false>(sv, P, s);
 }
 
 }  // namespace
@@ -519,45 +517,9 @@ int launch_typed(V* sv, const WideProgram& P, uint32_t* ticket, cudaStream_t s) 
 HS_BOUNDS_TAKE(bounds_take_wide)
 #endif
 
-int launch_wide(void* amp, int dtype, const WideProgram& P, uint32_t* ticket, cudaStream_t s) {
-  if (dtype == HS_DTYPE_C128) return launch_typed(static_cast<double2*>(amp), P, ticket, s);
-  return launch_typed(static_cast<float2*>(amp), P, ticket, s);
-}
-
-// The states' tile counters: one 32-byte sector each of a fixed array, so that a
-// launch needs no memory of its own and none is reset between launches.  (Calls
-// on one state are ordered among themselves; states share no counter.)
-namespace {
-constexpr int kTickets = 4096, kTicketStride = 8;
-__device__ uint32_t g_tickets[kTickets * kTicketStride];
-std::mutex g_ticket_mu;
-std::vector<int> g_ticket_free;
-int g_ticket_next = 0;
-}  // namespace
-
-int ticket_take() {
-  std::lock_guard<std::mutex> lk(g_ticket_mu);
-  if (!g_ticket_free.empty()) {
-    const int i = g_ticket_free.back();
-    g_ticket_free.pop_back();
-    return i;
-  }
-  return g_ticket_next < kTickets ? g_ticket_next++ : -1;
-}
-
-void ticket_give(int i) {
-  if (i < 0) return;
-  std::lock_guard<std::mutex> lk(g_ticket_mu);
-  g_ticket_free.push_back(i);
-}
-
-uint32_t* ticket_address(int i) {
-  void* p = nullptr;
-  if (i < 0 || cudaGetSymbolAddress(&p, g_tickets) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return static_cast<uint32_t*>(p) + size_t(i) * kTicketStride;
+int launch_wide(void* amp, int dtype, const WideProgram& P, cudaStream_t s) {
+  if (dtype == HS_DTYPE_C128) return launch_typed(static_cast<double2*>(amp), P, s);
+  return launch_typed(static_cast<float2*>(amp), P, s);
 }
 
 }  // namespace hisv
