@@ -127,6 +127,10 @@ int hs_event_destroy(void* ev);
 /* StateVector(n, numa) (py_wrapper.cpp:143, state_vector.hpp:60-119): a
  * device-resident 2^n state initialised to |0...0>, identity slot map. */
 int hs_state_create(int num_qubits, int dtype, hs_state** out);
+/* Waits for the state's work.  Device memory of states up to 16 MiB that were used
+ * on the default stream alone (and whose pointer was not handed out) is kept for
+ * the next state of the size, at most 32 MiB per device, and given back when an
+ * allocation of the library runs out of memory. */
 int hs_state_destroy(hs_state* st);
 int hs_state_num_qubits(const hs_state* st, int* n);
 int hs_state_dtype(const hs_state* st, int* dtype);
